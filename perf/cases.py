@@ -30,28 +30,28 @@ PROJ_N, PROJ_K, VOCAB = 6144, 2048, 151936     # the operator suite's projection
 def listed():
     return [
         # the operator suite at a handful of tokens: eager calls, where launches and host work count
-        dict(name="operator suite, 7 rows", kind="suite", rows=7),
+        dict(name="operator suite 7 rows", kind="suite", rows=7),
         # one user: a decode step of a small dense model from its captured graph
-        dict(name="decode dense, 1 sequence", kind="decode", model="qwen3-1.7b-shape", sequences=1, context=333, ragged=False),
+        dict(name="decode dense 1 sequence", kind="decode", model="qwen3-1.7b-shape", sequences=1, context=333, ragged=False),
         # a rollout batch of a small dense model whose sequences are at different lengths
-        dict(name="decode dense, ragged", kind="decode", model="qwen2-1.5b-shape", sequences=250, context=8192, ragged=True),
+        dict(name="decode dense ragged", kind="decode", model="qwen2-1.5b-shape", sequences=250, context=8192, ragged=True),
         # the headline workload: a rollout batch of the mixture-of-experts model, one of eight pipeline stages
-        dict(name="decode moe, 512 x 2048", kind="decode", model="qwen3-30b-a3b-shape", sequences=512, context=2048, ragged=False),
+        dict(name="decode moe 512 x 2048", kind="decode", model="qwen3-30b-a3b-shape", sequences=512, context=2048, ragged=False),
         # a rollout batch of the latent-attention model
-        dict(name="decode mla, 64 x 4096", kind="decode", model="moonlight-16b-a3b-shape", sequences=64, context=4096, ragged=False),
+        dict(name="decode mla 64 x 4096", kind="decode", model="moonlight-16b-a3b-shape", sequences=64, context=4096, ragged=False),
         # one chunk of a long prompt
-        dict(name="prefill dense, chunk", kind="prefill", model="qwen2-1.5b-shape", prompts=1, tokens=2048, past=2048),
+        dict(name="prefill dense chunk", kind="prefill", model="qwen2-1.5b-shape", prompts=1, tokens=2048, past=2048),
         # fresh prompts packed under the scheduler's token budget
-        dict(name="prefill moe, 3 prompts", kind="prefill", model="qwen3-30b-a3b-shape", prompts=3, tokens=2048, past=0),
-        dict(name="prefill mla, 4 prompts", kind="prefill", model="moonlight-16b-a3b-shape", prompts=4, tokens=3001, past=0),
+        dict(name="prefill moe 3 prompts", kind="prefill", model="qwen3-30b-a3b-shape", prompts=3, tokens=2048, past=0),
+        dict(name="prefill mla 4 prompts", kind="prefill", model="moonlight-16b-a3b-shape", prompts=4, tokens=3001, past=0),
         # a hybrid decoder (state space and latent attention) on fresh prompts
-        dict(name="prefill hybrid, 3 prompts", kind="hybrid", prompts=3, tokens=4096, decode=False),
+        dict(name="prefill hybrid 3 prompts", kind="hybrid", prompts=3, tokens=4096, decode=False),
         # the trainer's side of a rollout: attention over packed sequences, forward and backward
-        dict(name="train attention, 4 x 2048", kind="train_attention", model="qwen3-30b-a3b-shape", sequences=4, tokens=8192),
+        dict(name="train attention 4 x 2048", kind="train_attention", model="qwen3-30b-a3b-shape", sequences=4, tokens=8192),
         # one mixture-of-experts layer, forward and backward
-        dict(name="train experts, 4096 tokens", kind="train_experts", model="qwen3-30b-a3b-shape", tokens=4096, stacked=False),
+        dict(name="train experts 4096 tokens", kind="train_experts", model="qwen3-30b-a3b-shape", tokens=4096, stacked=False),
         # per-token log-probabilities of the trainer's logits, forward and backward
-        dict(name="train logprob, 2000 rows", kind="train_logprob", rows=2000, vocab=151936, dtype="bf16"),
+        dict(name="train logprob 2000 rows", kind="train_logprob", rows=2000, vocab=151936, dtype="bf16"),
     ]
 
 
