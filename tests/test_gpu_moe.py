@@ -484,3 +484,46 @@ def test_weight_gradient_kernels_tensor_core_and_cuda_core_forms(vb):
         assert not c[0].any() and not c[4].any()
     torch.cuda.synchronize()
     assert vb._lib.read_status()[0] == 0
+
+
+@pytest.mark.parametrize("E,k,T,H,I", [(4, 2, 150, 256, 200), (3, 1, 1111, 128, 72), (8, 4, 260, 192, 328)])
+def test_grouped_gemm_tile_heights_and_unfused_swiglu(vb, E, k, T, H, I):
+    """More than 64 rows per expert: tiles of up to 128 or 256 rows, cut evenly in steps of 16 and fetched in boxes by the
+    binary digits of their height.  A row's bits do not depend on its tile, so every tile height gives those of 64-row tiles;
+    the elementwise SwiGLU (16 bytes per thread, or 2 where a row stride does not allow it) rounds as the fused epilogue."""
+    from vexact_b200 import _lib, fused_moe as fm
+
+    g = torch.Generator().manual_seed(E * T)
+    x = torch.randn(T, H, generator=g).to(BF).cuda()
+    w = (torch.randn(E, 2 * I, H, generator=g) * 0.05).to(BF).cuda()
+    sel = torch.stack([torch.randperm(E, generator=g)[:k] for _ in range(T)]).cuda()
+    sel[: T // 2, 0] = sel[0, 0]                       # one crowded expert (top-1 or not: duplicates are rows of their own)
+    rw = torch.rand(T, k, generator=g).to(BF).cuda()
+    assert T * k > 64 * E
+    plan = fm._permute(sel, rw, x, E)
+    count = int(plan["tile_count"])
+    table = plan["tile_table"][:count].cpu()
+    cu = plan["cu_seqlens"].cpu()
+    for e in range(E):                                 # the tiles of an expert cover its rows, in order, evenly
+        mine = table[table[:, 0] == e]
+        rows = int(cu[e + 1] - cu[e])
+        assert mine[:, 2].sum() == rows and len(mine) == -(-rows // plan["tile_rows"])
+        if rows:
+            assert mine[0, 1] == cu[e] and mine[:, 2].max() <= plan["tile_rows"] and mine[:, 2].min() > 0
+            assert torch.equal(mine[1:, 1], mine[:-1, 1] + mine[:-1, 2])
+    tall = fm._grouped_gemm(plan["x_perm"], w, None, plan, 2 * I, mode=0)
+    low = dict(plan, tile_rows=64)
+    rows64 = [(e, r, min(64, int(cu[e + 1]) - r), 0) for e in range(E) for r in range(int(cu[e]), int(cu[e + 1]), 64)]
+    low.update(tile_table=torch.tensor(rows64, dtype=torch.int32).cuda(), max_tiles=len(rows64),
+               tile_count=torch.tensor([len(rows64)], dtype=torch.int32).cuda())
+    assert torch.equal(tall, fm._grouped_gemm(plan["x_perm"], w, None, low, 2 * I, mode=0))
+    fused = fm._grouped_gemm(plan["x_perm"], w, plan["row_scale"], low, I, mode=1)
+    odd = torch.empty(tall.shape[0], 2 * I + 2, dtype=BF, device="cuda")          # a row stride without 16-byte rows
+    odd[:, :2 * I] = tall
+    for gu in (tall, odd):
+        h = torch.empty_like(fused)
+        _lib.check(_lib.load().b200_swiglu_scale_strided(gu.data_ptr(), gu.data_ptr() + 2 * I, plan["row_scale"].data_ptr(),
+                                                         h.data_ptr(), gu.shape[0], I, gu.stride(0), _lib.current_stream()), "swiglu")
+        assert torch.equal(h, fused)
+    torch.cuda.synchronize()
+    assert vb._lib.read_status()[0] == 0

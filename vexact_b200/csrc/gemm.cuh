@@ -63,6 +63,8 @@ struct GemmParams {
   int fp16;             // plain dense mode: operands, bias and 16-bit output are fp16 instead of bf16
   int scalar_epilogue;  // development knob B200_GEMM_EPI_SCALAR=1: 2-byte stores in the plain epilogue
   const int* tile_count;
+  int tokens_first;  // tile order: a weight tile's token tiles one after the other (1), or a token tile's weight tiles (0)
+  int split_boxes;   // activation boxes by the binary digits of a tile's height instead of p.xbox rows each
   int xbox;       // rows per activation TMA box (multiple of 16)
   int xrows_max;  // largest token count of any tile (multiple of xbox, <= 256)
   int stages;
@@ -151,6 +153,19 @@ struct GemmTile {
   int group, row0, n, wt;
 };
 
+// Activation maps of one launch.  box[0] serves tiles that are fetched in boxes of p.xbox rows.  Tall grouped tiles
+// (p.split_boxes) are fetched exactly, rounded up to 16 rows, as the binary digits of their height: box[i] is 256 >> i rows
+// high, so a tile of 144 rows is one box of 128 and one of 16.  Fewer copies per stage matter: at 256-row tiles, boxes of
+// 64 / 32 / 16 rows made fc1 of 4096 tokens (128 experts, 2048 -> 1536) 260 / 297 / 393 us.
+struct GemmXMaps {
+  CUtensorMap box[5];
+};
+
+// Token columns that a tile of n rows occupies in shared and tensor memory.
+__device__ __forceinline__ int gemm_tile_cols(const GemmParams& p, int n) {
+  return p.split_boxes ? (n + 15) & ~15 : (n + p.xbox - 1) / p.xbox * p.xbox;
+}
+
 __device__ __forceinline__ bool gemm_tile(const GemmParams& p, int t_tiles, long long linear, GemmTile& t) {
   const long long per_product = (long long)t_tiles * p.w_tiles;
   if (linear >= per_product * (1 + p.batch_extra)) return false;
@@ -159,8 +174,14 @@ __device__ __forceinline__ bool gemm_tile(const GemmParams& p, int t_tiles, long
     product = (int)(linear / per_product);
     linear -= product * per_product;
   }
-  t.wt = (int)(linear / t_tiles);
-  const int tt = (int)(linear % t_tiles);
+  int tt;
+  if (p.tokens_first) {
+    t.wt = (int)(linear / t_tiles);
+    tt = (int)(linear % t_tiles);
+  } else {
+    tt = (int)(linear / p.w_tiles);
+    t.wt = (int)(linear % p.w_tiles);
+  }
   if (p.tile_table) {
     const int4 e = p.tile_table[tt];
     t.group = e.x;
@@ -176,10 +197,11 @@ __device__ __forceinline__ bool gemm_tile(const GemmParams& p, int t_tiles, long
 
 template <int MODE>
 __global__ void __launch_bounds__(GEMM_THREADS, 1)
-gemm_ws_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUtensorMap tm_x,
+gemm_ws_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ GemmXMaps tm_xs,
                const GemmParams p) {
   constexpr bool SWIGLU = MODE == GEMM_SWIGLU;
   constexpr bool HEAD = MODE == GEMM_HEAD;
+  const CUtensorMap& tm_x = tm_xs.box[0];
   extern __shared__ uint8_t smem_raw[];
   if (threadIdx.x == 0) GEMM_STAMP(0);   // CTA started
   // Control block, then 1024-byte aligned stages (the 128-byte swizzle repeats every 1024 B).
@@ -237,8 +259,7 @@ gemm_ws_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__
     if (gemm_tile(p, p.dense_t_tiles, blockIdx.x, t)) {   // the same for every lane
       prefetched = num_kb < S ? num_kb : S;
       if (ptx::elect_one()) {
-        const int nbox = (t.n + p.xbox - 1) / p.xbox;
-        const uint32_t tx = GEMM_WBYTES + (uint32_t)nbox * p.xbox * (GEMM_BK * 2);
+        const uint32_t tx = GEMM_WBYTES + (uint32_t)gemm_tile_cols(p, t.n) * (GEMM_BK * 2);
         const int wrow = t.group * p.w_rows_per_group + t.wt * GEMM_WTILE;
         for (int kb = 0; kb < prefetched; ++kb) {
           ptx::mbar_expect_tx(full_bar(kb), tx * KA);
@@ -313,8 +334,8 @@ gemm_ws_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__
       for (long long lin = blockIdx.x; ok; lin += gridDim.x) {
         GemmTile t;
         if (!gemm_tile(p, t_tiles, lin, t)) break;
-        const int nbox = (t.n + p.xbox - 1) / p.xbox;
-        const uint32_t tx = GEMM_WBYTES + (uint32_t)nbox * p.xbox * (GEMM_BK * 2);
+        const int cols = gemm_tile_cols(p, t.n);
+        const uint32_t tx = GEMM_WBYTES + (uint32_t)cols * (GEMM_BK * 2);
         const int wrow = t.group * p.w_rows_per_group + t.wt * (SWIGLU ? 64 : GEMM_WTILE);
         for (int kb = 0; kb < num_kb; ++kb, ++it, s = (s + 1 == S ? 0 : s + 1), ph ^= (s == 0)) {
           // the first tile's first `prefetched` stages were armed, and their weights requested, before pdl_wait
@@ -337,13 +358,24 @@ gemm_ws_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__
             } else {
               ptx::tma_load_2d(sw, &tm_w, full_bar(s), kcol, wrow, p.w_policy);
             }
-            for (int b = 0; b < nbox; ++b) {
-              if (p.batch_extra)
-                ptx::tma_load_3d(sx + (uint32_t)b * p.xbox * (GEMM_BK * 2), &tm_x, full_bar(s), kcol,
-                                 t.row0 + b * p.xbox, t.group, ptx::kEvictLast);
-              else
-                ptx::tma_load_2d(sx + (uint32_t)b * p.xbox * (GEMM_BK * 2), &tm_x, full_bar(s), kcol,
-                                 t.row0 + b * p.xbox, ptx::kEvictLast);
+            if (p.split_boxes) {
+              int at = 0;
+#pragma unroll
+              for (int i = 0; i < 5; ++i)
+                if (cols & (256 >> i)) {
+                  ptx::tma_load_2d(sx + (uint32_t)at * (GEMM_BK * 2), &tm_xs.box[i], full_bar(s), kcol, t.row0 + at,
+                                   ptx::kEvictLast);
+                  at += 256 >> i;
+                }
+            } else {
+              for (int at = 0; at < cols; at += p.xbox) {
+                if (p.batch_extra)
+                  ptx::tma_load_3d(sx + (uint32_t)at * (GEMM_BK * 2), &tm_x, full_bar(s), kcol, t.row0 + at, t.group,
+                                   ptx::kEvictLast);
+                else
+                  ptx::tma_load_2d(sx + (uint32_t)at * (GEMM_BK * 2), &tm_x, full_bar(s), kcol, t.row0 + at,
+                                   ptx::kEvictLast);
+              }
             }
           }
         }
@@ -359,9 +391,8 @@ gemm_ws_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__
         GemmTile t;
         if (!gemm_tile(p, t_tiles, lin, t)) break;
         const int buf = tile_it & 1;
-        const int nbox = (t.n + p.xbox - 1) / p.xbox;
-        const uint32_t idesc = p.fp16 ? ptx::umma_idesc_f16_m128((uint32_t)(nbox * p.xbox))
-                                      : ptx::umma_idesc_bf16_m128((uint32_t)(nbox * p.xbox));
+        const uint32_t cols = (uint32_t)gemm_tile_cols(p, t.n);
+        const uint32_t idesc = p.fp16 ? ptx::umma_idesc_f16_m128(cols) : ptx::umma_idesc_bf16_m128(cols);
         if (!ptx::mbar_wait(tempty_bar(buf), ((tile_it >> 1) & 1) ^ 1, abort_flag, 200 + buf)) break;
         ptx::tc_fence_after();
         const uint32_t d_tmem = tmem_base + (uint32_t)(buf * p.xrows_max);
@@ -696,7 +727,7 @@ inline int env_int(const char* name, int dflt) {
 }
 
 template <int MODE>
-inline int gemm_launch(const CUtensorMap& tw, const CUtensorMap& tx, GemmParams& p, long long max_tiles,
+inline int gemm_launch(const CUtensorMap& tw, const GemmXMaps& tx, GemmParams& p, long long max_tiles,
                        cudaStream_t st) {
   constexpr bool SWIGLU = MODE == GEMM_SWIGLU;
   static PerDeviceFlags attr_set;
@@ -934,6 +965,7 @@ inline int gemm_dense_16bit(const void* x, const void* w, const void* bias, void
   }
   p.tile_table = nullptr;
   p.tile_count = nullptr;
+  p.tokens_first = 1;
   p.xbox = p.rows_per_tile;
   p.xrows_max = p.rows_per_tile;
   p.out = out;
@@ -948,7 +980,8 @@ inline int gemm_dense_16bit(const void* x, const void* w, const void* bias, void
   p.gate = (const __nv_bfloat16*)ex.gate;
   p.gate_stride = ex.gate_row_stride;
   p.gate_batch_stride = ex.gate_batch_stride;
-  CUtensorMap tw, tx;
+  CUtensorMap tw;
+  GemmXMaps tx{};
   int rc;
   if (ex.batch > 1) {
     // the weights of all products form one 2-D view of whole rows, the activations a 3-D view [batch, T, K]
@@ -960,12 +993,12 @@ inline int gemm_dense_16bit(const void* x, const void* w, const void* bias, void
     rc = make_tmap_2d(&tw, w, (uint64_t)p.w_rows_per_group * (ex.batch - 1) + N, (uint64_t)K, (uint64_t)w_row_stride,
                       GEMM_WTILE);
     if (rc) return rc;
-    rc = make_tmap_3d(&tx, x, (uint64_t)ex.batch, (uint64_t)T, (uint64_t)K, (uint64_t)ex.x_batch_stride,
+    rc = make_tmap_3d(&tx.box[0], x, (uint64_t)ex.batch, (uint64_t)T, (uint64_t)K, (uint64_t)ex.x_batch_stride,
                       (uint64_t)x_row_stride, (uint32_t)p.xbox);
   } else {
     rc = make_tmap_2d(&tw, w, (uint64_t)N, (uint64_t)K, (uint64_t)w_row_stride, GEMM_WTILE, fp16);
     if (rc) return rc;
-    rc = make_tmap_2d(&tx, x, (uint64_t)T, (uint64_t)K, (uint64_t)x_row_stride, (uint32_t)p.xbox, fp16);
+    rc = make_tmap_2d(&tx.box[0], x, (uint64_t)T, (uint64_t)K, (uint64_t)x_row_stride, (uint32_t)p.xbox, fp16);
   }
   if (rc) return rc;
   return gemm_launch<GEMM_PLAIN>(tw, tx, p, (long long)p.w_tiles * p.dense_t_tiles * ex.batch, (cudaStream_t)stream);
@@ -1094,14 +1127,16 @@ extern "C" int b200_lm_head_greedy(const void* x, const void* w, void* partials,
       }
     }
   }
+  p.tokens_first = 1;
   p.xbox = p.rows_per_tile;
   p.xrows_max = p.rows_per_tile;
   p.head_part = (float4*)partials;
   p.w_policy = p.dense_t_tiles == 1 ? ptx::kEvictFirst : ptx::kEvictNormal;
-  CUtensorMap tw, tx;
+  CUtensorMap tw;
+  GemmXMaps tx{};
   int rc = make_tmap_2d(&tw, w, (uint64_t)V, (uint64_t)K, (uint64_t)w_row_stride, GEMM_WTILE);
   if (rc) return rc;
-  rc = make_tmap_2d(&tx, x, (uint64_t)T, (uint64_t)K, (uint64_t)x_row_stride, (uint32_t)p.xbox);
+  rc = make_tmap_2d(&tx.box[0], x, (uint64_t)T, (uint64_t)K, (uint64_t)x_row_stride, (uint32_t)p.xbox);
   if (rc) return rc;
   rc = gemm_launch<GEMM_HEAD>(tw, tx, p, (long long)p.w_tiles * p.dense_t_tiles, (cudaStream_t)stream);
   if (rc) return rc;
@@ -1144,6 +1179,10 @@ inline int moe_grouped_gemm_impl(const void* x, long long x_rows, long long x_ro
   // One activation box per stage when the tile height allows it (fewer TMA issues per stage).
   static const int xbox_env = env_int("B200_GEMM_XBOX", 64);
   p.xbox = (xbox_env == 16 || xbox_env == 32 || xbox_env == 64) && tile_rows_max % xbox_env == 0 ? xbox_env : 16;
+  // Tall tiles are for many rows per expert, where the rows no longer stay in L2 from one weight tile to the next: an
+  // expert's weight tiles run side by side over one token tile, so that both come from HBM once.
+  p.tokens_first = 0;
+  p.split_boxes = tile_rows_max > 64 && !gather_index;
   p.xrows_max = tile_rows_max;
   p.out = out;
   p.ldo = out_row_stride;
@@ -1155,12 +1194,19 @@ inline int moe_grouped_gemm_impl(const void* x, long long x_rows, long long x_ro
   p.scale_out = (const float*)scale_out;
   p.act = act;
   p.w_policy = ptx::kEvictFirst;
-  CUtensorMap tw, tx;
+  CUtensorMap tw;
+  GemmXMaps tx{};
   int rc = make_tmap_2d(&tw, w, (uint64_t)num_groups * p.w_rows_per_group, (uint64_t)K, (uint64_t)K,
                         mode == 1 ? 64 : GEMM_WTILE);
   if (rc) return rc;
-  rc = gather_index ? make_tmap_2d(&tx, x, (uint64_t)x_rows, (uint64_t)K, (uint64_t)x_row_stride, 1u)
-                    : make_tmap_2d(&tx, x, (uint64_t)x_rows, (uint64_t)K, (uint64_t)K, (uint32_t)p.xbox);
+  if (gather_index) {
+    rc = make_tmap_2d(&tx.box[0], x, (uint64_t)x_rows, (uint64_t)K, (uint64_t)x_row_stride, 1u);
+  } else if (p.split_boxes) {
+    for (int i = 0; i < 5 && !rc; ++i)
+      rc = make_tmap_2d(&tx.box[i], x, (uint64_t)x_rows, (uint64_t)K, (uint64_t)K, 256u >> i);
+  } else {
+    rc = make_tmap_2d(&tx.box[0], x, (uint64_t)x_rows, (uint64_t)K, (uint64_t)K, (uint32_t)p.xbox);
+  }
   if (rc) return rc;
   const long long tiles = (long long)max_tiles * p.w_tiles;
   if (mode == 1) return gemm_launch<GEMM_SWIGLU>(tw, tx, p, tiles, (cudaStream_t)stream);
@@ -1230,6 +1276,7 @@ extern "C" int b200_gemm_glu(const void* x, const void* w, const void* scale_out
   p.t_rows = (int)T;
   p.rows_per_tile = T <= 64 ? round_up((int)T, 16) : 64;
   p.dense_t_tiles = (int)((T + p.rows_per_tile - 1) / p.rows_per_tile);
+  p.tokens_first = 1;
   p.xbox = p.rows_per_tile;
   p.xrows_max = p.rows_per_tile;
   p.out = out;
@@ -1237,10 +1284,11 @@ extern "C" int b200_gemm_glu(const void* x, const void* w, const void* scale_out
   p.glu = act;
   p.scale_out = (const float*)scale_out_f32;
   p.w_policy = p.dense_t_tiles == 1 ? ptx::kEvictFirst : ptx::kEvictNormal;
-  CUtensorMap tw, tx;
+  CUtensorMap tw;
+  GemmXMaps tx{};
   int rc = make_tmap_2d(&tw, w, (uint64_t)2 * n_out, (uint64_t)K, (uint64_t)K, 64);
   if (rc) return rc;
-  rc = make_tmap_2d(&tx, x, (uint64_t)T, (uint64_t)K, (uint64_t)x_row_stride, (uint32_t)p.xbox);
+  rc = make_tmap_2d(&tx.box[0], x, (uint64_t)T, (uint64_t)K, (uint64_t)x_row_stride, (uint32_t)p.xbox);
   if (rc) return rc;
   return gemm_launch<GEMM_SWIGLU>(tw, tx, p, (long long)p.w_tiles * p.dense_t_tiles, (cudaStream_t)stream);
 }

@@ -432,7 +432,7 @@ moe_index_kernel(const TIdx* __restrict__ experts, long long n, int E, int tile_
       cu_seqlens[tid] = rexcl;
       for (int j = 0; j < tiles; ++j)
         if (texcl + j < max_tiles)
-          tile_table[texcl + j] = make_int4(tid, rexcl + j * tile_rows, min(tile_rows, rows - j * tile_rows), 0);
+          tile_table[texcl + j] = token_tile(tid, rexcl, rows, tiles, j);
       if (tid == E - 1) {
         cu_seqlens[E] = rexcl + rows;
         *tile_count = min(texcl + tiles, max_tiles);
@@ -883,6 +883,11 @@ transpose_last2_kernel(const uint16_t* __restrict__ x, uint16_t* __restrict__ ou
 }
 
 // h = bf16(bf16(bf16(silu(g)) * u) * s): the unfused tail of fc1 for split gate / up weights.
+//
+// HBM-bound: 2 reads and a write of 2 bytes per element, about 45 instructions for the exact exponential and division.  A
+// thread takes VEC elements of one row (VEC = 8: 16-byte loads and stores, one index division for the eight); VEC = 1 serves
+// widths, strides and bases that 16-byte accesses do not fit.
+template <int VEC>
 __global__ void __launch_bounds__(256)
 swiglu_scale_kernel(const __nv_bfloat16* __restrict__ gate, const __nv_bfloat16* __restrict__ up,
                     const __nv_bfloat16* __restrict__ row_scale, __nv_bfloat16* __restrict__ out, long long rows,
@@ -890,15 +895,30 @@ swiglu_scale_kernel(const __nv_bfloat16* __restrict__ gate, const __nv_bfloat16*
   pdl_trigger();
   pdl_wait();
   const long long i = (long long)blockIdx.x * 256 + threadIdx.x;
-  if (i >= rows * I) return;
-  const long long r = i / I;
-  const long long src = r * in_stride + (i - r * I);
-  const float g = bf2f(gate[src]);
-  const float u = bf2f(up[src]);
-  const float sg = round_bf(g / (1.0f + expf(-g)));
-  float h = round_bf(sg * u);
-  if (row_scale) h = round_bf(h * bf2f(row_scale[r]));
-  out[i] = f2bf(h);
+  const int per_row = I / VEC;
+  if (i >= rows * per_row) return;
+  const long long r = rows * per_row <= 0xffffffffLL ? (uint32_t)i / (uint32_t)per_row : i / per_row;
+  const long long c = (i - r * per_row) * VEC, src = r * in_stride + c;
+  const float s = row_scale ? bf2f(row_scale[r]) : 0.f;
+  auto one = [&](float g, float u) {
+    const float h = round_bf(round_bf(g / (1.0f + expf(-g))) * u);
+    return row_scale ? round_bf(h * s) : h;
+  };
+  if constexpr (VEC == 8) {
+    const uint4 gv = *reinterpret_cast<const uint4*>(gate + src), uv = *reinterpret_cast<const uint4*>(up + src);
+    const uint32_t g4[4] = {gv.x, gv.y, gv.z, gv.w}, u4[4] = {uv.x, uv.y, uv.z, uv.w};
+    uint32_t h4[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      float g0, g1, u0, u1;
+      unpack_bf2(g4[j], g0, g1);
+      unpack_bf2(u4[j], u0, u1);
+      h4[j] = pack_bf2(one(g0, u0), one(g1, u1));
+    }
+    *reinterpret_cast<uint4*>(out + r * I + c) = make_uint4(h4[0], h4[1], h4[2], h4[3]);
+  } else {
+    out[r * I + c] = f2bf(one(bf2f(gate[src]), bf2f(up[src])));
+  }
 }
 
 }  // namespace b200
@@ -1011,7 +1031,7 @@ moe_route_plan_kernel(const TIn* __restrict__ logits, long long row_stride, __nv
     cu_seqlens[e] = rexcl;
     for (int j = 0; j < tiles; ++j)
       if (texcl + j < max_tiles)
-        tile_table[texcl + j] = make_int4(e, rexcl + j * tile_rows, min(tile_rows, rows - j * tile_rows), 0);
+        tile_table[texcl + j] = token_tile(e, rexcl, rows, tiles, j);
     if (e == E - 1) {
       cu_seqlens[E] = rexcl + rows;
       *tile_count = min(texcl + tiles, max_tiles);
@@ -1363,10 +1383,13 @@ extern "C" int b200_swiglu_scale_strided(const void* gate, const void* up, const
   using namespace b200;
   if (!gate || !up || !out || rows < 0 || I <= 0 || in_row_stride < I) return B200_ERR_ARG;
   if (rows == 0) return B200_OK;
-  const long long n = rows * I;
-  launch_k(swiglu_scale_kernel, dim3((unsigned)((n + 255) / 256)), dim3(256), 0, (cudaStream_t)stream,
-           (const __nv_bfloat16*)gate, (const __nv_bfloat16*)up, (const __nv_bfloat16*)row_scale, (__nv_bfloat16*)out,
-           rows, I, in_row_stride);
+  const bool vec = I % 8 == 0 && in_row_stride % 8 == 0 &&
+                   ((reinterpret_cast<uintptr_t>(gate) | reinterpret_cast<uintptr_t>(up) | reinterpret_cast<uintptr_t>(out)) & 15) == 0;
+  const long long blocks = (rows * (vec ? I / 8 : I) + 255) / 256;
+  if (blocks > 0x7fffffffLL) return B200_ERR_SHAPE;
+  launch_k(vec ? swiglu_scale_kernel<8> : swiglu_scale_kernel<1>, dim3((unsigned)blocks), dim3(256), 0,
+           (cudaStream_t)stream, (const __nv_bfloat16*)gate, (const __nv_bfloat16*)up, (const __nv_bfloat16*)row_scale,
+           (__nv_bfloat16*)out, rows, I, in_row_stride);
   return launch_status();
 }
 

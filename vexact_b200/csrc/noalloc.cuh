@@ -88,7 +88,7 @@ tiles_from_cu_seqlens_kernel(const int* __restrict__ cu_seqlens, int num_groups,
     const int t0 = first_tile[g];
     for (int j = 0; j < tiles; ++j)
       if (t0 + j < max_tiles)
-        table[1 + t0 + j] = make_int4(g, r0 + j * tile_rows, min(tile_rows, rows - j * tile_rows), 0);
+        table[1 + t0 + j] = token_tile(g, r0, rows, tiles, j);
   }
 }
 
@@ -109,9 +109,9 @@ extern "C" int b200_moe_grouped_gemm_noalloc(const void* x, const void* w, const
   if (!x || !w || !out || !cu_seqlens || x_rows < 0 || num_groups <= 0 || n_out <= 0 || K <= 0 ||
       (mode != 0 && mode != 1))
     return B200_ERR_ARG;
-  constexpr int kTileRows = 64;
   if (num_groups > NOALLOC_MAX_GROUPS) return B200_ERR_SHAPE;
-  const long long bound = (long long)num_groups + x_rows / kTileRows;
+  const int tile_rows = mode == 0 ? grouped_tile_rows(x_rows, num_groups) : 64;
+  const long long bound = (long long)num_groups + x_rows / 64;
   if (bound > NOALLOC_MAX_TILES) return B200_ERR_SHAPE;
   if (x_rows == 0) return B200_OK;
   int4* table = nullptr;
@@ -119,10 +119,10 @@ extern "C" int b200_moe_grouped_gemm_noalloc(const void* x, const void* w, const
   if (rc) return rc;
   cudaStream_t st = (cudaStream_t)stream;
   if (x_rows > 0x7fffffffLL) return B200_ERR_SHAPE;
-  tiles_from_cu_seqlens_kernel<<<1, 1024, 0, st>>>((const int*)cu_seqlens, num_groups, kTileRows, table,
+  tiles_from_cu_seqlens_kernel<<<1, 1024, 0, st>>>((const int*)cu_seqlens, num_groups, tile_rows, table,
                                                    NOALLOC_MAX_TILES, (int)x_rows);
   rc = launch_status();
   if (rc) return rc;
   return b200_moe_grouped_gemm(x, w, row_scale, out, table + 1, table, x_rows, num_groups, n_out, K,
-                               out_row_stride, (int)bound, kTileRows, mode, stream);
+                               out_row_stride, (int)(num_groups + x_rows / tile_rows), tile_rows, mode, stream);
 }
