@@ -451,6 +451,8 @@ def _eager_packed(q, k, v, scale):
     ([65, 129], [65, 129], 4, 2, 128, 128),     # full causal prefill, tiles with ragged edges
     ([9, 23], [41, 57], 6, 3, 40, 40),          # a head dim the kernels do not tile (zero columns)
     ([5, 40], [33, 40], 4, 4, 192, 128),        # MLA dims
+    ([1, 128, 257], [700, 129, 257], 8, 1, 128, 128),   # one query, owned tiles with one row over, a long context
+    ([130, 64], [130, 511], 4, 2, 192, 128),    # owned and streamed tiles with remainders, MLA dims
 ])
 def test_packed_varlen_backward_matches_autograd_of_fp32_attention(vb, q_lens, kv_lens, hq, hkv, dk, dv):
     """dq, dk, dv of the packed call (reference kernels: triton_invariant_attention.py:194-431; reference tests:
@@ -498,7 +500,7 @@ def test_packed_varlen_backward_matches_autograd_of_fp32_attention(vb, q_lens, k
 
 
 def test_packed_varlen_backward_tensor_core_and_cuda_core_forms_agree(vb, tmp_path):
-    """The default backward runs on the tensor cores (mma.sync); B200_ATTN_BWD_SIMT=1 selects the CUDA-core kernels
+    """The default backward runs on the tensor cores; B200_ATTN_BWD_SIMT=1 selects the CUDA-core kernels
     (read once per process, hence the child process).  Same rounding points, different summation order inside a
     16-wide step: the two agree to 2^-6 of each gradient's largest magnitude."""
     import subprocess
@@ -533,3 +535,24 @@ torch.save([q.grad.cpu(), k.grad.cpu(), v.grad.cpu()], sys.argv[1])
         grads[form] = torch.load(path)
     for a, b in zip(grads["mma"], grads["simt"]):
         torch.testing.assert_close(a.float(), b.float(), rtol=0, atol=2 ** -6 * b.float().abs().max().item())
+
+
+def test_packed_varlen_backward_keeps_to_its_sequence(vb):
+    """The tensor-core backward streams 64-row tiles that reach past a sequence's end; what lies there (here infinities and
+    NaN of the next sequence) stays out of this sequence's gradients."""
+    g = torch.Generator().manual_seed(9)
+    lens, hq, hkv, d = [70, 40], 4, 2, 128
+    q, k, v, dout = (torch.randn(sum(lens), h, d, generator=g).to(BF).cuda() for h in (hq, hkv, hkv, hq))
+    cu = torch.tensor([0, 70, 110], dtype=torch.int32).cuda()
+
+    def run(q, k, v, dout, cu):
+        leaves = [t.clone().requires_grad_(True) for t in (q, k, v)]
+        out, _ = vb.flash_attn_varlen_func(*leaves, cu, cu, max_seqlen_q=70, max_seqlen_k=70, causal=True)
+        return torch.autograd.grad(out, leaves, dout)
+
+    alone = run(q[:70], k[:70], v[:70], dout[:70], cu[:2])
+    for t in (q, k, v, dout):
+        t[70::2] = float("nan")
+        t[71::2] = float("inf")
+    for a, b in zip(alone, run(q, k, v, dout, cu)):
+        assert torch.equal(a, b[:70])
