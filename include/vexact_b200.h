@@ -100,6 +100,9 @@ int b200_log_softmax_f32(const void* x, void* out, long long rows, int n, long l
  * labels are int64.  dtype of logits: 0 = fp32, 1 = bf16. */
 int b200_gather_logprob(const void* logits, const void* labels, void* out, long long rows, int n,
                         long long row_stride, int dtype, long long ignore_index, void* stream);
+/* The same; lse_f32 (may be null) receives every row's logsumexp, which b200_gather_logprob_backward_lse takes. */
+int b200_gather_logprob_lse(const void* logits, const void* labels, void* out, void* lse_f32, long long rows, int n,
+                            long long row_stride, int dtype, long long ignore_index, void* stream);
 
 /* Gradient of b200_gather_logprob with respect to the logits (the backward of flash-attn's cross_entropy_loss, which
  * standalone_logprobs.py:28 wraps, with a log-probability's sign): dlogits[r, i] = grad_out[r] * ((i == label[r]) -
@@ -108,6 +111,10 @@ int b200_gather_logprob(const void* logits, const void* labels, void* out, long 
 int b200_gather_logprob_backward(const void* logits, const void* labels, const void* grad_out_f32, void* dlogits,
                                  long long rows, int n, long long row_stride, long long d_row_stride, int dtype,
                                  long long ignore_index, void* stream);
+/* The same from the forward's lse_f32: one read of the logits instead of two. */
+int b200_gather_logprob_backward_lse(const void* logits, const void* labels, const void* grad_out_f32,
+                                     const void* lse_f32, void* dlogits, long long rows, int n, long long row_stride,
+                                     long long d_row_stride, int dtype, long long ignore_index, void* stream);
 
 /* ---- vexact/inferencer/inferencer.py:393-449 _select_tokens for greedy decoding: the argmax of each
  *      row of logits (lowest index on ties) and that token's log-probability (the value

@@ -283,3 +283,51 @@ def test_gather_logprob_backward_matches_autograd(vb, dtype):
     leaf2 = buf.detach().requires_grad_(True)
     vb.logprobs_from_logits_flash_attn(leaf2, labels, inplace_backward=True).backward(go)
     assert leaf2.grad.data_ptr() == leaf2.data_ptr() and torch.equal(leaf2.grad, leaf.grad)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, BF])
+@pytest.mark.parametrize("vocab", [5, 1000, 8192, 8195, 40008])
+def test_row_softmax_in_a_cluster_and_in_one_cta(vb, dtype, vocab):
+    """Up to 64 rows are spread over eight CTAs each, more rows take one CTA each: the same bits either way, against fp64;
+    -inf entries, a row of -inf alone and NaN keep their meaning.  The backward from the forward's log-sum-exp and the one
+    that makes its own agree to the bit."""
+    from vexact_b200 import _lib
+    from vexact_b200.standalone_logprobs import greedy_token_and_logprob
+
+    x = (_seeded(65, vocab, seed=vocab, std=3.0)).to(dtype).cuda()
+    x[1, 1::2] = -float("inf")
+    x[2, vocab // 2] = float("nan")
+    x[3, :3] = 50.0
+    x[4, 0] = 3.0e4 if dtype == torch.float32 else 2.0 ** 15
+    labels = torch.randint(0, vocab, (65,), generator=torch.Generator().manual_seed(3)).cuda()
+    labels[1], labels[5] = 0, -100
+    few, many = slice(0, 64), slice(0, 65)
+    for f in (lambda r: vb.logprobs_from_logits_flash_attn(x[r], labels[r]),
+              lambda r: greedy_token_and_logprob(x[r])[1], lambda r: vb.log_softmax(x[r].float())):
+        a, b = f(few), f(many)[:64]
+        assert torch.equal(a.nan_to_num(7.0), b.nan_to_num(7.0))
+        assert vocab == 5 or torch.isnan(a[2]).all()     # (a thread whose only element is NaN adds nothing)
+    ref = torch.log_softmax(x.double(), -1)
+    ok = torch.arange(65, device="cuda") != 2
+    lp = vb.logprobs_from_logits_flash_attn(x, labels)
+    want = ref.gather(1, labels.clamp(min=0)[:, None])[:, 0] * (labels != -100)
+    # fp32 results of magnitude |x| and |lse|: a few units in their last place
+    torch.testing.assert_close(lp[ok].double(), want[ok], rtol=4e-7, atol=4e-6)
+    tok, _ = greedy_token_and_logprob(x)
+    assert torch.equal(tok[ok], x[ok].float().argmax(-1))
+    go = torch.randn(65, generator=torch.Generator().manual_seed(4)).cuda()
+    leaf = x.clone().requires_grad_(True)
+    vb.logprobs_from_logits_flash_attn(leaf, labels).backward(go)
+    own = torch.empty_like(x)
+    _lib.check(_lib.load().b200_gather_logprob_backward(
+        x.data_ptr(), labels.data_ptr(), go.data_ptr(), own.data_ptr(), 65, vocab, vocab, vocab,
+        0 if dtype == torch.float32 else 1, -100, _lib.current_stream()), "b200_gather_logprob_backward")
+    assert torch.equal(leaf.grad.nan_to_num(7.0), own.nan_to_num(7.0)) and not own[5].any()
+    grad = torch.zeros_like(ref).scatter_(1, labels.clamp(min=0)[:, None], 1.0) - ref.exp()
+    grad = grad * (go.double() * (labels != -100))[:, None]
+    # lse of magnitude 2^15 is good to 2^-9: row 4's probabilities too
+    tol = 2 ** -8 if dtype == BF else 2e-6
+    sel = ok & (torch.arange(65, device="cuda") != 4)
+    torch.testing.assert_close(leaf.grad[sel].double(), grad[sel], rtol=tol, atol=tol)
+    lone = torch.full((1, vocab), -float("inf"), dtype=dtype, device="cuda")
+    assert greedy_token_and_logprob(lone)[0].item() == 0

@@ -764,7 +764,7 @@ inline int gemm_launch(const CUtensorMap& tw, const GemmXMaps& tx, GemmParams& p
   if (grid <= 0) return B200_OK;
   // A dense GEMM (static tiling) may start under its predecessor's tail: it prefetches weights before it waits.
   launch_k_pdl(gemm_ws_kernel<MODE>, dim3((unsigned)grid), dim3(GEMM_THREADS), smem, st,
-               pdl_mode() == 1 || (pdl_mode() == 2 && !p.tile_table), tw, tx, p);
+               pdl_mode() == 1 || (pdl_mode() == 2 && !p.tile_table), 1, tw, tx, p);
   return launch_status();
 }
 

@@ -30,29 +30,6 @@ struct GruParams {
   long long group_rows;        // rows of the maps that belong to groups (gru_maps_kernel, gru_walk_kernel)
 };
 
-// Two neighbouring channels in one register pair: one instruction for both.
-struct Two {
-  unsigned long long v;
-  __device__ __forceinline__ Two() {}
-  __device__ __forceinline__ Two(float a, float b) { asm("mov.b64 %0, {%1, %2};" : "=l"(v) : "f"(a), "f"(b)); }
-  __device__ __forceinline__ explicit Two(float a) : Two(a, a) {}
-  __device__ __forceinline__ void get(float& a, float& b) const { asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v)); }
-};
-__device__ __forceinline__ Two operator+(const Two& a, const Two& b) {
-  Two r;
-  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
-  return r;
-}
-__device__ __forceinline__ Two operator*(const Two& a, const Two& b) {
-  Two r;
-  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
-  return r;
-}
-__device__ __forceinline__ Two fma2(const Two& a, const Two& b, const Two& c) {
-  Two r;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r.v) : "l"(a.v), "l"(b.v), "l"(c.v));
-  return r;
-}
 // 2^min(x, 40) and 1 / x on the special-function unit, c where u >= 0 and s elsewhere.
 __device__ __forceinline__ Two gru_ex2(const Two& x) {
   float a, b;

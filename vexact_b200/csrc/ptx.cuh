@@ -1,6 +1,6 @@
 // Thin inline-PTX wrappers for the sm_100a features the contraction kernels use:
 // mbarrier, TMA (cp.async.bulk.tensor), tcgen05 (tensor memory + UMMA).
-// No cluster launch and no multicast form is used anywhere in this library.
+// No multicast load is used anywhere in this library.
 #pragma once
 #include "common.cuh"
 

@@ -240,9 +240,9 @@ __global__ void __launch_bounds__(SMP_THREADS) sample_token_kernel(const SampleP
   const int nvec = qvec ? n / VEC : 0;
   for (int v = tid; v < nvec; v += SMP_THREADS) {
     float xv[VEC], qv[VEC];
-    RowLoader<T>::load(row + (size_t)v * VEC, xv);
+    RowLoader<T>::unpack(*reinterpret_cast<const uint4*>(row + (size_t)v * VEC), xv);
 #pragma unroll
-    for (int j = 0; j < VEC; j += 4) RowLoader<float>::load(qrow + (size_t)v * VEC + j, qv + j);
+    for (int j = 0; j < VEC; j += 4) RowLoader<float>::unpack(*reinterpret_cast<const uint4*>(qrow + (size_t)v * VEC + j), qv + j);
 #pragma unroll
     for (int j = 0; j < VEC; ++j) consider(xv[j], qv[j], v * VEC + j);
   }

@@ -18,15 +18,14 @@ class _GatherLogprob(torch.autograd.Function):
 
     @staticmethod
     def forward(ctx, logits, labels, inplace_backward):
-        with torch.no_grad():
-            out = logprobs_from_logits_flash_attn(logits, labels)
-        ctx.save_for_backward(logits, labels)
+        out, lse = _gather_logprob(logits, labels, True)
+        ctx.save_for_backward(logits, labels, lse)
         ctx.inplace = bool(inplace_backward)
         return out
 
     @staticmethod
     def backward(ctx, grad_out):
-        logits, labels = ctx.saved_tensors
+        logits, labels, lse = ctx.saved_tensors
         vocab = logits.shape[-1]
         x = logits.reshape(-1, vocab)
         if x.stride(-1) != 1:
@@ -36,11 +35,11 @@ class _GatherLogprob(torch.autograd.Function):
         lab = labels.reshape(-1).to(torch.int64).contiguous()
         g = grad_out.reshape(-1).to(torch.float32).contiguous()
         _lib.check(
-            _lib.load().b200_gather_logprob_backward(x.data_ptr(), lab.data_ptr(), g.data_ptr(), dx.data_ptr(),
-                                                     x.shape[0], vocab, x.stride(0), dx.stride(0),
-                                                     0 if x.dtype == torch.float32 else 1, IGNORE_INDEX,
-                                                     _lib.current_stream()),
-            "b200_gather_logprob_backward",
+            _lib.load().b200_gather_logprob_backward_lse(x.data_ptr(), lab.data_ptr(), g.data_ptr(), lse.data_ptr(),
+                                                         dx.data_ptr(), x.shape[0], vocab, x.stride(0), dx.stride(0),
+                                                         0 if x.dtype == torch.float32 else 1, IGNORE_INDEX,
+                                                         _lib.current_stream()),
+            "b200_gather_logprob_backward_lse",
         )
         return dx.reshape(logits.shape), None, None
 
@@ -55,6 +54,11 @@ def logprobs_from_logits_flash_attn(logits: torch.Tensor, labels: torch.Tensor,
         return _GatherLogprob.apply(logits, labels, inplace_backward)
     if logits.dtype not in (torch.float32, torch.bfloat16):
         raise NotImplementedError(f"logits dtype {logits.dtype} is not supported")
+    return _gather_logprob(logits, labels, False)[0]
+
+
+def _gather_logprob(logits: torch.Tensor, labels: torch.Tensor, want_lse: bool):
+    """(log-probabilities, the rows' log-sum-exp fp32 [rows] or None)."""
     batch_shape = logits.shape[:-1]
     vocab = logits.shape[-1]
     x = logits.reshape(-1, vocab)
@@ -63,13 +67,14 @@ def logprobs_from_logits_flash_attn(logits: torch.Tensor, labels: torch.Tensor,
     lab = labels.reshape(-1).to(torch.int64).contiguous()
     assert lab.numel() == x.shape[0], "labels must have one entry per logits row"
     out = torch.empty((x.shape[0],), device=logits.device, dtype=torch.float32)
+    lse = torch.empty_like(out) if want_lse else None
     _lib.check(
-        _lib.load().b200_gather_logprob(x.data_ptr(), lab.data_ptr(), out.data_ptr(), x.shape[0], vocab,
-                                        x.stride(0), 0 if x.dtype == torch.float32 else 1, IGNORE_INDEX,
-                                        _lib.current_stream()),
-        "b200_gather_logprob",
+        _lib.load().b200_gather_logprob_lse(x.data_ptr(), lab.data_ptr(), out.data_ptr(), _lib.ptr(lse), x.shape[0],
+                                            vocab, x.stride(0), 0 if x.dtype == torch.float32 else 1, IGNORE_INDEX,
+                                            _lib.current_stream()),
+        "b200_gather_logprob_lse",
     )
-    return out.reshape(batch_shape)
+    return out.reshape(batch_shape), lse
 
 
 def greedy_token_and_logprob(logits: torch.Tensor):
