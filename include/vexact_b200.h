@@ -337,6 +337,22 @@ int b200_moe_grouped_gemm_noalloc(const void* x, const void* w, const void* row_
                                   const void* cu_seqlens, long long x_rows, int num_groups, int n_out, int K,
                                   long long out_row_stride, int mode, void* stream);
 
+/* ---- vexact/batch_invariant_ops/group_gemm/kernel/group_gemm.py:156 group_gemm_same_nk(transpose_b=False), the data
+ *      gradient: out[r, n] = sum_k x[r, k] * w[g(r), k, n] with w [num_groups, K, n_out] as a forward weight lies.  With w2
+ *      (may be null) w and w2 are [num_groups, K / 2, n_out], k below and from K / 2 on; K is then a multiple of 128.  n_out a
+ *      multiple of 8.  The noalloc form takes cu_seqlens as b200_moe_grouped_gemm_noalloc does. */
+int b200_moe_grouped_dgrad(const void* x, const void* w, const void* w2, void* out, const void* tile_table,
+                           const void* tile_count, long long x_rows, int num_groups, int n_out, int K,
+                           long long out_row_stride, int max_tiles, int tile_rows_max, void* stream);
+int b200_moe_grouped_dgrad_noalloc(const void* x, const void* w, void* out, const void* cu_seqlens, long long x_rows,
+                                   int num_groups, int n_out, int K, long long out_row_stride, void* stream);
+
+/* ---- vexact/batch_invariant_ops/fused_moe.py:113-236: the backward of b200_swiglu_scale with the rounding points of the
+ *      chain of torch operators there; also writes what fc2 consumed (h_scaled) and the rows' gradient of the scale. */
+int b200_swiglu_backward(const void* gate, const void* up, long long in_row_stride, const void* d_h, const void* row_scale,
+                         void* h_scaled, void* d_gate, void* d_up, long long d_row_stride, void* d_scale, long long rows,
+                         int I, void* stream);
+
 /* ---- vexact/batch_invariant_ops/fused_moe.py:325-336 for split gate / up weights. */
 int b200_swiglu_scale(const void* gate, const void* up, const void* row_scale, void* out, long long rows,
                       int I, void* stream);
@@ -365,18 +381,19 @@ int b200_moe_gather(const void* x, long long x_rows, const void* index_i32, long
                     long long index_stride_k, void* out, long long T, int topk, int H, void* stream);
 
 /* No counterpart in the reference (its Triton GEMM reads either layout): out[g, c, r] = x[g, r, c] for 2-byte
- * elements, x [G, R, C] and out [G, C, R] contiguous, R and C multiples of 8, 16-byte aligned.  Used to hand the
- * expert weights to the dgrad form of the grouped GEMM (group_gemm.py:156 with transpose_b=False). */
+ * elements, x [G, R, C] and out [G, C, R] contiguous, R and C multiples of 8, 16-byte aligned. */
 int b200_transpose_last2(const void* x, void* out, int G, int R, int C, void* stream);
 
 /* ---- vexact/batch_invariant_ops/group_gemm/kernel/group_gemm.py:360 group_gemm_same_mn(transpose_a=True): the
  *      weight gradient of a grouped GEMM, c[g] = a[rows of g]^T @ b[rows of g] with the rows of group g being
  *      [cu_seqlens[g], cu_seqlens[g + 1]).  a [rows, M], b [rows, N], c [num_groups, M, N], all bf16 contiguous;
  *      fp32 accumulation in ascending row order, one rounding; an empty group gets zeros.  M, N multiples of 4.
- *      A training-side operator: mma.sync tensor-core kernel when M and N are multiples of 8 and the pointers
- *      16-byte aligned (sum over 16-row steps in ascending order), a CUDA-core kernel otherwise. */
+ *      tcgen05 when M and N are multiples of 8 and the pointers 16-byte aligned (sum over 16-row steps in ascending
+ *      order), a CUDA-core kernel otherwise.  The strided form takes rows of a and b that far apart (multiples of 8). */
 int b200_moe_grouped_wgrad(const void* a, const void* b, void* c, const void* cu_seqlens, long long rows,
                            int num_groups, int M, int N, void* stream);
+int b200_moe_grouped_wgrad_strided(const void* a, long long a_row_stride, const void* b, long long b_row_stride, void* c,
+                                   const void* cu_seqlens, long long rows, int num_groups, int M, int N, void* stream);
 
 /* b200_moe_unpermute_reduce followed by b200_add_rmsnorm (the residual add and input RMSNorm the next
  * decoder layer starts with) in one launch, with that pair's arithmetic element for element:

@@ -527,3 +527,76 @@ def test_grouped_gemm_tile_heights_and_unfused_swiglu(vb, E, k, T, H, I):
         assert torch.equal(h, fused)
     torch.cuda.synchronize()
     assert vb._lib.read_status()[0] == 0
+
+
+@pytest.mark.parametrize("M, N", [(8, 8), (128, 256), (136, 264), (200, 520), (768, 64)])
+def test_grouped_weight_gradient_edges(M, N):
+    """Groups of every length around the 16 rows of an instruction and the 64 of a step, empty ones between them; a group's
+    NaN and infinities stay its own; rows of the operands may lie apart."""
+    from vexact_b200 import _lib
+
+    lens = [0, 1, 15, 16, 17, 0, 63, 64, 65, 200, 5, 0]
+    cu = torch.tensor([0, *torch.tensor(lens).cumsum(0)], dtype=torch.int32, device="cuda")
+    R, G = sum(lens), len(lens)
+    gen = torch.Generator(device="cuda").manual_seed(M + N)
+    wide = torch.randn(R, 2 * M, device="cuda", generator=gen).to(BF)
+    a, b = wide[:, M:], torch.randn(R, N, device="cuda", generator=gen).to(BF)
+    bad = 10                                             # the group of five rows
+    wide[cu[bad]:cu[bad + 1]] = float("nan")
+    b[cu[bad]:cu[bad + 1]] = float("inf")
+
+    def run():
+        c = torch.full((G, M, N), 7.0, dtype=BF, device="cuda")
+        _lib.check(_lib.load().b200_moe_grouped_wgrad_strided(a.data_ptr(), a.stride(0), b.data_ptr(), b.stride(0), c.data_ptr(),
+                                                              cu.data_ptr(), R, G, M, N, _lib.current_stream()), "wgrad")
+        return c
+
+    c = run()
+    for g, n in enumerate(lens):
+        if g == bad:
+            assert torch.isnan(c[g]).all()
+            continue
+        s = slice(int(cu[g]), int(cu[g + 1]))
+        ref = a[s].double().t() @ b[s].double()
+        # one rounding to bf16 of an fp32 sum of n products of order 1
+        torch.testing.assert_close(c[g].double(), ref, rtol=2 ** -8, atol=1e-6 * max(n, 1))
+    assert torch.equal(c.nan_to_num(3.0), run().nan_to_num(3.0))
+
+
+@pytest.mark.parametrize("K, N", [(64, 8), (72, 136), (192, 128), (768, 520)])
+@pytest.mark.parametrize("tokens", [3, 130, 700])
+def test_grouped_data_gradient_reads_weights_as_they_lie(K, N, tokens):
+    """out = x @ w[g] with w [groups, K, N]: the bits of the forward form on the transposed weights, and both halves of a
+    product in one accumulation when they come from two tensors."""
+    from vexact_b200 import _lib, group_gemm as gg
+    from vexact_b200.fused_moe import _permute
+
+    E, k = 5, 2
+    gen = torch.Generator(device="cuda").manual_seed(K + N + tokens)
+    sel = torch.randint(0, E, (tokens, k), device="cuda", generator=gen)
+    plan = _permute(sel, None, None, E)
+    ends, R = plan["cu_seqlens"][1:], tokens * k
+    x = torch.randn(R, K, device="cuda", generator=gen).to(BF)
+    w = torch.randn(E, K, N, device="cuda", generator=gen).to(BF)
+    out = gg.group_gemm_same_nk(x, w, ends, R, transpose_b=False)
+    assert torch.equal(out, gg.group_gemm_same_nk(x, w.transpose(1, 2).contiguous(), ends, R, transpose_b=True))
+    cu = plan["cu_seqlens"].tolist()
+    ref = torch.cat([x[cu[e]:cu[e + 1]].double() @ w[e].double() for e in range(E)])
+    tol = dict(rtol=2 ** -8, atol=1e-6 * K)
+    torch.testing.assert_close(out.double(), ref, **tol)
+    if K % 64:
+        return
+    x2 = torch.randn(R, 2 * K, device="cuda", generator=gen).to(BF)
+    w2 = torch.randn(E, K, N, device="cuda", generator=gen).to(BF)
+
+    def product(a, first, second):
+        y = torch.empty(R, N, dtype=BF, device="cuda")
+        _lib.check(_lib.load().b200_moe_grouped_dgrad(
+            a.data_ptr(), first.data_ptr(), _lib.ptr(second), y.data_ptr(), plan["tile_table"].data_ptr(),
+            plan["tile_count"].data_ptr(), R, E, N, a.shape[1], y.stride(0), plan["max_tiles"], plan["tile_rows"],
+            _lib.current_stream()), "dgrad")
+        return y
+
+    assert torch.equal(product(x2, w, w2), product(x2, torch.cat([w, w2], 1), None))
+    ref = torch.cat([x2[cu[e]:cu[e + 1]].double() @ torch.cat([w[e], w2[e]]).double() for e in range(E)])
+    torch.testing.assert_close(product(x2, w, w2).double(), ref, **tol)

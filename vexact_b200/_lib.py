@@ -97,7 +97,11 @@ SIGNATURES = {
     "b200_moe_unpermute_reduce": [P, P, P, P, LL, I, I, P],
     "b200_moe_scatter": [P, LL, P, LL, LL, P, LL, LL, I, I, P],
     "b200_moe_gather": [P, LL, P, LL, LL, P, LL, I, I, P],
+    "b200_moe_grouped_dgrad": [P, P, P, P, P, P, LL, I, I, I, LL, I, I, P],
+    "b200_moe_grouped_dgrad_noalloc": [P, P, P, P, LL, I, I, I, LL, P],
+    "b200_swiglu_backward": [P, P, LL, P, P, P, P, P, LL, P, LL, I, P],
     "b200_moe_grouped_wgrad": [P, P, P, P, LL, I, I, I, P],
+    "b200_moe_grouped_wgrad_strided": [P, LL, P, LL, P, P, LL, I, I, I, P],
     "b200_transpose_last2": [P, P, I, I, I, P],
     "b200_varlen_attn_backward": [P, P, P, P, P, P, P, P, P, P, P, P, I, I, I, LL, LL, I, I, I, I, F, P],
     "b200_moe_unpermute_add_rmsnorm": [P, P, P, P, P, P, P, LL, I, I, F, I, P],

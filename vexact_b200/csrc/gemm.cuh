@@ -64,6 +64,10 @@ struct GemmParams {
   int scalar_epilogue;  // development knob B200_GEMM_EPI_SCALAR=1: 2-byte stores in the plain epilogue
   const int* tile_count;
   int tokens_first;  // tile order: a weight tile's token tiles one after the other (1), or a token tile's weight tiles (0)
+  // Data gradient (grouped plain mode): the weights lie with the features contiguous, [groups, k, features], and are read
+  // MN-major through 3-D maps, two boxes of 64 k rows x 64 features per atom.  K steps from k_second on come from a second
+  // tensor of the same shape (0: there is none).
+  int k_second;
   int split_boxes;   // activation boxes by the binary digits of a tile's height instead of p.xbox rows each
   int xbox;       // rows per activation TMA box (multiple of 16)
   int xrows_max;  // largest token count of any tile (multiple of xbox, <= 256)
@@ -99,6 +103,8 @@ constexpr int GEMM_PLAIN = 0;   // out = acc (+ bias)
 constexpr int GEMM_SWIGLU = 1;  // gate / up rows stacked on M, out = silu(gate) * up * row_scale
 constexpr int GEMM_HEAD = 2;    // lm_head: no logits are stored; per (token, weight tile) the maximum, the sum of
                                 // exp(x - max) and the arg-max of the tile's 128 bf16-rounded logits
+constexpr int GEMM_DGRAD = 3;   // GEMM_PLAIN with MN-major weights (a mode of its own: with few tokens the loops that issue
+                                // copies and products bound the kernel, and a test in them costs decode steps up to 10 %)
 constexpr float kLog2e = 1.4426950408889634f;
 
 // Activations of the plain epilogue, applied in fp32 before the one rounding to the output type.
@@ -159,6 +165,7 @@ struct GemmTile {
 // 64 / 32 / 16 rows made fc1 of 4096 tokens (128 experts, 2048 -> 1536) 260 / 297 / 393 us.
 struct GemmXMaps {
   CUtensorMap box[5];
+  CUtensorMap w2;      // p.k_second
 };
 
 // Token columns that a tile of n rows occupies in shared and tensor memory.
@@ -200,7 +207,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
 gemm_ws_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ GemmXMaps tm_xs,
                const GemmParams p) {
   constexpr bool SWIGLU = MODE == GEMM_SWIGLU;
-  constexpr bool HEAD = MODE == GEMM_HEAD;
+  constexpr bool HEAD = MODE == GEMM_HEAD, W_MN = MODE == GEMM_DGRAD;
   const CUtensorMap& tm_x = tm_xs.box[0];
   extern __shared__ uint8_t smem_raw[];
   if (threadIdx.x == 0) GEMM_STAMP(0);   // CTA started
@@ -352,6 +359,12 @@ gemm_ws_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__
             const uint32_t sx = sw + GEMM_WBYTES;
             const int kcol = (kb * KA + a) * GEMM_BK;
             if (early) {
+            } else if (W_MN) {
+              const bool second = p.k_second && kcol >= p.k_second;
+#pragma unroll
+              for (int h = 0; h < 2; ++h)
+                ptx::tma_load_3d(sw + h * (GEMM_WBYTES / 2), second ? &tm_xs.w2 : &tm_w, full_bar(s), t.wt * GEMM_WTILE + h * 64,
+                                 second ? kcol - p.k_second : kcol, t.group, p.w_policy);
             } else if (SWIGLU) {
               ptx::tma_load_2d(sw, &tm_w, full_bar(s), kcol, wrow, p.w_policy);
               ptx::tma_load_2d(sw + 64 * GEMM_BK * 2, &tm_w, full_bar(s), kcol, wrow + p.up_offset, p.w_policy);
@@ -392,7 +405,10 @@ gemm_ws_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__
         if (!gemm_tile(p, t_tiles, lin, t)) break;
         const int buf = tile_it & 1;
         const uint32_t cols = (uint32_t)gemm_tile_cols(p, t.n);
-        const uint32_t idesc = p.fp16 ? ptx::umma_idesc_f16_m128(cols) : ptx::umma_idesc_bf16_m128(cols);
+        const uint32_t idesc = (p.fp16 ? ptx::umma_idesc_f16_m128(cols) : ptx::umma_idesc_bf16_m128(cols)) |
+                               (W_MN ? 1u << 15 : 0u);   // bit 15: A is MN-major
+        // start-address step (16-byte units) of a 16-element K step of the weights, and their leading byte offset
+        constexpr uint32_t w_step = W_MN ? 16 * 128 / 16 : 2, w_lead = W_MN ? GEMM_WBYTES / 2 / 16 : 1;
         if (!ptx::mbar_wait(tempty_bar(buf), ((tile_it >> 1) & 1) ^ 1, abort_flag, 200 + buf)) break;
         ptx::tc_fence_after();
         const uint32_t d_tmem = tmem_base + (uint32_t)(buf * p.xrows_max);
@@ -406,12 +422,12 @@ gemm_ws_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__
           if (it == 0) GEMM_STAMP(2);    // first stage landed
           for (int a = 0; a < KA; ++a) {
             const uint32_t sw = stage_base + (uint32_t)s * stage_bytes + (uint32_t)a * atom_bytes;
-            // descriptors differ only in the start-address field: +2 (32 bytes) per 16-element K step
-            const uint64_t da = desc_hi | (uint64_t)(((sw & 0x3FFFFu) >> 4) | (1u << 16));
+            // descriptors differ only in the start-address field: +2 (32 bytes) per 16-element K step of a K-major tile
+            const uint64_t da = desc_hi | (uint64_t)(((sw & 0x3FFFFu) >> 4) | (w_lead << 16));
             const uint64_t db = desc_hi | (uint64_t)((((sw + GEMM_WBYTES) & 0x3FFFFu) >> 4) | (1u << 16));
             ptx::umma_bf16(d_tmem, da, db, idesc, (kb | a) != 0 ? 1u : 0u);
 #pragma unroll
-            for (int kk = 1; kk < GEMM_BK / 16; ++kk) ptx::umma_bf16_acc(d_tmem, da + 2 * kk, db + 2 * kk, idesc);
+            for (int kk = 1; kk < GEMM_BK / 16; ++kk) ptx::umma_bf16_acc(d_tmem, da + w_step * kk, db + 2 * kk, idesc);
           }
           ptx::umma_commit(empty_bar(s));  // stage is free once these MMAs have read it
         }
@@ -1157,7 +1173,7 @@ inline int moe_grouped_gemm_impl(const void* x, long long x_rows, long long x_ro
                                  const void* tile_count, int num_groups, int n_out, int K, long long out_row_stride,
                                  int max_tiles, int tile_rows_max, int mode, void* stream, int glu = GLU_REFERENCE,
                                  const void* scale_in = nullptr, const void* scale_out = nullptr,
-                                 int act = GEMM_ACT_NONE) {
+                                 int act = GEMM_ACT_NONE, bool w_mn = false, const void* w2 = nullptr) {
   if (!x || !w || !out || !tile_table || !tile_count || x_rows < 0 || num_groups <= 0 || n_out <= 0 || K <= 0 ||
       max_tiles < 0 || (mode != 0 && mode != 1))
     return B200_ERR_ARG;
@@ -1196,8 +1212,18 @@ inline int moe_grouped_gemm_impl(const void* x, long long x_rows, long long x_ro
   p.w_policy = ptx::kEvictFirst;
   CUtensorMap tw;
   GemmXMaps tx{};
-  int rc = make_tmap_2d(&tw, w, (uint64_t)num_groups * p.w_rows_per_group, (uint64_t)K, (uint64_t)K,
-                        mode == 1 ? 64 : GEMM_WTILE);
+  int rc;
+  if (w_mn) {
+    // [groups, k, features]: rows past a group's k and columns past its features read as zero
+    if (mode != 0 || gather_index || n_out % 8 != 0 || (w2 && K % (2 * GEMM_BK) != 0)) return B200_ERR_SHAPE;
+    const int k_one = w2 ? K / 2 : K;
+    p.k_second = w2 ? k_one : 0;
+    rc = make_tmap_3d(&tw, w, (uint64_t)num_groups, (uint64_t)k_one, (uint64_t)n_out, (uint64_t)k_one * n_out, (uint64_t)n_out, GEMM_BK);
+    if (!rc && w2)
+      rc = make_tmap_3d(&tx.w2, w2, (uint64_t)num_groups, (uint64_t)k_one, (uint64_t)n_out, (uint64_t)k_one * n_out, (uint64_t)n_out, GEMM_BK);
+  } else {
+    rc = make_tmap_2d(&tw, w, (uint64_t)num_groups * p.w_rows_per_group, (uint64_t)K, (uint64_t)K, mode == 1 ? 64 : GEMM_WTILE);
+  }
   if (rc) return rc;
   if (gather_index) {
     rc = make_tmap_2d(&tx.box[0], x, (uint64_t)x_rows, (uint64_t)K, (uint64_t)x_row_stride, 1u);
@@ -1210,6 +1236,7 @@ inline int moe_grouped_gemm_impl(const void* x, long long x_rows, long long x_ro
   if (rc) return rc;
   const long long tiles = (long long)max_tiles * p.w_tiles;
   if (mode == 1) return gemm_launch<GEMM_SWIGLU>(tw, tx, p, tiles, (cudaStream_t)stream);
+  if (w_mn) return gemm_launch<GEMM_DGRAD>(tw, tx, p, tiles, (cudaStream_t)stream);
   return gemm_launch<GEMM_PLAIN>(tw, tx, p, tiles, (cudaStream_t)stream);
 }
 }  // namespace b200
@@ -1220,6 +1247,18 @@ extern "C" int b200_moe_grouped_gemm(const void* x, const void* w, const void* r
                                      int max_tiles, int tile_rows_max, int mode, void* stream) {
   return b200::moe_grouped_gemm_impl(x, x_rows, K, nullptr, w, row_scale, out, tile_table, tile_count, num_groups,
                                      n_out, K, out_row_stride, max_tiles, tile_rows_max, mode, stream);
+}
+
+// Data gradient: out[r, n] = sum_k x[r, k] * w[g(r), k, n], w [num_groups, K, n_out] as a forward weight [., features,
+// inputs] lies; the weights are read MN-major, no transposed copy is made, and the products and their order are those of
+// b200_moe_grouped_gemm on the transposed tensor.  With w2, w and w2 are [num_groups, K / 2, n_out] and hold k below and from
+// K / 2 on (K a multiple of 128): the sum of two products in one accumulation.  n_out a multiple of 8.
+extern "C" int b200_moe_grouped_dgrad(const void* x, const void* w, const void* w2, void* out, const void* tile_table,
+                                      const void* tile_count, long long x_rows, int num_groups, int n_out, int K,
+                                      long long out_row_stride, int max_tiles, int tile_rows_max, void* stream) {
+  return b200::moe_grouped_gemm_impl(x, x_rows, K, nullptr, w, nullptr, out, tile_table, tile_count, num_groups, n_out, K,
+                                     out_row_stride, max_tiles, tile_rows_max, 0, stream, b200::GLU_REFERENCE, nullptr, nullptr,
+                                     b200::GEMM_ACT_NONE, true, w2);
 }
 
 // The same GEMM reading its activation rows where they lie: x is the unpermuted [T, K] matrix and sorted row r

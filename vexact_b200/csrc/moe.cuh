@@ -16,6 +16,7 @@
 // returned in descending weight order (what torch.topk(sorted=True) returns).
 #pragma once
 #include "common.cuh"
+#include "moe_wgrad_tc.cuh"
 #include "norm.cuh"
 
 namespace b200 {
@@ -692,8 +693,8 @@ moe_gather_checked_kernel(const __nv_bfloat16* __restrict__ x, long long x_rows,
 
 // Weight gradient of a grouped GEMM, the contraction running over each group's own rows ("ragged K"):
 //   c[g, m, n] = sum over rows r of group g, ascending, of a[r, m] * b[r, n]      (fp32 fmaf chain, one rounding)
-// (group_gemm/kernel/group_gemm.py:255-400 group_gemm_same_mn with transpose_a).  A training-side operator kept
-// simple: one CTA per 64 x 64 tile of one group's output, rows staged 16 at a time through shared memory, fp32
+// (group_gemm/kernel/group_gemm.py:255-400 group_gemm_same_mn with transpose_a), for widths and pointers that
+// moe_wgrad_tc_kernel's copies do not fit: one CTA per 64 x 64 tile of one group's output, rows staged 16 at a time through shared memory, fp32
 // FMAs on the CUDA cores.  With ~rows/groups rows per group the work is a few GFLOP and the kernel is bound by
 // writing c (groups * M * N * 2 bytes); an empty group gets zeros.  A group whose bounds leave [0, rows] or
 // decrease is clipped and reported through the status word.
@@ -767,87 +768,6 @@ moe_wgrad_kernel(const __nv_bfloat16* __restrict__ a, const __nv_bfloat16* __res
   }
 }
 
-// The same weight gradient on the tensor cores (mma.sync m16n8k16, bf16 x bf16 -> fp32): one CTA per 128 x 128
-// tile of one group's output, eight warps of 64 x 32 each, the group's rows staged 32 at a time as bf16 and read
-// with transposing ldmatrix (both operands have the contraction as their row dimension).  Products are exact,
-// the sum runs over 16-row steps in ascending order with the instruction's own order inside a step: deterministic,
-// and within fp32 rounding of the CUDA-core kernel above.  M and N multiples of 8, 16-byte aligned pointers.
-constexpr int WGM_TILE = 128, WGM_ROWS = 32, WGM_LD = WGM_TILE + 8;   // padded row: ldmatrix rows 272 bytes apart
-__global__ void __launch_bounds__(256)
-moe_wgrad_mma_kernel(const __nv_bfloat16* __restrict__ a, const __nv_bfloat16* __restrict__ b,
-                     __nv_bfloat16* __restrict__ c, const int* __restrict__ cu_seqlens, long long rows, int M, int N) {
-  pdl_trigger();
-  pdl_wait();
-  __shared__ __align__(16) __nv_bfloat16 sa[WGM_ROWS][WGM_LD], sb[WGM_ROWS][WGM_LD];
-  const int g = blockIdx.z, m0 = blockIdx.y * WGM_TILE, n0 = blockIdx.x * WGM_TILE;
-  long long r0 = cu_seqlens[g], r1 = cu_seqlens[g + 1];
-  if (r0 < 0 || r1 > rows || r1 < r0) {
-    if (threadIdx.x == 0 && blockIdx.x == 0 && blockIdx.y == 0) report_status(B200_STATUS_BAD_INDEX, g);
-    r0 = r0 < 0 ? 0 : (r0 > rows ? rows : r0);
-    r1 = r1 > rows ? rows : r1;
-    if (r1 < r0) r1 = r0;
-  }
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int wm = (warp >> 2) * 64, wn = (warp & 3) * 32;        // this warp's 64 x 32 corner inside the tile
-  float acc[4][4][4];                                            // [m16 tile][n8 tile][fragment]
-#pragma unroll
-  for (int i = 0; i < 4; ++i)
-#pragma unroll
-    for (int j = 0; j < 4; ++j)
-#pragma unroll
-      for (int e = 0; e < 4; ++e) acc[i][j][e] = 0.f;
-  const uint32_t sa_base = (uint32_t)__cvta_generic_to_shared(&sa[0][0]);
-  const uint32_t sb_base = (uint32_t)__cvta_generic_to_shared(&sb[0][0]);
-  for (long long r = r0; r < r1; r += WGM_ROWS) {
-    __syncthreads();                                             // the previous chunk has been consumed
-#pragma unroll
-    for (int it = 0; it < 2; ++it) {                             // 32 rows x 16 vectors of 8 columns per operand
-      const int e = tid + it * 256, lr = e >> 4, lc = (e & 15) * 8;
-      uint4 va = make_uint4(0, 0, 0, 0), vb = make_uint4(0, 0, 0, 0);
-      if (r + lr < r1) {
-        if (m0 + lc < M) va = *reinterpret_cast<const uint4*>(a + (r + lr) * M + m0 + lc);
-        if (n0 + lc < N) vb = *reinterpret_cast<const uint4*>(b + (r + lr) * N + n0 + lc);
-      }
-      *reinterpret_cast<uint4*>(&sa[lr][lc]) = va;
-      *reinterpret_cast<uint4*>(&sb[lr][lc]) = vb;
-    }
-    __syncthreads();
-#pragma unroll
-    for (int kk0 = 0; kk0 < WGM_ROWS; kk0 += 16) {
-      uint32_t bf[4][2];
-#pragma unroll
-      for (int jp = 0; jp < 2; ++jp) {                           // two n8 tiles per ldmatrix
-        const int row = kk0 + (lane & 7) + ((lane >> 3) & 1) * 8, col = wn + jp * 16 + (lane >> 4) * 8;
-        ldmatrix_x4_trans(sb_base + (uint32_t)(row * WGM_LD + col) * 2, bf[2 * jp][0], bf[2 * jp][1],
-                          bf[2 * jp + 1][0], bf[2 * jp + 1][1]);
-      }
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        const int row = kk0 + (lane & 7) + (lane >> 4) * 8, col = wm + i * 16 + ((lane >> 3) & 1) * 8;
-        uint32_t a0, a1, a2, a3;
-        ldmatrix_x4_trans(sa_base + (uint32_t)(row * WGM_LD + col) * 2, a0, a1, a2, a3);
-#pragma unroll
-        for (int j = 0; j < 4; ++j) mma_bf16_16816(acc[i][j], a0, a1, a2, a3, bf[j][0], bf[j][1]);
-      }
-    }
-  }
-  __nv_bfloat16* cg = c + (long long)g * M * N;
-  const int gid = lane >> 2, tig = lane & 3;
-#pragma unroll
-  for (int i = 0; i < 4; ++i)
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const int n = n0 + wn + j * 8 + 2 * tig;
-      if (n >= N) continue;
-#pragma unroll
-      for (int half = 0; half < 2; ++half) {
-        const int m = m0 + wm + i * 16 + gid + half * 8;
-        if (m < M)
-          *reinterpret_cast<uint32_t*>(cg + (long long)m * N + n) = pack_bf2(acc[i][j][2 * half], acc[i][j][2 * half + 1]);
-      }
-    }
-}
-
 // out[g, c, r] = x[g, r, c] for 2-byte elements: 64 x 64 tiles through shared memory, 16-byte loads and stores.
 // R and C multiples of 8.  (The dgrad grouped GEMM reads the expert weights with the other dimension contiguous.)
 __global__ void __launch_bounds__(256)
@@ -919,6 +839,56 @@ swiglu_scale_kernel(const __nv_bfloat16* __restrict__ gate, const __nv_bfloat16*
   } else {
     out[r * I + c] = f2bf(one(bf2f(gate[src]), bf2f(up[src])));
   }
+}
+
+// Backward of the expert activation h = bf16(bf16(silu(g)) * u) * s over rows of I elements, with the rounding points of the
+// reference's chain of torch operators (fused_moe.py:113-236): from g, u and the gradient d of h * s it gives
+//   h_scaled = bf16(act * s), d_g = silu'(g) * bf16(d_a * u), d_u = bf16(silu(g)) * d_a, d_a = bf16(d * s), and the rows'
+//   d_s = sum of bf16(act * d), in fp32 with one rounding.
+// One warp per row, 16 bytes a lane; three reads and three writes of 2 bytes per element where the chain of eight kernels made
+// eighteen (330 us for 32768 rows of 768).
+__global__ void __launch_bounds__(256)
+swiglu_backward_kernel(const __nv_bfloat16* __restrict__ gate, const __nv_bfloat16* __restrict__ up, long long in_stride,
+                       const __nv_bfloat16* __restrict__ d_h, const __nv_bfloat16* __restrict__ row_scale,
+                       __nv_bfloat16* __restrict__ h_scaled, __nv_bfloat16* __restrict__ d_gate, __nv_bfloat16* __restrict__ d_up,
+                       long long d_stride, __nv_bfloat16* __restrict__ d_scale, long long rows, int I) {
+  pdl_trigger();
+  pdl_wait();
+  const long long r = (long long)blockIdx.x * 8 + (threadIdx.x >> 5);
+  if (r >= rows) return;
+  const int lane = threadIdx.x & 31;
+  const float s = bf2f(row_scale[r]);
+  float sum = 0.f;
+  for (int c = lane * 8; c < I; c += 256) {
+    const uint4 gv = *reinterpret_cast<const uint4*>(gate + r * in_stride + c), uv = *reinterpret_cast<const uint4*>(up + r * in_stride + c),
+                dv = *reinterpret_cast<const uint4*>(d_h + r * I + c);
+    const uint32_t g4[4] = {gv.x, gv.y, gv.z, gv.w}, u4[4] = {uv.x, uv.y, uv.z, uv.w}, d4[4] = {dv.x, dv.y, dv.z, dv.w};
+    uint32_t h[4], dg[4], du[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      float g[2], u[2], d[2], oh[2], og[2], ou[2];
+      unpack_bf2(g4[j], g[0], g[1]);
+      unpack_bf2(u4[j], u[0], u[1]);
+      unpack_bf2(d4[j], d[0], d[1]);
+#pragma unroll
+      for (int k = 0; k < 2; ++k) {
+        const float den = 1.f + expf(-g[k]), sig = 1.f / den, sg = round_bf(g[k] / den), act = round_bf(sg * u[k]);
+        const float da = round_bf(d[k] * s);
+        sum += round_bf(act * d[k]);
+        oh[k] = act * s;
+        ou[k] = sg * da;
+        og[k] = round_bf(da * u[k]) * sig * (1.f + g[k] * (1.f - sig));
+      }
+      h[j] = pack_bf2(oh[0], oh[1]);
+      dg[j] = pack_bf2(og[0], og[1]);
+      du[j] = pack_bf2(ou[0], ou[1]);
+    }
+    *reinterpret_cast<uint4*>(h_scaled + r * I + c) = make_uint4(h[0], h[1], h[2], h[3]);
+    *reinterpret_cast<uint4*>(d_gate + r * d_stride + c) = make_uint4(dg[0], dg[1], dg[2], dg[3]);
+    *reinterpret_cast<uint4*>(d_up + r * d_stride + c) = make_uint4(du[0], du[1], du[2], du[3]);
+  }
+  sum = warp_sum(sum);
+  if (lane == 0) d_scale[r] = f2bf(sum);
 }
 
 }  // namespace b200
@@ -1330,29 +1300,32 @@ extern "C" int b200_transpose_last2(const void* x, void* out, int G, int R, int 
   return launch_status();
 }
 
-// c[g] = a[rows of g]^T @ b[rows of g]: a [rows, M], b [rows, N], c [G, M, N] bf16 contiguous, cu_seqlens
-// [G + 1] i32 (rows of group g are [cu[g], cu[g + 1])).  M and N multiples of 4, 8-byte aligned pointers.
-extern "C" int b200_moe_grouped_wgrad(const void* a, const void* b, void* c, const void* cu_seqlens, long long rows,
-                                      int num_groups, int M, int N, void* stream) {
+// c[g] = a[rows of g]^T @ b[rows of g]: a [rows, M], b [rows, N] with rows a_row_stride and b_row_stride apart, c [G, M, N]
+// bf16 contiguous, cu_seqlens [G + 1] i32 (rows of group g are [cu[g], cu[g + 1])).  M, N and the strides multiples of 8
+// and 16-byte aligned pointers; contiguous a and b also with multiples of 4 and 8-byte aligned pointers.
+extern "C" int b200_moe_grouped_wgrad_strided(const void* a, long long a_row_stride, const void* b, long long b_row_stride,
+                                              void* c, const void* cu_seqlens, long long rows, int num_groups, int M, int N,
+                                              void* stream) {
   using namespace b200;
   if (!a || !b || !c || !cu_seqlens || rows < 0 || num_groups <= 0 || M <= 0 || N <= 0) return B200_ERR_ARG;
-  if (M % 4 != 0 || N % 4 != 0 || num_groups > 65535 || (M + WG_TILE - 1) / WG_TILE > 65535) return B200_ERR_SHAPE;
-  static const int simt = env_int("B200_WGRAD_SIMT", 0);        // development knob: the CUDA-core kernel
-  const bool vec16 = M % 8 == 0 && N % 8 == 0 &&
-                     ((reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(b)) & 15) == 0 &&
-                     (reinterpret_cast<uintptr_t>(c) & 3) == 0;
-  if (vec16 && !simt) {
-    launch_k(moe_wgrad_mma_kernel, dim3((unsigned)((N + WGM_TILE - 1) / WGM_TILE),
-                                        (unsigned)((M + WGM_TILE - 1) / WGM_TILE), (unsigned)num_groups),
-             dim3(256), 0, (cudaStream_t)stream, (const __nv_bfloat16*)a, (const __nv_bfloat16*)b,
-             (__nv_bfloat16*)c, (const int*)cu_seqlens, rows, M, N);
-    return launch_status();
-  }
+  if (M % 4 != 0 || N % 4 != 0 || num_groups > 65535 || (M + WG_TILE - 1) / WG_TILE > 65535 || rows > 0x7fffffffLL)
+    return B200_ERR_SHAPE;
+  const bool vec16 = M % 8 == 0 && N % 8 == 0 && a_row_stride % 8 == 0 && b_row_stride % 8 == 0 &&
+                     ((reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(b) | reinterpret_cast<uintptr_t>(c)) & 15) == 0;
+  if (vec16)
+    return moe_wgrad_tc_launch(a, a_row_stride, b, b_row_stride, c, (const int*)cu_seqlens, rows, num_groups, M, N,
+                               (cudaStream_t)stream);
+  if (a_row_stride != M || b_row_stride != N) return B200_ERR_SHAPE;
   launch_k(moe_wgrad_kernel, dim3((unsigned)((N + WG_TILE - 1) / WG_TILE), (unsigned)((M + WG_TILE - 1) / WG_TILE),
                                   (unsigned)num_groups),
            dim3(256), 0, (cudaStream_t)stream, (const __nv_bfloat16*)a, (const __nv_bfloat16*)b, (__nv_bfloat16*)c,
            (const int*)cu_seqlens, rows, M, N);
   return launch_status();
+}
+
+extern "C" int b200_moe_grouped_wgrad(const void* a, const void* b, void* c, const void* cu_seqlens, long long rows,
+                                      int num_groups, int M, int N, void* stream) {
+  return b200_moe_grouped_wgrad_strided(a, M, b, N, c, cu_seqlens, rows, num_groups, M, N, stream);
 }
 
 // b200_moe_unpermute_reduce + b200_add_rmsnorm in one launch: sum_out = residual + moe output (the new
@@ -1396,4 +1369,22 @@ extern "C" int b200_swiglu_scale_strided(const void* gate, const void* up, const
 extern "C" int b200_swiglu_scale(const void* gate, const void* up, const void* row_scale, void* out,
                                  long long rows, int I, void* stream) {
   return b200_swiglu_scale_strided(gate, up, row_scale, out, rows, I, I, stream);
+}
+
+// The backward of b200_swiglu_scale (swiglu_backward_kernel): gate and up rows in_row_stride apart, d_gate and d_up rows
+// d_row_stride apart, d_h and h_scaled [rows, I] contiguous.  I and the strides multiples of 8, 16-byte aligned pointers.
+extern "C" int b200_swiglu_backward(const void* gate, const void* up, long long in_row_stride, const void* d_h,
+                                    const void* row_scale, void* h_scaled, void* d_gate, void* d_up, long long d_row_stride,
+                                    void* d_scale, long long rows, int I, void* stream) {
+  using namespace b200;
+  if (!gate || !up || !d_h || !row_scale || !h_scaled || !d_gate || !d_up || !d_scale || rows < 0 || I <= 0) return B200_ERR_ARG;
+  if (I % 8 != 0 || in_row_stride % 8 != 0 || d_row_stride % 8 != 0 || in_row_stride < I || d_row_stride < I ||
+      ((reinterpret_cast<uintptr_t>(gate) | reinterpret_cast<uintptr_t>(up) | reinterpret_cast<uintptr_t>(d_h) |
+        reinterpret_cast<uintptr_t>(h_scaled) | reinterpret_cast<uintptr_t>(d_gate) | reinterpret_cast<uintptr_t>(d_up)) & 15) != 0)
+    return B200_ERR_SHAPE;
+  if (rows == 0) return B200_OK;
+  launch_k(swiglu_backward_kernel, dim3((unsigned)((rows + 7) / 8)), dim3(256), 0, (cudaStream_t)stream, (const __nv_bfloat16*)gate,
+           (const __nv_bfloat16*)up, in_row_stride, (const __nv_bfloat16*)d_h, (const __nv_bfloat16*)row_scale,
+           (__nv_bfloat16*)h_scaled, (__nv_bfloat16*)d_gate, (__nv_bfloat16*)d_up, d_row_stride, (__nv_bfloat16*)d_scale, rows, I);
+  return launch_status();
 }

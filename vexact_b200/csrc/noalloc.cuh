@@ -94,18 +94,10 @@ tiles_from_cu_seqlens_kernel(const int* __restrict__ cu_seqlens, int num_groups,
 
 }  // namespace b200
 
-// Same arithmetic and the same GEMM kernel as b200_moe_grouped_gemm (modes 0 and 1), for rows
-// already sorted by group, with the tile table kept in the library's fixed device array.
-//   x [x_rows, K] bf16, w [num_groups, n_out | 2*n_out, K] bf16, cu_seqlens [num_groups + 1] int32
-//   (device memory: rows of group g are cu_seqlens[g] .. cu_seqlens[g+1]), out [x_rows, n_out] bf16.
-// Limits: num_groups <= 1024 and num_groups + x_rows / 64 <= 4095 token tiles; beyond them the
-// call returns -2 and launches nothing.  It calls no cudaMalloc / cudaFree.  The first call on a
-// device looks up the array's device address; make that call before any stream capture begins.
-extern "C" int b200_moe_grouped_gemm_noalloc(const void* x, const void* w, const void* row_scale, void* out,
-                                             const void* cu_seqlens, long long x_rows, int num_groups,
-                                             int n_out, int K, long long out_row_stride, int mode,
-                                             void* stream) {
-  using namespace b200;
+namespace b200 {
+inline int grouped_gemm_noalloc(const void* x, const void* w, const void* row_scale, void* out, const void* cu_seqlens,
+                                long long x_rows, int num_groups, int n_out, int K, long long out_row_stride, int mode,
+                                bool dgrad, void* stream) {
   if (!x || !w || !out || !cu_seqlens || x_rows < 0 || num_groups <= 0 || n_out <= 0 || K <= 0 ||
       (mode != 0 && mode != 1))
     return B200_ERR_ARG;
@@ -123,6 +115,29 @@ extern "C" int b200_moe_grouped_gemm_noalloc(const void* x, const void* w, const
                                                    NOALLOC_MAX_TILES, (int)x_rows);
   rc = launch_status();
   if (rc) return rc;
-  return b200_moe_grouped_gemm(x, w, row_scale, out, table + 1, table, x_rows, num_groups, n_out, K,
-                               out_row_stride, (int)(num_groups + x_rows / tile_rows), tile_rows, mode, stream);
+  return moe_grouped_gemm_impl(x, x_rows, K, nullptr, w, row_scale, out, table + 1, table, num_groups, n_out, K, out_row_stride,
+                               (int)(num_groups + x_rows / tile_rows), tile_rows, mode, stream, GLU_REFERENCE, nullptr, nullptr,
+                               GEMM_ACT_NONE, dgrad);
+}
+}  // namespace b200
+
+// Same arithmetic and the same GEMM kernel as b200_moe_grouped_gemm (modes 0 and 1), for rows
+// already sorted by group, with the tile table kept in the library's fixed device array.
+//   x [x_rows, K] bf16, w [num_groups, n_out | 2*n_out, K] bf16, cu_seqlens [num_groups + 1] int32
+//   (device memory: rows of group g are cu_seqlens[g] .. cu_seqlens[g+1]), out [x_rows, n_out] bf16.
+// Limits: num_groups <= 1024 and num_groups + x_rows / 64 <= 4095 token tiles; beyond them the
+// call returns -2 and launches nothing.  It calls no cudaMalloc / cudaFree.  The first call on a
+// device looks up the array's device address; make that call before any stream capture begins.
+extern "C" int b200_moe_grouped_gemm_noalloc(const void* x, const void* w, const void* row_scale, void* out,
+                                             const void* cu_seqlens, long long x_rows, int num_groups,
+                                             int n_out, int K, long long out_row_stride, int mode,
+                                             void* stream) {
+  return b200::grouped_gemm_noalloc(x, w, row_scale, out, cu_seqlens, x_rows, num_groups, n_out, K, out_row_stride, mode, false,
+                                    stream);
+}
+
+// b200_moe_grouped_dgrad in the same terms: w [num_groups, K, n_out].
+extern "C" int b200_moe_grouped_dgrad_noalloc(const void* x, const void* w, void* out, const void* cu_seqlens, long long x_rows,
+                                              int num_groups, int n_out, int K, long long out_row_stride, void* stream) {
+  return b200::grouped_gemm_noalloc(x, w, nullptr, out, cu_seqlens, x_rows, num_groups, n_out, K, out_row_stride, 0, true, stream);
 }

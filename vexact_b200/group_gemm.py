@@ -7,9 +7,8 @@ reference's tests call directly.  `fused_moe_forward` in this package runs the s
 launches; these are for callers that hold the reference's intermediate tensors (a scatter index, an
 inclusive cumulative sum of rows per expert) and want one step at a time.
 
-The two GEMM forms of the backward are here too, correct but not tuned: `transpose_b=False` (dgrad) runs
-the forward kernel over a transposed copy of the weights, `group_gemm_same_mn` (the ragged-K weight gradient)
-is a CUDA-core kernel.  `moe_add_gather`, fused activations and accumulation into `c` raise NotImplementedError.
+The two GEMM forms of the backward are here too: `transpose_b=False` (dgrad) is the forward kernel reading the
+weights as they lie, `group_gemm_same_mn` (the ragged-K weight gradient) has a tcgen05 kernel of its own.  `moe_add_gather`, fused activations and accumulation into `c` raise NotImplementedError.
 """
 from __future__ import annotations
 
@@ -27,17 +26,6 @@ def _index_i32(index: torch.Tensor) -> torch.Tensor:
     if index.dtype not in (torch.int32, torch.int64):
         raise ValueError(f"index must be int32 or int64, got {index.dtype}")
     return index if index.dtype == torch.int32 else index.to(torch.int32)
-
-
-def _transpose_last2(x: torch.Tensor) -> torch.Tensor:
-    """[G, R, C] -> contiguous [G, C, R] (tiled kernel for 2-byte elements with R, C multiples of 8)."""
-    G, R, C = x.shape
-    if x.element_size() != 2 or R % 8 or C % 8 or not x.is_contiguous() or x.data_ptr() % 16:
-        return x.transpose(1, 2).contiguous()
-    out = torch.empty((G, C, R), dtype=x.dtype, device=x.device)
-    _lib.check(_lib.load().b200_transpose_last2(x.data_ptr(), out.data_ptr(), G, R, C, _lib.current_stream()),
-               "b200_transpose_last2")
-    return out
 
 
 def expert_histogram(input: torch.Tensor, num_bins: int) -> torch.Tensor:
@@ -142,11 +130,13 @@ def group_gemm_same_nk(
     del max_M
     assert not transpose_a, "Transpose A not tested yet."
     if not transpose_b:
-        # dgrad: b is [G, K, N] with N contiguous.  The tensor-core kernel reads weights K-major, so the weights
-        # are transposed into scratch first (one extra pass over them); the products and their order are those
-        # of the forward form on the transposed tensor.
+        # dgrad: b is [G, K, N] with N contiguous, read as it lies; the products and their order are those of the
+        # forward form on the transposed tensor, which serves rows and pointers that a 16-byte copy does not fit.
         assert b.dim() == 3 and a.shape[1] == b.shape[1]
-        return group_gemm_same_nk(a, _transpose_last2(b), cumsum_M, 0, transpose_b=True)
+        if b.shape[2] % 8 or b.data_ptr() % 16 or not b.is_contiguous() or b.element_size() != 2:
+            return group_gemm_same_nk(a, b.transpose(1, 2).contiguous(), cumsum_M, 0, transpose_b=True)
+        # (a fused activation or c was not passed on by this form, and is not looked at here either)
+        activation, save_activation, c = None, False, None
     if activation is not None or save_activation:
         raise NotImplementedError("a fused activation is not offered here; fused_moe_forward fuses SwiGLU itself")
     if c is not None:
@@ -156,13 +146,20 @@ def group_gemm_same_nk(
     if a.dtype != torch.bfloat16 or b.dtype != torch.bfloat16:
         raise NotImplementedError("the grouped GEMM is implemented for bf16")
     assert a.is_cuda and a.device == b.device, f"a.device = {a.device}, b.device = {b.device}"
-    G, N, K = b.shape
+    G, N, K = b.shape if transpose_b else (b.shape[0], b.shape[2], b.shape[1])
     assert len(cumsum_M) == G
     assert a.is_contiguous() and b.is_contiguous(), "Not implemented: Noncontiguous input."
     assert a.shape[1] == K
     cu = torch.zeros(G + 1, dtype=torch.int32, device=a.device)
     cu[1:] = cumsum_M
     out = torch.empty((a.shape[0], N), dtype=a.dtype, device=a.device)
+    if not transpose_b:
+        _lib.check(
+            _lib.load().b200_moe_grouped_dgrad_noalloc(a.data_ptr(), b.data_ptr(), out.data_ptr(), cu.data_ptr(),
+                                                       a.shape[0], G, N, K, out.stride(0), _lib.current_stream()),
+            "b200_moe_grouped_dgrad_noalloc",
+        )
+        return out
     _lib.check(
         _lib.load().b200_moe_grouped_gemm_noalloc(a.data_ptr(), b.data_ptr(), None, out.data_ptr(), cu.data_ptr(),
                                                   a.shape[0], G, N, K, out.stride(0), 0, _lib.current_stream()),
