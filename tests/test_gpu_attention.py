@@ -451,7 +451,8 @@ def _eager_packed(q, k, v, scale):
     ([65, 129], [65, 129], 4, 2, 128, 128),     # full causal prefill, tiles with ragged edges
     ([9, 23], [41, 57], 6, 3, 40, 40),          # a head dim the kernels do not tile (zero columns)
     ([5, 40], [33, 40], 4, 4, 192, 128),        # MLA dims
-    ([1, 128, 257], [700, 129, 257], 8, 1, 128, 128),   # one query, owned tiles with one row over, a long context
+    ([1, 128], [700, 129], 8, 1, 128, 128),     # one query on a long context, owned tiles with one row over
+    ([128, 257], [128, 257], 8, 1, 128, 128),   # whole owned tiles, and one row more
     ([130, 64], [130, 511], 4, 2, 192, 128),    # owned and streamed tiles with remainders, MLA dims
 ])
 def test_packed_varlen_backward_matches_autograd_of_fp32_attention(vb, q_lens, kv_lens, hq, hkv, dk, dv):
@@ -556,3 +557,40 @@ def test_packed_varlen_backward_keeps_to_its_sequence(vb):
         t[71::2] = float("inf")
     for a, b in zip(alone, run(q, k, v, dout, cu)):
         assert torch.equal(a, b[:70])
+
+
+def test_rows_kernel_for_192_wide_keys_gives_the_columns_kernels_bits(vb):
+    """Key dim 192 / value dim 128: the rows-on-lanes kernel (two K blocks, one V block, one query tile in shared memory) and
+    the keys-on-lanes kernel, over tiles of one and several blocks, whole and partial, many tiles per CTA, query heads alone
+    and in groups; query and output tiles by TMA and by lanes; each sequence's last query as a decode step."""
+    g = torch.Generator().manual_seed(79)
+    for (hq, hkv, page, q_lens, ctx) in [(16, 16, 16, [130, 40, 1, 7, 700], [130, 200, 257, 7, 701]),
+                                         (16, 4, 128, [300, 1], [300, 513]),
+                                         (12, 2, 16, [257, 64], [1000, 64]),
+                                         (16, 1, 16, [70], [70])]:
+        S, dk, dv = len(ctx), 192, 128
+        pages = max((c + page - 1) // page for c in ctx)
+        kc = torch.randn(S * pages + 1, page, hkv, dk, generator=g).to(BF).cuda()
+        vc = torch.randn(S * pages + 1, page, hkv, dv, generator=g).to(BF).cuda()
+        table = torch.randperm(S * pages, generator=g).view(S, pages).to(torch.int32).cuda()
+        q = torch.randn(sum(q_lens), hq, dk, generator=g).to(BF).cuda()
+        cu = torch.tensor([0] + torch.tensor(q_lens).cumsum(0).tolist(), dtype=torch.int32).cuda()
+        used = torch.tensor(ctx, dtype=torch.int32).cuda()
+        kw = dict(cu_seqlens_q=cu, max_seqlen_q=max(q_lens), seqused_k=used, page_table=table, softmax_scale=dk ** -0.5,
+                  causal=True)
+
+        def run(**env):
+            os.environ.update(env)
+            try:
+                return vb.flash_attn_varlen_func(q, kc, vc, **kw)[0]
+            finally:
+                for k in env:
+                    del os.environ[k]
+
+        rows = run()
+        assert torch.equal(rows, run(B200_ATTN_PREFILL="cols"))
+        assert torch.equal(rows, run(B200_ATTN_Q_TMA="0", B200_ATTN_O_TMA="0"))
+        last = (cu[1:] - 1).long()
+        one = vb.flash_attn_varlen_func(q[last], kc, vc, cu_seqlens_q=torch.arange(S + 1, dtype=torch.int32).cuda(),
+                                        max_seqlen_q=1, seqused_k=used, page_table=table, softmax_scale=dk ** -0.5, causal=True)[0]
+        assert torch.equal(one, rows[last])

@@ -402,7 +402,7 @@ inline bool attn_use_tensor_memory() {
 int attn_tc_dispatch(const CUtensorMap& tk, const CUtensorMap& tv, const AttnParams& p, dim3 grid, int dk, int nc,
                      cudaStream_t st);
 int attn_rows_dispatch(const CUtensorMap& tk, const CUtensorMap& tv, const CUtensorMap& tq, const CUtensorMap& to,
-                       const AttnParams& p, cudaStream_t st);
+                       const AttnParams& p, int dk, cudaStream_t st);
 
 // Queries as a 3-D tensor [tokens][heads][dim] with a box of {64 dims, box_heads, box_tokens}: the box's rows
 // land in shared memory in (token, head) order, 128 bytes each, 128-byte swizzle, which is the row order of a
@@ -423,7 +423,7 @@ inline int make_tmap_q(CUtensorMap* m, const void* q, long long tokens, int head
                    CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   return r == CUDA_SUCCESS ? B200_OK : B200_ERR_DRIVER;
 }
-// Prefill tiles of head dim 128: rows-on-lanes kernel unless B200_ATTN_PREFILL=cols.
+// Prefill tiles: rows-on-lanes kernel unless B200_ATTN_PREFILL=cols.
 // (Read at every call, so that a test can run both kernels in one process and compare their bits.)
 inline bool attn_prefill_rows() {
   const char* v = getenv("B200_ATTN_PREFILL");
@@ -530,11 +530,11 @@ extern "C" int b200_paged_attn_fwd_ordered(const void* q, const void* k_cache, c
   if (attn_use_tensor_memory() && dv == 128 && (dk == 128 || dk == 192) && q_tok_stride % 8 == 0 &&
       q_head_stride % 8 == 0 && (reinterpret_cast<uintptr_t>(q) & 15) == 0) {
     // tcgen05 kernels.  A decode step (one query per sequence) uses the narrow keys-on-lanes tile (16
-    // columns); steps with longer query runs use 128-row tiles with a row per thread (attn_rows.cuh) for
-    // head dim 128 and the 32-column keys-on-lanes tile for the 192 / 128 dims.  B200_ATTN_PREFILL=cols
-    // keeps the 64-column keys-on-lanes tile for head dim 128 (the same bits, for cross-checks).
-    const bool rows = max_seqlen_q > 1 && dk == 128 && attn_prefill_rows();
-    const int nc = max_seqlen_q == 1 ? 16 : (dk == 128 ? (rows ? 128 : 64) : 32);
+    // columns); steps with longer query runs use 128-row tiles with two threads per row (attn_rows.cuh): four
+    // prompts of together 3001 tokens, 16 heads of 192 / 128, took 225 us on 32-column keys-on-lanes tiles, whose
+    // softmax crosses lanes.  B200_ATTN_PREFILL=cols keeps those tiles (the same bits, for cross-checks).
+    const bool rows = max_seqlen_q > 1 && attn_prefill_rows();
+    const int nc = max_seqlen_q == 1 ? 16 : rows ? 128 : dk == 128 ? 64 : 32;
     p.pos_per_tile = nc / hh;
     dim3 grid((unsigned)((max_seqlen_q + p.pos_per_tile - 1) / p.pos_per_tile),
               (unsigned)(num_kv_heads * p.head_chunks), (unsigned)num_seqs);
@@ -571,7 +571,7 @@ extern "C" int b200_paged_attn_fwd_ordered(const void* q, const void* k_cache, c
           make_tmap_q(&to, out, total_q, num_q_heads, dv, o_tok_stride, o_head_stride, hh_const, 32 / hh_const, true) ==
               B200_OK)
         p.o_tma = 1;
-      return attn_rows_dispatch(tk, tv, tq, to, p, st);
+      return attn_rows_dispatch(tk, tv, tq, to, p, dk, st);
     }
     return attn_tc_dispatch(tk, tv, p, grid, dk, nc, st);
   }

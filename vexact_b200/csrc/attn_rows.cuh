@@ -90,18 +90,19 @@ __global__ void __launch_bounds__(ATR_THREADS, 1)
 paged_attn_rows_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CUtensorMap tm_v,
                        const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_out,
                        const __grid_constant__ CUtensorMap tm_gate, const AttnParams p) {
-  constexpr int DV = 128, NC = ATR_ROWS, KST = 2, VST = 2;
+  // 192-wide keys: their second ring stage takes the place of the second V block and the second Q buffer
+  constexpr int DV = 128, NC = ATR_ROWS, KST = 2, VST = DK > 128 ? 1 : 2;
   constexpr bool EXTRAS = FORM != ATTN_PLAIN, SIGMOID = FORM == ATTN_SIGMOID;
   constexpr int KH = DK / 64, VH = DV / 64;
   constexpr int K_BYTES = ATC_BN * DK * 2, V_BYTES = ATC_BN * DV * 2;
   constexpr int KV_BYTES = KST * K_BYTES + VST * V_BYTES;
   constexpr int Q_BYTES = KH * NC * 128;   // KH halves of [128 rows][128 B]; QBUFS such buffers
-  constexpr int QBUFS = EXACT ? 1 : 2;
+  constexpr int QBUFS = EXACT || DK > 128 ? 1 : 2;
   constexpr int P_TILE = 2 * NC * 128;     // two 64-key halves of [128 rows][128 B]
   constexpr int P_BYTES = EXACT ? 2 * P_TILE : P_TILE;   // hi, lo
   // Q buffer of a tile, and the parity of its use
-  auto q_buf = [](uint32_t it) { return EXACT ? 0u : it & 1u; };
-  auto q_par = [](uint32_t it) { return EXACT ? it & 1u : (it >> 1) & 1u; };
+  auto q_buf = [](uint32_t it) { return QBUFS == 1 ? 0u : it & 1u; };
+  auto q_par = [](uint32_t it) { return QBUFS == 1 ? it & 1u : (it >> 1) & 1u; };
   // key block j of a tile's walk
   auto block_of = [](const AtcTile& t, int j) {
     if constexpr (EXTRAS) return j < t.head ? j : t.blk0 + j - t.head;
@@ -739,7 +740,7 @@ template <int DK, bool EXACT, int FORM>
 inline int attn_rows_launch(const CUtensorMap& tk, const CUtensorMap& tv, const CUtensorMap& tq, const CUtensorMap& to,
                             const CUtensorMap& tg, const AttnParams& p, cudaStream_t st) {
   // tiles (K ring, V ring, Q buffers, P) + small arrays (barriers, alpha, l, TMEM slot, abort flag) + alignment
-  constexpr int tiles = ATC_BN * (2 * DK + 2 * 128) * 2 + (EXACT ? 1 : 2) * (DK / 64) * ATR_ROWS * 128 +
+  constexpr int tiles = ATC_BN * (2 * DK + (DK > 128 ? 1 : 2) * 128) * 2 + (EXACT || DK > 128 ? 1 : 2) * (DK / 64) * ATR_ROWS * 128 +
                         (EXACT ? 4 : 2) * ATR_ROWS * 128;
   constexpr int small = 256 + 4 * ATR_ROWS * 4 + 16;
   constexpr int smem = (tiles + small + 1023 <= 227 * 1024) ? tiles + small + 1023 : 227 * 1024;
@@ -752,8 +753,9 @@ inline int attn_rows_launch(const CUtensorMap& tk, const CUtensorMap& tv, const 
 }
 
 inline int attn_rows_dispatch(const CUtensorMap& tk, const CUtensorMap& tv, const CUtensorMap& tq, const CUtensorMap& to,
-                              const AttnParams& p, cudaStream_t st) {
-  return attn_rows_launch<128, false, ATTN_PLAIN>(tk, tv, tq, to, tk, p, st);
+                              const AttnParams& p, int dk, cudaStream_t st) {
+  return dk == 128 ? attn_rows_launch<128, false, ATTN_PLAIN>(tk, tv, tq, to, tk, p, st)
+                   : attn_rows_launch<192, false, ATTN_PLAIN>(tk, tv, tq, to, tk, p, st);
 }
 
 }  // namespace b200
