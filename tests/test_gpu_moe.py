@@ -600,3 +600,16 @@ def test_grouped_data_gradient_reads_weights_as_they_lie(K, N, tokens):
     assert torch.equal(product(x2, w, w2), product(x2, torch.cat([w, w2], 1), None))
     ref = torch.cat([x2[cu[e]:cu[e + 1]].double() @ torch.cat([w[e], w2[e]]).double() for e in range(E)])
     torch.testing.assert_close(product(x2, w, w2).double(), ref, **tol)
+
+
+@pytest.mark.parametrize("T, N, K", [(1024, 64, 64), (1025, 67, 96), (517, 130, 2048), (70000, 1, 32)])
+def test_fp32_products_in_groups_have_the_single_outputs_bits(vb, T, N, K):
+    """Many outputs run 4 x 4 to eight lanes, few a warp each: the same partial sums joined in the same order."""
+    from vexact_b200.batch_invariant_ops import linear_f32_from_bf16
+
+    x, w = _seeded(T, K, seed=T).cuda(), _seeded(N, K, seed=N).cuda()
+    many = linear_f32_from_bf16(x, w)
+    for r in (slice(0, 1), slice(T // 2, T // 2 + 3), slice(T - 1, T)):
+        assert torch.equal(many[r], linear_f32_from_bf16(x[r], w))
+    # K fp32 products of order 1
+    torch.testing.assert_close(many.double(), x.double() @ w.double().t(), rtol=1e-6, atol=2e-7 * K)

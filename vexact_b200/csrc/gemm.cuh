@@ -811,6 +811,86 @@ gemm_f32_kernel(const TIn* __restrict__ x, const TIn* __restrict__ w, const floa
   acc = warp_sum(acc);
   if (lane == 0) out[t * out_stride + n] = acc + (bias ? bias[n] : 0.f);
 }
+
+// The same products and sums for many outputs.  An output is 32 partial sums, one per k mod 32, joined by the butterfly; a
+// warp for one output loads two values for one FMA (136 us for 3001 x 64 outputs of 2048).  Here eight lanes hold the 32 sums,
+// four each (8- or 16-byte loads), of 4 tokens x 4 features, so eight loads feed 64 FMAs and the FMA pipe is the bound.
+constexpr int GF_TOKENS = 8, GF_FEATURES = 64;     // of a CTA: 2 x 4 warps of 4 tokens x 16 features
+template <typename TIn>
+__device__ __forceinline__ void gf_load(const TIn* p, float (&v)[4]) {
+  if constexpr (sizeof(TIn) == 2) {
+    const uint2 t = *reinterpret_cast<const uint2*>(p);
+    unpack_bf2(t.x, v[0], v[1]);
+    unpack_bf2(t.y, v[2], v[3]);
+  } else {
+    const float4 t = *reinterpret_cast<const float4*>(p);
+    v[0] = t.x, v[1] = t.y, v[2] = t.z, v[3] = t.w;
+  }
+}
+template <typename TIn>
+__global__ void __launch_bounds__(256)
+gemm_f32_group_kernel(const TIn* __restrict__ x, const TIn* __restrict__ w, const float* __restrict__ bias,
+                      float* __restrict__ out, long long T, int N, int K, long long x_stride, long long w_stride,
+                      long long out_stride) {
+  pdl_trigger();
+  pdl_wait();
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, l = lane & 7;
+  const long long t0 = (long long)blockIdx.x * GF_TOKENS + (warp & 1) * 4;
+  const int n0 = (int)blockIdx.y * GF_FEATURES + (warp >> 1) * 16 + (lane >> 3) * 4;
+  const TIn *xr[4], *wr[4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    xr[i] = x + (t0 + i < T ? t0 + i : T - 1) * x_stride + 4 * l;
+    wr[i] = w + (long long)min(n0 + i, N - 1) * w_stride + 4 * l;
+  }
+  float acc[4][4][4] = {};
+#pragma unroll 2
+  for (int k = 0; k < K; k += 32) {
+    float a[4][4], b[4][4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) gf_load(xr[i] + k, a[i]);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) gf_load(wr[i] + k, b[i]);
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) acc[i][j][e] = fmaf(a[i][e], b[j][e], acc[i][j][e]);
+  }
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      // partial sum 4 l + e: the butterfly's steps 16, 8, 4 are lanes l ^ 4, l ^ 2, l ^ 1, then 2 and 1 are e
+      float s[4];
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        s[e] = acc[i][j][e];
+#pragma unroll
+        for (int o = 4; o > 0; o >>= 1) s[e] += __shfl_xor_sync(0xffffffffu, s[e], o);
+      }
+      const float v = (s[0] + s[2]) + (s[1] + s[3]);
+      if (l == 0 && t0 + i < T && n0 + j < N) out[(t0 + i) * out_stride + n0 + j] = v + (bias ? bias[n0 + j] : 0.f);
+    }
+}
+
+// From about seven full warps of grouped outputs per SM on; fewer outputs keep a warp each, for the latency.
+template <typename TIn>
+inline int gemm_f32_launch(const void* x, const void* w, const void* bias, void* out, long long T, int N, int K,
+                           long long x_stride, long long w_stride, long long out_stride, cudaStream_t st) {
+  const long long tiles = (T + GF_TOKENS - 1) / GF_TOKENS;
+  const bool vec = K % 32 == 0 && x_stride % 4 == 0 && w_stride % 4 == 0 &&
+                   ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(w)) & (4 * sizeof(TIn) - 1)) == 0;
+  if (vec && T * N >= 65536 && tiles <= 0x7fffffffLL && (N + GF_FEATURES - 1) / GF_FEATURES <= 65535) {
+    launch_k(gemm_f32_group_kernel<TIn>, dim3((unsigned)tiles, (unsigned)((N + GF_FEATURES - 1) / GF_FEATURES)), dim3(256), 0, st,
+             (const TIn*)x, (const TIn*)w, (const float*)bias, (float*)out, T, N, K, x_stride, w_stride, out_stride);
+    return launch_status();
+  }
+  launch_k(gemm_f32_kernel<TIn>, dim3((unsigned)((T * N + 7) / 8)), dim3(256), 0, st, (const TIn*)x, (const TIn*)w,
+           (const float*)bias, (float*)out, T, N, K, x_stride, w_stride, out_stride);
+  return launch_status();
+}
 }  // namespace b200
 
 namespace b200 {
@@ -909,11 +989,7 @@ extern "C" int b200_gemm_f32(const void* x, const void* w, const void* bias, voi
   using namespace b200;
   if (!x || !w || !out || T < 0 || N <= 0 || K <= 0) return B200_ERR_ARG;
   if (T == 0) return B200_OK;
-  const long long warps = T * N;
-  launch_k(gemm_f32_kernel<float>, dim3((unsigned)((warps + 7) / 8)), dim3(256), 0, (cudaStream_t)stream,
-           (const float*)x, (const float*)w, (const float*)bias, (float*)out, T, N, K, x_row_stride, w_row_stride,
-           out_row_stride);
-  return launch_status();
+  return gemm_f32_launch<float>(x, w, bias, out, T, N, K, x_row_stride, w_row_stride, out_row_stride, (cudaStream_t)stream);
 }
 
 // The DeepSeek-V3 router on bf16 tensors: out_f32[T, N] = float(x) @ float(w)^T, bit-identical to
@@ -925,11 +1001,7 @@ extern "C" int b200_gemm_f32_from_bf16(const void* x, const void* w, void* out, 
   using namespace b200;
   if (!x || !w || !out || T < 0 || N <= 0 || K <= 0) return B200_ERR_ARG;
   if (T == 0) return B200_OK;
-  const long long warps = T * N;
-  launch_k(gemm_f32_kernel<__nv_bfloat16>, dim3((unsigned)((warps + 7) / 8)), dim3(256), 0, (cudaStream_t)stream,
-           (const __nv_bfloat16*)x, (const __nv_bfloat16*)w, (const float*)nullptr, (float*)out, T, N, K,
-           x_row_stride, w_row_stride, out_row_stride);
-  return launch_status();
+  return gemm_f32_launch<__nv_bfloat16>(x, w, nullptr, out, T, N, K, x_row_stride, w_row_stride, out_row_stride, (cudaStream_t)stream);
 }
 
 // out[T, N] = x[T, K] @ w[N, K]^T (+ bias[N], added in fp32 before the cast).
