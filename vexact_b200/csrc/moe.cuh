@@ -346,6 +346,10 @@ moe_route_sigmoid_group_topk_kernel(const float* __restrict__ logits, long long 
 // warp's private per-expert counter, so every entry learns its rank among the warp's earlier
 // entries of the same expert.  A per-expert scan over the 32 warps and a scan over the experts
 // turn those ranks into global positions.  All of it is integer arithmetic: bit-exact.
+//
+// The walk is bound by the latency of its loads (16384 / 32768 entries took 25 / 47 us one step at a time), so a warp requests
+// eight steps' entries at once.
+constexpr int MOE_INDEX_AHEAD = 8;
 template <typename TIdx>
 __global__ void __launch_bounds__(1024)
 moe_index_kernel(const TIdx* __restrict__ experts, long long n, int E, int tile_rows,
@@ -364,27 +368,36 @@ moe_index_kernel(const TIdx* __restrict__ experts, long long n, int E, int tile_
   const long long seg = ((n + 31) / 32 + 31) / 32 * 32;  // entries per warp, a multiple of 32
   const long long w0 = warp * seg;
   // pass 1: rank of every entry among the warp's earlier entries of the same expert
-  for (long long o = 0; o < seg; o += 32) {
-    const long long i = w0 + o + lane;
-    int e = -1;
-    if (i < n) {
-      const long long ev = (long long)experts[i];
-      if (ev >= 0 && ev < E)
-        e = (int)ev;
-      else
-        report_status(B200_STATUS_BAD_INDEX, (int)ev);
+  for (long long o = 0; o < seg; o += 32 * MOE_INDEX_AHEAD) {
+    long long ev[MOE_INDEX_AHEAD];
+#pragma unroll
+    for (int u = 0; u < MOE_INDEX_AHEAD; ++u) {
+      const long long i = w0 + o + 32 * u + lane;
+      ev[u] = o + 32 * u < seg && i < n ? (long long)experts[i] : -1;
     }
-    const unsigned mask = __match_any_sync(0xffffffffu, e);
-    const int rank = __popc(mask & ((1u << lane) - 1u));
-    const int leader = __ffs(mask) - 1;
-    int old = 0;
-    if (rank == 0 && e >= 0) {
-      old = cnt[warp][e];
-      cnt[warp][e] = old + __popc(mask);
+#pragma unroll
+    for (int u = 0; u < MOE_INDEX_AHEAD; ++u) {
+      if (o + 32 * u >= seg) break;
+      const long long i = w0 + o + 32 * u + lane;
+      int e = -1;
+      if (i < n) {
+        if (ev[u] >= 0 && ev[u] < E)
+          e = (int)ev[u];
+        else
+          report_status(B200_STATUS_BAD_INDEX, (int)ev[u]);
+      }
+      const unsigned mask = __match_any_sync(0xffffffffu, e);
+      const int rank = __popc(mask & ((1u << lane) - 1u));
+      const int leader = __ffs(mask) - 1;
+      int old = 0;
+      if (rank == 0 && e >= 0) {
+        old = cnt[warp][e];
+        cnt[warp][e] = old + __popc(mask);
+      }
+      old = __shfl_sync(0xffffffffu, old, leader);
+      if (i < n) scatter_index[i] = e >= 0 ? old + rank : -1;
+      __syncwarp();
     }
-    old = __shfl_sync(0xffffffffu, old, leader);
-    if (i < n) scatter_index[i] = e >= 0 ? old + rank : -1;
-    __syncwarp();
   }
   __syncthreads();
   // per expert: exclusive scan over the warps, total into base[]
@@ -442,12 +455,21 @@ moe_index_kernel(const TIdx* __restrict__ experts, long long n, int E, int tile_
   }
   __syncthreads();
   // pass 2: local rank -> global position
-  for (long long o = 0; o < seg; o += 32) {
-    const long long i = w0 + o + lane;
-    if (i < n) {
-      const long long ev = (long long)experts[i];
-      if (ev >= 0 && ev < E) {
-        const int pos = scatter_index[i] + base[(int)ev] + cnt[warp][(int)ev];
+  for (long long o = 0; o < seg; o += 32 * MOE_INDEX_AHEAD) {
+    long long ev[MOE_INDEX_AHEAD];
+    int rank[MOE_INDEX_AHEAD];
+#pragma unroll
+    for (int u = 0; u < MOE_INDEX_AHEAD; ++u) {
+      const long long i = w0 + o + 32 * u + lane;
+      const bool in = o + 32 * u < seg && i < n;
+      ev[u] = in ? (long long)experts[i] : -1;
+      rank[u] = in ? scatter_index[i] : 0;
+    }
+#pragma unroll
+    for (int u = 0; u < MOE_INDEX_AHEAD; ++u) {
+      const long long i = w0 + o + 32 * u + lane;
+      if (ev[u] >= 0 && ev[u] < E) {
+        const int pos = rank[u] + base[(int)ev[u]] + cnt[warp][(int)ev[u]];
         scatter_index[i] = pos;
         // the inverse map for a GEMM that gathers its rows (sorted row -> token), and the routing weight
         // of each sorted row, so that no permuted copy of the activations has to be made
