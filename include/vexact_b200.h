@@ -347,6 +347,10 @@ int b200_moe_grouped_dgrad(const void* x, const void* w, const void* w2, void* o
 int b200_moe_grouped_dgrad_noalloc(const void* x, const void* w, void* out, const void* cu_seqlens, long long x_rows,
                                    int num_groups, int n_out, int K, long long out_row_stride, void* stream);
 
+/* No counterpart in the reference: order [n] receives the indices of context_lens [n] (both int32) by descending value,
+ * ties by index, as b200_paged_attn_fwd_ordered takes them.  n <= 4096. */
+int b200_seq_order(const void* context_lens_i32, void* order_i32, int n, void* stream);
+
 /* ---- vexact/batch_invariant_ops/fused_moe.py:113-236: the backward of b200_swiglu_scale with the rounding points of the
  *      chain of torch operators there; also writes what fc2 consumed (h_scaled) and the rows' gradient of the scale. */
 int b200_swiglu_backward(const void* gate, const void* up, long long in_row_stride, const void* d_h, const void* row_scale,

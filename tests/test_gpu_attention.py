@@ -594,3 +594,11 @@ def test_rows_kernel_for_192_wide_keys_gives_the_columns_kernels_bits(vb):
         one = vb.flash_attn_varlen_func(q[last], kc, vc, cu_seqlens_q=torch.arange(S + 1, dtype=torch.int32).cuda(),
                                         max_seqlen_q=1, seqused_k=used, page_table=table, softmax_scale=dk ** -0.5, causal=True)[0]
         assert torch.equal(one, rows[last])
+
+
+@pytest.mark.parametrize("n", [1, 2, 255, 256, 257, 4096])
+def test_sequences_by_descending_context(vb, n):
+    from vexact_b200.attention import descending_contexts
+
+    lens = torch.randint(0, 40, (n,), generator=torch.Generator().manual_seed(n)).int().cuda()     # many ties
+    assert torch.equal(descending_contexts(lens).long(), torch.sort(lens, descending=True, stable=True).indices)

@@ -90,6 +90,19 @@ def paged_attention(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tenso
     return out
 
 
+SEQ_ORDER_MAX = 4096      # sequences that `descending_contexts` ranks
+
+
+def descending_contexts(context_lens: torch.Tensor) -> torch.Tensor:
+    """int32 [num_seqs]: the sequences by descending context length, ties by index, for `paged_attention`'s seq_order."""
+    _require_cuda_int32("context_lens", context_lens)
+    lens = context_lens.contiguous()
+    order = torch.empty_like(lens)
+    _lib.check(_lib.load().b200_seq_order(lens.data_ptr(), order.data_ptr(), lens.numel(), _lib.current_stream()),
+               "b200_seq_order")
+    return order
+
+
 def flash_attn_varlen_func(
     q: torch.Tensor,
     k: torch.Tensor,

@@ -16,13 +16,13 @@ libvexact_b200.so.  The whole stage forward is captured in a CUDA graph per toke
 from __future__ import annotations
 
 import os
-from dataclasses import dataclass, field
+from dataclasses import dataclass, field, replace
 from typing import Optional
 
 import torch
 
 from . import _lib
-from .attention import paged_attention
+from .attention import SEQ_ORDER_MAX, descending_contexts, paged_attention
 from .batch_invariant_ops import add_rms_norm, batch_invariant_rms_norm, hf_rms_norm, linear, linear_f32_from_bf16
 from .fused_moe import (TILE_ROWS, PendingMoE, _grouped_gemm, fused_moe_forward, route_plan_softmax_topk,
                         route_sigmoid_group_topk,
@@ -36,6 +36,9 @@ BF = torch.bfloat16
 # default: inside the captured decode step it measured 0.0-0.5 % (32.04 -> 31.87-32.04 ms), within run-to-run
 # noise, and the stable order is the simpler thing to reason about.
 _ROUTE_PLAN = os.environ.get("B200_MOE_ROUTE_PLAN", "0") == "1"
+# (sequence, KV head) pairs from which a step without an order ranks its sequences by context: about one per SM, below which
+# no persistent attention CTA has a second tile
+ORDER_MIN_TILES = 148
 
 
 @dataclass(frozen=True)
@@ -408,6 +411,9 @@ class StageRunner:
 
     def forward(self, inp: StepInputs) -> torch.Tensor:
         """Hidden states after the local layers ([T, H]); the residual stream is complete."""
+        if inp.seq_order is None and ORDER_MIN_TILES < inp.context_lens.numel() * self.shape.num_kv_heads \
+                and inp.context_lens.numel() <= SEQ_ORDER_MAX:
+            inp = replace(inp, seq_order=descending_contexts(inp.context_lens))
         if self.is_first:
             h = _gather_rows(self.w.embed, ids=inp.input_ids)
         else:
