@@ -447,7 +447,7 @@ def run_skew(args, shape):
     under near-uniform routing (router std 0.02) and under the Zipf(1.1) router bias."""
     import vexact_b200 as vb
     from vexact_b200 import _lib
-    from vexact_b200.fused_moe import FUSED_SWIGLU_MAX_ROWS_PER_EXPERT, _grouped_gemm, _permute
+    from vexact_b200.fused_moe import _grouped_gemm, _permute
 
     dev = torch.device("cuda", 0)
     torch.cuda.set_device(dev)
@@ -484,9 +484,7 @@ def run_skew(args, shape):
         plan = _permute(sel, rw, hidden, E)
         xp, rs = plan["x_perm"], plan["row_scale"]
         hit = int((counts > 0).sum())
-        fused = T * k <= FUSED_SWIGLU_MAX_ROWS_PER_EXPERT * E
-        fc1 = (lambda: _grouped_gemm(xp, gate_up, rs, plan, I, mode=1)) if fused else \
-              (lambda: _grouped_gemm(xp, gate_up, None, plan, 2 * I, mode=0))
+        fc1 = lambda: _grouped_gemm(xp, gate_up, rs, plan, I, mode=1)
         hmid = _grouped_gemm(xp, gate_up, rs, plan, I, mode=1)
         e = {"rows_per_expert_max": int(counts.max()), "rows_per_expert_mean": float(counts.float().mean()),
              "experts_hit": hit, "token_tiles": int(plan["tile_count"].item()),

@@ -357,6 +357,11 @@ int b200_swiglu_backward(const void* gate, const void* up, long long in_row_stri
                          void* h_scaled, void* d_gate, void* d_up, long long d_row_stride, void* d_scale, long long rows,
                          int I, void* stream);
 
+/* ---- vexact/batch_invariant_ops/fused_moe.py:319-336 for one dense MLP: out[t, i] = silu(x[t] . w[i]) *
+ *      (x[t] . w[n_out + i]), w [2 * n_out, K] with the gate rows first; each product, silu and the result bf16. */
+int b200_gemm_swiglu(const void* x, const void* w, void* out, long long T, int n_out, int K, long long x_row_stride,
+                     long long w_row_stride, long long out_row_stride, void* stream);
+
 /* ---- vexact/batch_invariant_ops/fused_moe.py:325-336 for split gate / up weights. */
 int b200_swiglu_scale(const void* gate, const void* up, const void* row_scale, void* out, long long rows,
                       int I, void* stream);

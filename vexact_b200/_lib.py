@@ -97,6 +97,7 @@ SIGNATURES = {
     "b200_moe_unpermute_reduce": [P, P, P, P, LL, I, I, P],
     "b200_moe_scatter": [P, LL, P, LL, LL, P, LL, LL, I, I, P],
     "b200_moe_gather": [P, LL, P, LL, LL, P, LL, I, I, P],
+    "b200_gemm_swiglu": [P, P, P, LL, I, I, LL, LL, LL, P],
     "b200_seq_order": [P, P, I, P],
     "b200_moe_grouped_dgrad": [P, P, P, P, P, P, LL, I, I, I, LL, I, I, P],
     "b200_moe_grouped_dgrad_noalloc": [P, P, P, P, LL, I, I, I, LL, P],

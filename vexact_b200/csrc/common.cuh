@@ -81,6 +81,19 @@ __device__ __forceinline__ Two fma2(const Two& a, const Two& b, const Two& c) {
   return r;
 }
 
+// 1 / (1 + exp(-g)) on the special-function unit: 2^x and 1 / x with relative errors below 2^-22, far inside the bf16 rounding
+// that follows every use (the exact exponential and division took 45 of the 60 instructions per element of the SwiGLU kernels,
+// which they bound).  exp(-g) = inf gives 0.
+__device__ __forceinline__ float sigmoid_sfu(float g) {
+  float e, r;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e) : "f"(g * -1.4426950408889634f));
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(1.f + e));
+  return r;
+}
+// One element of the expert and dense SwiGLU with the rounding points of fused_moe.py:319-336: silu(g) and its product with u
+// are bf16 tensors.
+__device__ __forceinline__ float swiglu_reference(float g, float u) { return round_bf(round_bf(g * sigmoid_sfu(g)) * u); }
+
 // Fixed butterfly reductions over a full warp.
 __device__ __forceinline__ float warp_sum(float v) {
 #pragma unroll

@@ -42,7 +42,7 @@ constexpr int GEMM_WBYTES = GEMM_WTILE * GEMM_BK * 2;
 constexpr int GEMM_THREADS = 192;       // producer warp, MMA warp, 4 epilogue warps
 constexpr int GEMM_MAX_STAGES = 12;
 constexpr int GEMM_SMEM_BUDGET = 227 * 1024;
-constexpr int GEMM_EXCH_PAD = 8;  // the SwiGLU exchange buffer holds xrows_max + 8 bf16 per feature row
+constexpr int GEMM_EXCH_PAD = 2;  // the SwiGLU exchange buffer holds xrows_max + 2 bf16 per feature row: an odd pitch in words
 
 struct GemmParams {
   int n_w;               // output features per group (plain: N; SwiGLU: intermediate size I)
@@ -261,18 +261,21 @@ gemm_ws_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__
   // requests its first ring of weight tiles before it waits, so that under programmatic dependent launch
   // their HBM latency runs alongside the predecessor's tail.
   int prefetched = 0;
-  if (warp == 0 && !SWIGLU && !p.tile_table && !p.gather_idx) {
+  if (warp == 0 && !p.tile_table && !p.gather_idx) {
     GemmTile t;
     if (gemm_tile(p, p.dense_t_tiles, blockIdx.x, t)) {   // the same for every lane
       prefetched = num_kb < S ? num_kb : S;
       if (ptx::elect_one()) {
         const uint32_t tx = GEMM_WBYTES + (uint32_t)gemm_tile_cols(p, t.n) * (GEMM_BK * 2);
-        const int wrow = t.group * p.w_rows_per_group + t.wt * GEMM_WTILE;
+        const int wrow = t.group * p.w_rows_per_group + t.wt * (SWIGLU ? 64 : GEMM_WTILE);
         for (int kb = 0; kb < prefetched; ++kb) {
           ptx::mbar_expect_tx(full_bar(kb), tx * KA);
-          for (int a = 0; a < KA; ++a)
-            ptx::tma_load_2d(stage_base + (uint32_t)kb * stage_bytes + (uint32_t)a * atom_bytes, &tm_w, full_bar(kb),
-                             (kb * KA + a) * GEMM_BK, wrow, p.w_policy);
+          for (int a = 0; a < KA; ++a) {
+            const uint32_t sw = stage_base + (uint32_t)kb * stage_bytes + (uint32_t)a * atom_bytes;
+            const int kcol = (kb * KA + a) * GEMM_BK;
+            ptx::tma_load_2d(sw, &tm_w, full_bar(kb), kcol, wrow, p.w_policy);
+            if (SWIGLU) ptx::tma_load_2d(sw + 64 * GEMM_BK * 2, &tm_w, full_bar(kb), kcol, wrow + p.up_offset, p.w_policy);
+          }
         }
       }
     }
@@ -624,53 +627,64 @@ gemm_ws_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__
           }
         }
       } else {
-        // Lanes 0..63 hold the gate rows, lanes 64..127 the up rows of the same 64 features.
+        // Lanes 0..63 hold the gate rows, lanes 64..127 the up rows of the same 64 features.  In the reference form, whose
+        // gate is a bf16 tensor too, both pairs of warps do the activation: the gate warps for the first half of the columns,
+        // the up warps for the rest, each handing the other what it lacks.  (With the exact exponential and the gate warps
+        // alone this bound the kernel at many rows per expert, and prefill took two plain products and an elementwise
+        // kernel: 2 x 49 + 30 us for 2048 tokens, 1536 -> 8960.)
         const int fi = (q & 1) * 32 + lane;
-        if (q >= 2) {
-          for (int c0 = 0; c0 < ncol; c0 += 16) {
-            uint32_t r[16];
-            ptx::tmem_ld16(taddr + c0, r);
-            ptx::tmem_ld_wait();
+        const bool both = p.glu == GLU_REFERENCE;
+        const int mid = both ? (ncol / 16 + 1) / 2 * 16 : ncol;
+        const int give0 = q < 2 ? mid : 0, give1 = q < 2 ? ncol : mid, take0 = q < 2 ? 0 : mid, take1 = q < 2 ? mid : ncol;
+        __nv_bfloat16* mine = exch + fi * exch_pitch;
+        for (int c0 = give0; c0 < give1; c0 += 16) {
+          uint32_t r[16];
+          ptx::tmem_ld16(taddr + c0, r);
+          ptx::tmem_ld_wait();
 #pragma unroll
-            for (int j = 0; j < 16; ++j) exch[fi * exch_pitch + c0 + j] = f2bf(__uint_as_float(r[j]));
-          }
+          for (int j = 0; j < 16; j += 2)
+            *reinterpret_cast<uint32_t*>(mine + c0 + j) = pack_bf2(__uint_as_float(r[j]), __uint_as_float(r[j + 1]));
         }
         ptx::named_barrier_sync(1, 128);
-        if (q < 2) {
-          const int f = t.wt * 64 + fi;
-          const bool fvalid = f < p.n_w;
-          for (int c0 = 0; c0 < ncol; c0 += 16) {
-            uint32_t r[16];
-            ptx::tmem_ld16(taddr + c0, r);
-            ptx::tmem_ld_wait();
-            if (fvalid && p.glu != GLU_REFERENCE) {
+        const int f = t.wt * 64 + fi;
+        const bool fvalid = f < p.n_w;
+        for (int c0 = take0; c0 < take1; c0 += 16) {
+          uint32_t r[16];
+          ptx::tmem_ld16(taddr + c0, r);
+          ptx::tmem_ld_wait();
+          float other[16];
 #pragma unroll
-              for (int j = 0; j < 16; ++j) {
-                const int c = c0 + j;
-                if (c < t.n) {
-                  const float si = p.scale_in ? p.scale_in[t.row0 + c] : 1.f;
-                  const float so = p.scale_out ? p.scale_out[t.row0 + c] : 1.f;
-                  const float u = bf2f(exch[fi * exch_pitch + c]);
-                  reinterpret_cast<__nv_bfloat16*>(p.out)[(long long)(t.row0 + c) * p.ldo + f] =
-                      f2bf(so * glu_value<__nv_bfloat16>(p.glu, si * __uint_as_float(r[j]), si * u));
-                }
-              }
-            } else if (fvalid) {
+          for (int j = 0; j < 16; j += 2)
+            unpack_bf2(*reinterpret_cast<const uint32_t*>(mine + c0 + j), other[j], other[j + 1]);
+          if (fvalid && !both) {
 #pragma unroll
-              for (int j = 0; j < 16; ++j) {
-                const int c = c0 + j;
-                if (c < t.n) {
-                  // Rounding points of fused_moe.py:319-336: each GEMM output, silu(), the
-                  // gate*up product and the routing-weight product are bf16 tensors.
-                  const float g = round_bf(__uint_as_float(r[j]));
-                  const float u = bf2f(exch[fi * exch_pitch + c]);
-                  const float sg = round_bf(g / (1.0f + expf(-g)));
-                  float h = round_bf(sg * u);
-                  if (p.row_scale) h = round_bf(h * bf2f(p.row_scale[t.row0 + c]));
-                  reinterpret_cast<__nv_bfloat16*>(p.out)[(long long)(t.row0 + c) * p.ldo + f] = f2bf(h);
-                }
+            for (int j = 0; j < 16; ++j) {
+              const int c = c0 + j;
+              if (c < t.n) {
+                const float si = p.scale_in ? p.scale_in[t.row0 + c] : 1.f;
+                const float so = p.scale_out ? p.scale_out[t.row0 + c] : 1.f;
+                reinterpret_cast<__nv_bfloat16*>(p.out)[(long long)(t.row0 + c) * p.ldo + f] =
+                    f2bf(so * glu_value<__nv_bfloat16>(p.glu, si * __uint_as_float(r[j]), si * other[j]));
               }
             }
+          } else if (fvalid) {
+            float h[16];
+#pragma unroll
+            for (int j = 0; j < 16; ++j) {
+              // rounding points of fused_moe.py:319-336: each GEMM output, silu(), the gate*up product and (below) the
+              // routing-weight product are bf16 tensors
+              const float own = round_bf(__uint_as_float(r[j]));
+              h[j] = swiglu_reference(q < 2 ? own : other[j], q < 2 ? other[j] : own);
+            }
+            if (p.row_scale) {
+#pragma unroll
+              for (int j = 0; j < 16; ++j)
+                if (c0 + j < t.n) h[j] *= bf2f(p.row_scale[t.row0 + c0 + j]);
+            }
+#pragma unroll
+            for (int j = 0; j < 16; ++j)
+              if (c0 + j < t.n)
+                reinterpret_cast<__nv_bfloat16*>(p.out)[(long long)(t.row0 + c0 + j) * p.ldo + f] = f2bf(h[j]);
           }
         }
         ptx::named_barrier_sync(1, 128);  // exchange buffer is reused by the next tile
@@ -1016,6 +1030,29 @@ struct GemmExtra {
   long long x_batch_stride = 0, w_batch_stride = 0, out_batch_stride = 0;
 };
 
+// Token tiling of a dense product, `features` outputs per weight tile.  A token's result does not depend on the tile it lands
+// in (tokens are independent UMMA columns), so the tile width is chosen for speed only.  Every tile streams K/64 stages of
+// (16 KiB of weights + 128 B per token) into shared memory and the persistent CTAs work through the tiles in rounds, so the
+// cost of a tiling is rounds x bytes per stage; take the cheapest.  (Tiles of fewer weight rows, to put one token's product on
+// more SMs, gain nothing: 6144 -> 2048 took 24 us with 128 rows a tile and 23 with 32.)
+inline void gemm_dense_tiles(GemmParams& p, long long T, int N, int batch, int features = GEMM_WTILE) {
+  const int sms = sm_count();
+  const int min_tiles = (int)((T + 255) / 256), max_tiles = (int)((T + 15) / 16);
+  long long best_cost = -1;
+  p.w_tiles = (N + features - 1) / features;
+  for (int tt = min_tiles; tt <= max_tiles; ++tt) {
+    const int rows = round_up((int)((T + tt - 1) / tt), 16);
+    const int tiles_t = (int)((T + rows - 1) / rows);
+    const long long rounds = ((long long)tiles_t * p.w_tiles * batch + sms - 1) / sms;
+    const long long cost = rounds * (GEMM_WBYTES + rows * GEMM_BK * 2);
+    if (best_cost < 0 || cost < best_cost) {
+      best_cost = cost;
+      p.rows_per_tile = rows;
+      p.dense_t_tiles = tiles_t;
+    }
+  }
+}
+
 inline int gemm_dense_16bit(const void* x, const void* w, const void* bias, void* out, long long T, int N, int K,
                             long long x_row_stride, long long w_row_stride, long long out_row_stride, int out_dtype,
                             bool fp16, void* stream, const GemmExtra& ex = GemmExtra()) {
@@ -1026,31 +1063,10 @@ inline int gemm_dense_16bit(const void* x, const void* w, const void* bias, void
   GemmParams p{};
   p.n_w = N;
   p.k = K;
-  p.w_tiles = (N + GEMM_WTILE - 1) / GEMM_WTILE;
   p.w_rows_per_group = N;
   p.up_offset = 0;
   p.t_rows = (int)T;
-  // Token tiling.  A token's result does not depend on the tile it lands in (tokens are independent
-  // UMMA columns), so the tile width is chosen for speed only.  Every tile streams K/64 stages of
-  // (16 KiB of weights + 128 B per token) into shared memory and the persistent CTAs work through
-  // the tiles in rounds, so the cost of a tiling is rounds x bytes per stage; take the cheapest.
-  {
-    const int sms = sm_count();
-    const int min_tiles = (int)((T + 255) / 256);
-    const int max_tiles = (int)((T + 15) / 16);
-    long long best_cost = -1;
-    for (int tt = min_tiles; tt <= max_tiles; ++tt) {
-      const int rows = round_up((int)((T + tt - 1) / tt), 16);
-      const int tiles_t = (int)((T + rows - 1) / rows);
-      const long long rounds = ((long long)tiles_t * p.w_tiles * ex.batch + sms - 1) / sms;
-      const long long cost = rounds * (GEMM_WBYTES + rows * GEMM_BK * 2);
-      if (best_cost < 0 || cost < best_cost) {
-        best_cost = cost;
-        p.rows_per_tile = rows;
-        p.dense_t_tiles = tiles_t;
-      }
-    }
-  }
+  gemm_dense_tiles(p, T, N, ex.batch);
   p.tile_table = nullptr;
   p.tile_count = nullptr;
   p.tokens_first = 1;
@@ -1092,6 +1108,45 @@ inline int gemm_dense_16bit(const void* x, const void* w, const void* bias, void
   return gemm_launch<GEMM_PLAIN>(tw, tx, p, (long long)p.w_tiles * p.dense_t_tiles * ex.batch, (cudaStream_t)stream);
 }
 }  // namespace b200
+
+namespace b200 {
+// One gated product over T rows as they lie (no tile table): w [2 * n_out, K], gate rows first.
+inline int gemm_dense_gated(const void* x, const void* w, const void* scale_out, void* out, long long T, int n_out, int K,
+                            long long x_row_stride, long long w_row_stride, long long out_row_stride, int glu, void* stream) {
+  if (!x || !w || !out || T < 0 || n_out <= 0 || K <= 0) return B200_ERR_ARG;
+  if (K % 8 != 0 || x_row_stride % 8 != 0 || w_row_stride % 8 != 0 || T > 0x7fffffffLL) return B200_ERR_SHAPE;
+  if (T == 0) return B200_OK;
+  GemmParams p{};
+  p.n_w = n_out;
+  p.k = K;
+  p.w_rows_per_group = 2 * n_out;
+  p.up_offset = n_out;
+  p.t_rows = (int)T;
+  gemm_dense_tiles(p, T, n_out, 1, 64);
+  p.tokens_first = 1;
+  p.xbox = p.rows_per_tile;
+  p.xrows_max = p.rows_per_tile;
+  p.out = out;
+  p.ldo = out_row_stride;
+  p.glu = glu;
+  p.scale_out = (const float*)scale_out;
+  p.w_policy = p.dense_t_tiles == 1 ? ptx::kEvictFirst : ptx::kEvictNormal;
+  CUtensorMap tw;
+  GemmXMaps tx{};
+  int rc = make_tmap_2d(&tw, w, 2 * (uint64_t)n_out, (uint64_t)K, (uint64_t)w_row_stride, 64);
+  if (!rc) rc = make_tmap_2d(&tx.box[0], x, (uint64_t)T, (uint64_t)K, (uint64_t)x_row_stride, (uint32_t)p.xbox);
+  if (rc) return rc;
+  return gemm_launch<GEMM_SWIGLU>(tw, tx, p, (long long)p.w_tiles * p.dense_t_tiles, (cudaStream_t)stream);
+}
+}  // namespace b200
+
+// out[t, i] = silu(x[t] . w[i]) * (x[t] . w[n_out + i]) with the rounding points of the reference's chain (each product, silu
+// and the result are bf16).
+extern "C" int b200_gemm_swiglu(const void* x, const void* w, void* out, long long T, int n_out, int K, long long x_row_stride,
+                                long long w_row_stride, long long out_row_stride, void* stream) {
+  return b200::gemm_dense_gated(x, w, nullptr, out, T, n_out, K, x_row_stride, w_row_stride, out_row_stride, b200::GLU_REFERENCE,
+                                stream);
+}
 
 extern "C" int b200_gemm_bf16(const void* x, const void* w, const void* bias, void* out, long long T, int N,
                               int K, long long x_row_stride, long long w_row_stride, long long out_row_stride,
@@ -1374,34 +1429,8 @@ extern "C" int b200_moe_grouped_gemm_act(const void* x, const void* w, const voi
 // One product of the gated form over T rows as they lie (no tile table): w [2 * n_out, K].
 extern "C" int b200_gemm_glu(const void* x, const void* w, const void* scale_out_f32, void* out, long long T, int n_out,
                              int K, long long x_row_stride, long long out_row_stride, int act, void* stream) {
-  using namespace b200;
-  if (!x || !w || !out || T < 0 || n_out <= 0 || K <= 0 || (act != GLU_SILU && act != GLU_GELU_TANH)) return B200_ERR_ARG;
-  if (K % 8 != 0 || x_row_stride % 8 != 0 || T > 0x7fffffffLL) return B200_ERR_SHAPE;
-  if (T == 0) return B200_OK;
-  GemmParams p{};
-  p.n_w = n_out;
-  p.k = K;
-  p.w_tiles = (n_out + 63) / 64;
-  p.w_rows_per_group = 2 * n_out;
-  p.up_offset = n_out;
-  p.t_rows = (int)T;
-  p.rows_per_tile = T <= 64 ? round_up((int)T, 16) : 64;
-  p.dense_t_tiles = (int)((T + p.rows_per_tile - 1) / p.rows_per_tile);
-  p.tokens_first = 1;
-  p.xbox = p.rows_per_tile;
-  p.xrows_max = p.rows_per_tile;
-  p.out = out;
-  p.ldo = out_row_stride;
-  p.glu = act;
-  p.scale_out = (const float*)scale_out_f32;
-  p.w_policy = p.dense_t_tiles == 1 ? ptx::kEvictFirst : ptx::kEvictNormal;
-  CUtensorMap tw;
-  GemmXMaps tx{};
-  int rc = make_tmap_2d(&tw, w, (uint64_t)2 * n_out, (uint64_t)K, (uint64_t)K, 64);
-  if (rc) return rc;
-  rc = make_tmap_2d(&tx.box[0], x, (uint64_t)T, (uint64_t)K, (uint64_t)x_row_stride, (uint32_t)p.xbox);
-  if (rc) return rc;
-  return gemm_launch<GEMM_SWIGLU>(tw, tx, p, (long long)p.w_tiles * p.dense_t_tiles, (cudaStream_t)stream);
+  if (act != b200::GLU_SILU && act != b200::GLU_GELU_TANH) return B200_ERR_ARG;
+  return b200::gemm_dense_gated(x, w, scale_out_f32, out, T, n_out, K, x_row_stride, K, out_row_stride, act, stream);
 }
 
 // The grouped GEMM in true fp32: out[r, n] = x[r] . w[group, n], with act 3 as b200_moe_grouped_gemm_act; tile table

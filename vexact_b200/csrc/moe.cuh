@@ -826,8 +826,7 @@ transpose_last2_kernel(const uint16_t* __restrict__ x, uint16_t* __restrict__ ou
 
 // h = bf16(bf16(bf16(silu(g)) * u) * s): the unfused tail of fc1 for split gate / up weights.
 //
-// HBM-bound: 2 reads and a write of 2 bytes per element, about 45 instructions for the exact exponential and division.  A
-// thread takes VEC elements of one row (VEC = 8: 16-byte loads and stores, one index division for the eight); VEC = 1 serves
+// HBM-bound: 2 reads and a write of 2 bytes per element.  A thread takes VEC elements of one row (VEC = 8: 16-byte loads and stores, one index division for the eight); VEC = 1 serves
 // widths, strides and bases that 16-byte accesses do not fit.
 template <int VEC>
 __global__ void __launch_bounds__(256)
@@ -843,7 +842,7 @@ swiglu_scale_kernel(const __nv_bfloat16* __restrict__ gate, const __nv_bfloat16*
   const long long c = (i - r * per_row) * VEC, src = r * in_stride + c;
   const float s = row_scale ? bf2f(row_scale[r]) : 0.f;
   auto one = [&](float g, float u) {
-    const float h = round_bf(round_bf(g / (1.0f + expf(-g))) * u);
+    const float h = swiglu_reference(g, u);
     return row_scale ? round_bf(h * s) : h;
   };
   if constexpr (VEC == 8) {
@@ -894,7 +893,7 @@ swiglu_backward_kernel(const __nv_bfloat16* __restrict__ gate, const __nv_bfloat
       unpack_bf2(d4[j], d[0], d[1]);
 #pragma unroll
       for (int k = 0; k < 2; ++k) {
-        const float den = 1.f + expf(-g[k]), sig = 1.f / den, sg = round_bf(g[k] / den), act = round_bf(sg * u[k]);
+        const float sig = sigmoid_sfu(g[k]), sg = round_bf(g[k] * sig), act = round_bf(sg * u[k]);
         const float da = round_bf(d[k] * s);
         sum += round_bf(act * d[k]);
         oh[k] = act * s;

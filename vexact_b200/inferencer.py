@@ -24,7 +24,7 @@ import torch
 from . import _lib
 from .attention import SEQ_ORDER_MAX, descending_contexts, paged_attention
 from .batch_invariant_ops import add_rms_norm, batch_invariant_rms_norm, hf_rms_norm, linear, linear_f32_from_bf16
-from .fused_moe import (TILE_ROWS, PendingMoE, _grouped_gemm, fused_moe_forward, route_plan_softmax_topk,
+from .fused_moe import (PendingMoE, fused_moe_forward, route_plan_softmax_topk,
                         route_sigmoid_group_topk,
                         route_softmax_topk)
 from .standalone_logprobs import greedy_token_and_logprob, lm_head_greedy
@@ -292,28 +292,14 @@ class StageRunner:
         self.is_first = pp_rank == 0
         self.is_last = pp_rank == pp_size - 1
         self._graphs: dict = {}
-        self._dense_tiles: dict = {}
         # None = greedy; else dict(temperature=..., top_k=..., top_p=...) applied to every request
         self.sampling: Optional[dict] = None
         # greedy decoding without the [num_seqs, vocab] logits: lm_head and token selection fused
         # (`select_tokens` then returns None for the logits)
         self.fused_head = False
 
-    # -- dense MLP through the grouped-GEMM kernel's fused SwiGLU epilogue (one group)
-    def _dense_plan(self, T: int, device):
-        plan = self._dense_tiles.get(T)
-        if plan is None:
-            tile = TILE_ROWS
-            rows = [(0, r, min(tile, T - r), 0) for r in range(0, T, tile)]
-            plan = dict(tile_table=torch.tensor(rows, dtype=torch.int32, device=device),
-                        tile_count=torch.tensor([len(rows)], dtype=torch.int32, device=device),
-                        max_tiles=len(rows), tile_rows=tile)
-            self._dense_tiles[T] = plan
-        return plan
-
     def prepare(self, T: int, device="cuda") -> None:
-        """Build host-constructed constants for a token count (call before graph capture)."""
-        self._dense_plan(T, device)
+        """Hook before graph capture of a step of T tokens: nothing here depends on the token count."""
 
     def _norm(self, x, w):
         s = self.shape
@@ -366,23 +352,14 @@ class StageRunner:
                                (a.qk_nope + a.qk_rope) ** -0.5, inp.max_seqlen_q, seq_order=inp.seq_order)
         return linear(attn.view(T, heads * a.v_head), lw.o)
 
-    # Above this many tokens the fused SwiGLU epilogue (two of the four epilogue warps do the
-    # activation math of a whole 128 x 256 tile) costs more than it saves: two plain GEMMs and the
-    # elementwise kernel are used instead.  Both routes round at the same points, so a token's result
-    # is the same bits either way (tests/test_gpu_model.py).
-    DENSE_FUSED_MAX_TOKENS = 64
-
     def _dense_mlp(self, xn, gate_up, down, width):
         T = xn.shape[0]
-        if T <= self.DENSE_FUSED_MAX_TOKENS:
-            plan = self._dense_plan(T, xn.device)
-            act = _grouped_gemm(xn, gate_up.view(1, 2 * width, self.shape.hidden), None, plan, width, mode=1)
-        else:
-            g = linear(xn, gate_up[:width])
-            u = linear(xn, gate_up[width:])
-            act = torch.empty_like(g)
-            _lib.check(_lib.load().b200_swiglu_scale(g.data_ptr(), u.data_ptr(), None, act.data_ptr(), T, width,
-                                                     _lib.current_stream()), "b200_swiglu_scale")
+        act = torch.empty((T, width), device=xn.device, dtype=BF)
+        _lib.check(
+            _lib.load().b200_gemm_swiglu(xn.data_ptr(), gate_up.data_ptr(), act.data_ptr(), T, width, xn.shape[1],
+                                         xn.stride(0), gate_up.stride(0), act.stride(0), _lib.current_stream()),
+            "b200_gemm_swiglu",
+        )
         return linear(act, down)
 
     def _mlp_block(self, lw: LayerWeights, xn: torch.Tensor) -> torch.Tensor:
