@@ -209,3 +209,31 @@ def test_conv3d_under_the_mode_is_deterministic_and_batch_invariant(vb):
     finally:
         torch.backends.cudnn.enabled = cudnn_was
         torch.use_deterministic_algorithms(False)
+
+
+@pytest.mark.parametrize("T, N, K", [(1000, 128, 64), (1001, 200, 64), (1023, 384, 320), (1300, 1000, 72), (2048, 2056, 128),
+                                     (4097, 136, 2048), (1000, 2048, 200)])
+def test_products_on_cta_pairs_have_the_single_ctas_bits(vb, T, N, K):
+    """From 1000 tokens on a product may run on CTA pairs (odd and partial weight tiles, partial token tiles, K with and
+    without whole 64-wide atoms): every token's bits are those of the same token in a narrow batch, plain, with bias and gated."""
+    from vexact_b200 import _lib
+
+    gen = torch.Generator(device="cuda").manual_seed(T + N + K)
+    x, w = (torch.randn(r, K, device="cuda", generator=gen).to(torch.bfloat16) for r in (T, 2 * N))
+    bias = torch.randn(N, device="cuda", generator=gen).to(torch.bfloat16)
+
+    def gated(a):
+        out = torch.empty(a.shape[0], N, dtype=torch.bfloat16, device="cuda")
+        _lib.check(_lib.load().b200_gemm_swiglu(a.data_ptr(), w.data_ptr(), out.data_ptr(), a.shape[0], N, K, K, K, N,
+                                                _lib.current_stream()), "b200_gemm_swiglu")
+        return out
+
+    for f in (lambda a: vb.linear(a, w[:N]), lambda a: vb.linear(a, w[:N], bias), gated):
+        wide = f(x)
+        for r in (slice(0, 3), slice(T // 2 - 40, T // 2 + 41), slice(T - 130, T)):
+            assert torch.equal(wide[r], f(x[r]))
+    ref = x.double() @ w[:N].double().t()
+    torch.testing.assert_close(vb.linear(x, w[:N]).double(), ref, rtol=2 ** -8, atol=1e-6 * K)
+    g, u = (x.double() @ w.double().t()).to(torch.bfloat16).double().chunk(2, 1)
+    # three bf16 roundings after the products
+    torch.testing.assert_close(gated(x).double(), torch.nn.functional.silu(g) * u, rtol=2 ** -6, atol=2 ** -6 * K ** 0.5)

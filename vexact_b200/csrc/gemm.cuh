@@ -25,6 +25,13 @@
 // other accumulator (tcgen05.ld), apply the epilogue and store.  All waits are
 // bounded (ptx::mbar_wait).
 //
+// CTA pairs (PAIR).  A tile of 128 weight rows x 256 tokens takes 48 KB of operands per 64-element K step, 768 cycles of
+// shared-memory fill at 64 B a cycle against 512 of tensor pipe: wide tiles are bound by the fill (2048 tokens, 6144 -> 2048:
+// with three instructions in four left out, 35 us instead of 38).  Two CTAs of a cluster therefore work on 256 weight rows
+// x the same tokens (cta_group::2): each holds its own 128 weight rows and half of the token rows, 32 KB per step, and the
+// products come out as from a CTA's own instruction, to the bit.  4096 tokens, 1536 -> 8960: 79 us alone, 67 in pairs;
+// 2048 -> 10304: 111 and 94.
+//
 // Algorithmic bytes per launch: 2*(N*K + T*K + T*N); the weight term dominates
 // for decode shapes, so the roofline is HBM bandwidth.
 #pragma once
@@ -42,6 +49,10 @@ constexpr int GEMM_WBYTES = GEMM_WTILE * GEMM_BK * 2;
 constexpr int GEMM_THREADS = 192;       // producer warp, MMA warp, 4 epilogue warps
 constexpr int GEMM_MAX_STAGES = 12;
 constexpr int GEMM_SMEM_BUDGET = 227 * 1024;
+// Tokens from which a dense product may run on CTA pairs: their set-up and the meeting of the CTAs cost about a microsecond,
+// which narrow products do not gain back (2048 -> 4096 for 512 / 1000 / 2048 tokens: 13.4 / 18.3 / 29.1 us alone,
+// 14.4 / 17.8 / 26.9 in pairs).
+constexpr int GEMM_PAIR_TOKENS = 1000;
 constexpr int GEMM_EXCH_PAD = 2;  // the SwiGLU exchange buffer holds xrows_max + 2 bf16 per feature row: an odd pitch in words
 
 struct GemmParams {
@@ -169,7 +180,9 @@ struct GemmXMaps {
 };
 
 // Token columns that a tile of n rows occupies in shared and tensor memory.
+template <bool PAIR>
 __device__ __forceinline__ int gemm_tile_cols(const GemmParams& p, int n) {
+  if (PAIR) return p.split_boxes ? (n + 31) & ~31 : 2 * p.xbox;   // half in either CTA, in whole steps of 16
   return p.split_boxes ? (n + 15) & ~15 : (n + p.xbox - 1) / p.xbox * p.xbox;
 }
 
@@ -202,12 +215,20 @@ __device__ __forceinline__ bool gemm_tile(const GemmParams& p, int t_tiles, long
   return true;
 }
 
-template <int MODE>
+template <int MODE, bool PAIR>
 __global__ void __launch_bounds__(GEMM_THREADS, 1)
 gemm_ws_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ GemmXMaps tm_xs,
                const GemmParams p) {
   constexpr bool SWIGLU = MODE == GEMM_SWIGLU;
   constexpr bool HEAD = MODE == GEMM_HEAD, W_MN = MODE == GEMM_DGRAD;
+  // place in the pair, and this CTA's or pair's place in the tile walk (a pair's weight tile is two)
+  const int rank = PAIR ? (int)ptx::cluster_rank() : 0;
+  const long long lin0 = PAIR ? blockIdx.x >> 1 : blockIdx.x, lin_step = PAIR ? gridDim.x >> 1 : gridDim.x;
+  auto tile_at = [&](int t_tiles, long long lin, GemmTile& t) {
+    if (!gemm_tile(p, t_tiles, lin, t)) return false;
+    if (PAIR) t.wt = 2 * t.wt + rank;
+    return true;
+  };
   const CUtensorMap& tm_x = tm_xs.box[0];
   extern __shared__ uint8_t smem_raw[];
   if (threadIdx.x == 0) GEMM_STAMP(0);   // CTA started
@@ -218,7 +239,7 @@ gemm_ws_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem_raw + (2 * GEMM_MAX_STAGES + 4) * 8 + 8);
   const uint32_t smem_base = ptx::smem_u32(smem_raw);
   const uint32_t stage_base = (smem_base + 256 + 1023) & ~1023u;
-  const int atom_bytes = GEMM_WBYTES + p.xrows_max * (GEMM_BK * 2);
+  const int atom_bytes = GEMM_WBYTES + p.xrows_max / (PAIR ? 2 : 1) * (GEMM_BK * 2);
   const int KA = p.katoms;
   const int stage_bytes = atom_bytes * KA;
   __nv_bfloat16* exch =
@@ -239,23 +260,41 @@ gemm_ws_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__
     }
     for (int b = 0; b < 2; ++b) {
       ptx::mbar_init(tfull_bar(b), 1);
-      ptx::mbar_init(tempty_bar(b), 128);
+      ptx::mbar_init(tempty_bar(b), PAIR ? 8 : 128);   // pairs: the epilogue warps of both CTAs, on rank 0's barrier
     }
     ptx::fence_barrier_init();
     ptx::prefetch_tensormap(&tm_w);
     ptx::prefetch_tensormap(&tm_x);
   }
   if (warp == 1) {
-    ptx::tmem_alloc(ptx::smem_u32(tmem_slot), (uint32_t)p.tmem_cols);
-    ptx::tmem_relinquish();
+    if (PAIR) {
+      ptx::tmem_alloc_pair(ptx::smem_u32(tmem_slot), (uint32_t)p.tmem_cols);
+      ptx::tmem_relinquish_pair();
+    } else {
+      ptx::tmem_alloc(ptx::smem_u32(tmem_slot), (uint32_t)p.tmem_cols);
+      ptx::tmem_relinquish();
+    }
   }
   ptx::tc_fence_before();
   __syncthreads();
+  if (PAIR) ptx::cluster_sync();   // both CTAs' barriers are up before either is signalled from the other
   ptx::tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
   pdl_trigger();
   if (threadIdx.x == 0) GEMM_STAMP(1);   // set-up done
   const int num_kb = (p.k + GEMM_BK * KA - 1) / (GEMM_BK * KA);  // K beyond the tensor reads as zero
+  // A pair's copies complete on the barrier of rank 0, which arms it for both CTAs' bytes.
+  auto load_2d = [&](uint32_t dst, const CUtensorMap* map, int s, int x, int y, uint64_t policy) {
+    if (PAIR) ptx::tma_load_2d_pair(dst, map, ptx::cluster_addr(full_bar(s), 0), x, y, policy);
+    else ptx::tma_load_2d(dst, map, full_bar(s), x, y, policy);
+  };
+  auto load_3d = [&](uint32_t dst, const CUtensorMap* map, int s, int x, int y, int z, uint64_t policy) {
+    if (PAIR) ptx::tma_load_3d_pair(dst, map, ptx::cluster_addr(full_bar(s), 0), x, y, z, policy);
+    else ptx::tma_load_3d(dst, map, full_bar(s), x, y, z, policy);
+  };
+  auto arm = [&](int s, uint32_t bytes) {
+    if (!PAIR || rank == 0) ptx::mbar_expect_tx(full_bar(s), bytes);
+  };
   // Everything above is set-up.  What the previous kernel wrote (activations, the tile table) is read only
   // after pdl_wait().  The weights are not its output: with a static tiling (no tile table) the producer
   // requests its first ring of weight tiles before it waits, so that under programmatic dependent launch
@@ -263,18 +302,18 @@ gemm_ws_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__
   int prefetched = 0;
   if (warp == 0 && !p.tile_table && !p.gather_idx) {
     GemmTile t;
-    if (gemm_tile(p, p.dense_t_tiles, blockIdx.x, t)) {   // the same for every lane
+    if (tile_at(p.dense_t_tiles, lin0, t)) {   // the same for every lane
       prefetched = num_kb < S ? num_kb : S;
       if (ptx::elect_one()) {
-        const uint32_t tx = GEMM_WBYTES + (uint32_t)gemm_tile_cols(p, t.n) * (GEMM_BK * 2);
+        const uint32_t tx = (PAIR ? 2 : 1) * GEMM_WBYTES + (uint32_t)gemm_tile_cols<PAIR>(p, t.n) * (GEMM_BK * 2);
         const int wrow = t.group * p.w_rows_per_group + t.wt * (SWIGLU ? 64 : GEMM_WTILE);
         for (int kb = 0; kb < prefetched; ++kb) {
-          ptx::mbar_expect_tx(full_bar(kb), tx * KA);
+          arm(kb, tx * KA);
           for (int a = 0; a < KA; ++a) {
             const uint32_t sw = stage_base + (uint32_t)kb * stage_bytes + (uint32_t)a * atom_bytes;
             const int kcol = (kb * KA + a) * GEMM_BK;
-            ptx::tma_load_2d(sw, &tm_w, full_bar(kb), kcol, wrow, p.w_policy);
-            if (SWIGLU) ptx::tma_load_2d(sw + 64 * GEMM_BK * 2, &tm_w, full_bar(kb), kcol, wrow + p.up_offset, p.w_policy);
+            load_2d(sw, &tm_w, kb, kcol, wrow, p.w_policy);
+            if (SWIGLU) load_2d(sw + 64 * GEMM_BK * 2, &tm_w, kb, kcol, wrow + p.up_offset, p.w_policy);
           }
         }
       }
@@ -283,7 +322,7 @@ gemm_ws_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__
   pdl_wait();
   const int t_tiles = p.tile_table ? *p.tile_count : p.dense_t_tiles;
 
-  if (warp == 0 && p.gather_idx) {
+  if (!PAIR && warp == 0 && p.gather_idx) {
     // ------------------------------------------------------------ TMA producer, gathered activation rows
     // The whole warp runs the loop: lane 0 arms the barrier and loads the weights, lane l fetches rows
     // 4l .. 4l+3 of the tile by index.  Rows past the tile's end repeat its first row (their columns are
@@ -341,11 +380,12 @@ gemm_ws_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__
       int s = 0;         // ring slot of `it`
       uint32_t ph = 0;   // parity of the slot's current use
       bool ok = true;
-      for (long long lin = blockIdx.x; ok; lin += gridDim.x) {
+      for (long long lin = lin0; ok; lin += lin_step) {
         GemmTile t;
-        if (!gemm_tile(p, t_tiles, lin, t)) break;
-        const int cols = gemm_tile_cols(p, t.n);
-        const uint32_t tx = GEMM_WBYTES + (uint32_t)cols * (GEMM_BK * 2);
+        if (!tile_at(t_tiles, lin, t)) break;
+        const int cols = gemm_tile_cols<PAIR>(p, t.n);
+        const uint32_t tx = (PAIR ? 2 : 1) * GEMM_WBYTES + (uint32_t)cols * (GEMM_BK * 2);
+        const int own = PAIR ? cols / 2 : cols, row0 = t.row0 + rank * own;   // token rows of this CTA
         const int wrow = t.group * p.w_rows_per_group + t.wt * (SWIGLU ? 64 : GEMM_WTILE);
         for (int kb = 0; kb < num_kb; ++kb, ++it, s = (s + 1 == S ? 0 : s + 1), ph ^= (s == 0)) {
           // the first tile's first `prefetched` stages were armed, and their weights requested, before pdl_wait
@@ -355,7 +395,7 @@ gemm_ws_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__
               ok = false;
               break;
             }
-            ptx::mbar_expect_tx(full_bar(s), tx * KA);
+            arm(s, tx * KA);
           }
           for (int a = 0; a < KA; ++a) {
             const uint32_t sw = stage_base + (uint32_t)s * stage_bytes + (uint32_t)a * atom_bytes;
@@ -366,30 +406,30 @@ gemm_ws_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__
               const bool second = p.k_second && kcol >= p.k_second;
 #pragma unroll
               for (int h = 0; h < 2; ++h)
-                ptx::tma_load_3d(sw + h * (GEMM_WBYTES / 2), second ? &tm_xs.w2 : &tm_w, full_bar(s), t.wt * GEMM_WTILE + h * 64,
+                load_3d(sw + h * (GEMM_WBYTES / 2), second ? &tm_xs.w2 : &tm_w, s, t.wt * GEMM_WTILE + h * 64,
                                  second ? kcol - p.k_second : kcol, t.group, p.w_policy);
             } else if (SWIGLU) {
-              ptx::tma_load_2d(sw, &tm_w, full_bar(s), kcol, wrow, p.w_policy);
-              ptx::tma_load_2d(sw + 64 * GEMM_BK * 2, &tm_w, full_bar(s), kcol, wrow + p.up_offset, p.w_policy);
+              load_2d(sw, &tm_w, s, kcol, wrow, p.w_policy);
+              load_2d(sw + 64 * GEMM_BK * 2, &tm_w, s, kcol, wrow + p.up_offset, p.w_policy);
             } else {
-              ptx::tma_load_2d(sw, &tm_w, full_bar(s), kcol, wrow, p.w_policy);
+              load_2d(sw, &tm_w, s, kcol, wrow, p.w_policy);
             }
             if (p.split_boxes) {
               int at = 0;
 #pragma unroll
               for (int i = 0; i < 5; ++i)
-                if (cols & (256 >> i)) {
-                  ptx::tma_load_2d(sx + (uint32_t)at * (GEMM_BK * 2), &tm_xs.box[i], full_bar(s), kcol, t.row0 + at,
+                if (own & (256 >> i)) {
+                  load_2d(sx + (uint32_t)at * (GEMM_BK * 2), &tm_xs.box[i], s, kcol, row0 + at,
                                    ptx::kEvictLast);
                   at += 256 >> i;
                 }
             } else {
-              for (int at = 0; at < cols; at += p.xbox) {
+              for (int at = 0; at < own; at += p.xbox) {
                 if (p.batch_extra)
-                  ptx::tma_load_3d(sx + (uint32_t)at * (GEMM_BK * 2), &tm_x, full_bar(s), kcol, t.row0 + at, t.group,
+                  load_3d(sx + (uint32_t)at * (GEMM_BK * 2), &tm_x, s, kcol, row0 + at, t.group,
                                    ptx::kEvictLast);
                 else
-                  ptx::tma_load_2d(sx + (uint32_t)at * (GEMM_BK * 2), &tm_x, full_bar(s), kcol, t.row0 + at,
+                  load_2d(sx + (uint32_t)at * (GEMM_BK * 2), &tm_x, s, kcol, row0 + at,
                                    ptx::kEvictLast);
               }
             }
@@ -399,16 +439,21 @@ gemm_ws_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------ MMA issuer
-    if (ptx::elect_one()) {
+    if (rank == 0 && ptx::elect_one()) {
+      auto commit = [&](uint32_t b) {
+        if (PAIR) ptx::umma_commit_pair(b);
+        else ptx::umma_commit(b);
+      };
       uint32_t it = 0, tile_it = 0, ph = 0;
       int s = 0;
       bool ok = true;
-      for (long long lin = blockIdx.x; ok; lin += gridDim.x, ++tile_it) {
+      for (long long lin = lin0; ok; lin += lin_step, ++tile_it) {
         GemmTile t;
-        if (!gemm_tile(p, t_tiles, lin, t)) break;
+        if (!tile_at(t_tiles, lin, t)) break;
         const int buf = tile_it & 1;
-        const uint32_t cols = (uint32_t)gemm_tile_cols(p, t.n);
-        const uint32_t idesc = (p.fp16 ? ptx::umma_idesc_f16_m128(cols) : ptx::umma_idesc_bf16_m128(cols)) |
+        const uint32_t cols = (uint32_t)gemm_tile_cols<PAIR>(p, t.n);
+        // (the M field counts 16 rows: 8 + 8 for a pair)
+        const uint32_t idesc = (PAIR ? 128u / 16 << 24 : 0u) + (p.fp16 ? ptx::umma_idesc_f16_m128(cols) : ptx::umma_idesc_bf16_m128(cols)) |
                                (W_MN ? 1u << 15 : 0u);   // bit 15: A is MN-major
         // start-address step (16-byte units) of a 16-element K step of the weights, and their leading byte offset
         constexpr uint32_t w_step = W_MN ? 16 * 128 / 16 : 2, w_lead = W_MN ? GEMM_WBYTES / 2 / 16 : 1;
@@ -428,13 +473,19 @@ gemm_ws_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__
             // descriptors differ only in the start-address field: +2 (32 bytes) per 16-element K step of a K-major tile
             const uint64_t da = desc_hi | (uint64_t)(((sw & 0x3FFFFu) >> 4) | (w_lead << 16));
             const uint64_t db = desc_hi | (uint64_t)((((sw + GEMM_WBYTES) & 0x3FFFFu) >> 4) | (1u << 16));
-            ptx::umma_bf16(d_tmem, da, db, idesc, (kb | a) != 0 ? 1u : 0u);
+            if (PAIR) {
 #pragma unroll
-            for (int kk = 1; kk < GEMM_BK / 16; ++kk) ptx::umma_bf16_acc(d_tmem, da + w_step * kk, db + 2 * kk, idesc);
+              for (int kk = 0; kk < GEMM_BK / 16; ++kk)
+                ptx::umma_bf16_pair(d_tmem, da + w_step * kk, db + 2 * kk, idesc, (kb | a | kk) != 0 ? 1u : 0u);
+            } else {
+              ptx::umma_bf16(d_tmem, da, db, idesc, (kb | a) != 0 ? 1u : 0u);
+#pragma unroll
+              for (int kk = 1; kk < GEMM_BK / 16; ++kk) ptx::umma_bf16_acc(d_tmem, da + w_step * kk, db + 2 * kk, idesc);
+            }
           }
-          ptx::umma_commit(empty_bar(s));  // stage is free once these MMAs have read it
+          commit(empty_bar(s));  // stage is free once these MMAs have read it
         }
-        if (ok) ptx::umma_commit(tfull_bar(buf));
+        if (ok) commit(tfull_bar(buf));
         GEMM_STAMP(3);                   // last MMA of the tile issued
       }
     }
@@ -442,9 +493,9 @@ gemm_ws_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__
     // ------------------------------------------------------------ epilogue (warps 2..5)
     const int q = warp & 3;              // tensor-memory lane quadrant this warp may read
     uint32_t tile_it = 0;
-    for (long long lin = blockIdx.x;; lin += gridDim.x, ++tile_it) {
+    for (long long lin = lin0;; lin += lin_step, ++tile_it) {
       GemmTile t;
-      if (!gemm_tile(p, t_tiles, lin, t)) break;
+      if (!tile_at(t_tiles, lin, t)) break;
       const int buf = tile_it & 1;
       const bool ready = ptx::mbar_wait(tfull_bar(buf), (tile_it >> 1) & 1, abort_flag, 400 + buf);
       if (SWIGLU || HEAD) {
@@ -690,7 +741,12 @@ gemm_ws_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__
         ptx::named_barrier_sync(1, 128);  // exchange buffer is reused by the next tile
       }
       ptx::tc_fence_before();
-      ptx::mbar_arrive(tempty_bar(buf));
+      if (PAIR) {
+        __syncwarp();
+        if (lane == 0) ptx::mbar_arrive_cluster(ptx::cluster_addr(tempty_bar(buf), 0));
+      } else {
+        ptx::mbar_arrive(tempty_bar(buf));
+      }
       if (threadIdx.x == 64) GEMM_STAMP(5);   // tile stored
     }
   }
@@ -702,10 +758,12 @@ gemm_ws_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__
     while (global_timer_ns() - t0 < 200000ull) {
     }
   }
+  if (PAIR) ptx::cluster_sync();   // neither CTA leaves while the other's instructions or arrivals may still reach it
   ptx::tc_fence_after();
   if (warp == 1) {
     __syncwarp();
-    ptx::tmem_dealloc(tmem_base, (uint32_t)p.tmem_cols);
+    if (PAIR) ptx::tmem_dealloc_pair(tmem_base, (uint32_t)p.tmem_cols);
+    else ptx::tmem_dealloc(tmem_base, (uint32_t)p.tmem_cols);
   }
 }
 
@@ -756,13 +814,14 @@ inline int env_int(const char* name, int dflt) {
   return v ? atoi(v) : dflt;
 }
 
-template <int MODE>
+// max_tiles: tiles of one CTA, or of a pair.
+template <int MODE, bool PAIR = false>
 inline int gemm_launch(const CUtensorMap& tw, const GemmXMaps& tx, GemmParams& p, long long max_tiles,
                        cudaStream_t st) {
   constexpr bool SWIGLU = MODE == GEMM_SWIGLU;
   static PerDeviceFlags attr_set;
-  if (int rc = set_max_dyn_smem_once(attr_set, gemm_ws_kernel<MODE>, GEMM_SMEM_BUDGET)) return rc;
-  const int atom_bytes = GEMM_WBYTES + p.xrows_max * GEMM_BK * 2;
+  if (int rc = set_max_dyn_smem_once(attr_set, gemm_ws_kernel<MODE, PAIR>, GEMM_SMEM_BUDGET)) return rc;
+  const int atom_bytes = GEMM_WBYTES + p.xrows_max / (PAIR ? 2 : 1) * GEMM_BK * 2;
   // epilogue scratch after the stages: the SwiGLU exchange buffer, or the head mode's per-warp partials
   const int exch_bytes_pre = SWIGLU ? 64 * (p.xrows_max + GEMM_EXCH_PAD) * 2
                                     : (MODE == GEMM_HEAD ? 3 * 4 * p.xrows_max * 4 : 4 * 16 * 32 * 2);
@@ -790,11 +849,12 @@ inline int gemm_launch(const CUtensorMap& tw, const GemmXMaps& tx, GemmParams& p
   if (cols > 512) return B200_ERR_SHAPE;
   p.tmem_cols = cols;
   const size_t smem = 256 + 1024 + (size_t)stages * stage_bytes + exch_bytes;
-  long long grid = max_tiles < sm_count() ? max_tiles : sm_count();
+  const int width = PAIR ? 2 : 1;
+  long long grid = max_tiles < sm_count() / width ? max_tiles : sm_count() / width;
   if (grid <= 0) return B200_OK;
   // A dense GEMM (static tiling) may start under its predecessor's tail: it prefetches weights before it waits.
-  launch_k_pdl(gemm_ws_kernel<MODE>, dim3((unsigned)grid), dim3(GEMM_THREADS), smem, st,
-               pdl_mode() == 1 || (pdl_mode() == 2 && !p.tile_table), 1, tw, tx, p);
+  launch_k_pdl(gemm_ws_kernel<MODE, PAIR>, dim3((unsigned)grid * width), dim3(GEMM_THREADS), smem, st,
+               pdl_mode() == 1 || (pdl_mode() == 2 && !p.tile_table), width, tw, tx, p);
   return launch_status();
 }
 
@@ -1035,22 +1095,39 @@ struct GemmExtra {
 // (16 KiB of weights + 128 B per token) into shared memory and the persistent CTAs work through the tiles in rounds, so the
 // cost of a tiling is rounds x bytes per stage; take the cheapest.  (Tiles of fewer weight rows, to put one token's product on
 // more SMs, gain nothing: 6144 -> 2048 took 24 us with 128 rows a tile and 23 with 32.)
-inline void gemm_dense_tiles(GemmParams& p, long long T, int N, int batch, int features = GEMM_WTILE) {
+// Pairs, where the caller may use them: the same with two CTAs to a tile, each with half of its token rows.
+inline bool gemm_dense_tiles(GemmParams& p, long long T, int N, int batch, int features = GEMM_WTILE) {
   const int sms = sm_count();
   const int min_tiles = (int)((T + 255) / 256), max_tiles = (int)((T + 15) / 16);
   long long best_cost = -1;
-  p.w_tiles = (N + features - 1) / features;
+  const int w_tiles = (N + features - 1) / features;
   for (int tt = min_tiles; tt <= max_tiles; ++tt) {
     const int rows = round_up((int)((T + tt - 1) / tt), 16);
     const int tiles_t = (int)((T + rows - 1) / rows);
-    const long long rounds = ((long long)tiles_t * p.w_tiles * batch + sms - 1) / sms;
-    const long long cost = rounds * (GEMM_WBYTES + rows * GEMM_BK * 2);
+    const long long rounds = ((long long)tiles_t * w_tiles * batch + sms - 1) / sms;
+    const long long cost = rounds * (GEMM_WTILE + rows);
     if (best_cost < 0 || cost < best_cost) {
       best_cost = cost;
+      p.w_tiles = w_tiles;
       p.rows_per_tile = rows;
       p.dense_t_tiles = tiles_t;
     }
   }
+  bool pair = false;
+  for (int tt = min_tiles; T >= GEMM_PAIR_TOKENS && tt <= max_tiles; ++tt) {
+    const int rows = round_up((int)((T + tt - 1) / tt), 32);
+    const int tiles_t = (int)((T + rows - 1) / rows), w2 = (w_tiles + 1) / 2;
+    const long long rounds = ((long long)tiles_t * w2 * batch + sms / 2 - 1) / (sms / 2);
+    const long long cost = rounds * (GEMM_WTILE + rows / 2);
+    if (cost < best_cost) {
+      best_cost = cost;
+      pair = true;
+      p.w_tiles = w2;
+      p.rows_per_tile = rows;
+      p.dense_t_tiles = tiles_t;
+    }
+  }
+  return pair;
 }
 
 inline int gemm_dense_16bit(const void* x, const void* w, const void* bias, void* out, long long T, int N, int K,
@@ -1066,11 +1143,11 @@ inline int gemm_dense_16bit(const void* x, const void* w, const void* bias, void
   p.w_rows_per_group = N;
   p.up_offset = 0;
   p.t_rows = (int)T;
-  gemm_dense_tiles(p, T, N, ex.batch);
+  const bool pair = gemm_dense_tiles(p, T, N, ex.batch);
   p.tile_table = nullptr;
   p.tile_count = nullptr;
   p.tokens_first = 1;
-  p.xbox = p.rows_per_tile;
+  p.xbox = pair ? p.rows_per_tile / 2 : p.rows_per_tile;
   p.xrows_max = p.rows_per_tile;
   p.out = out;
   p.ldo = out_row_stride;
@@ -1105,7 +1182,9 @@ inline int gemm_dense_16bit(const void* x, const void* w, const void* bias, void
     rc = make_tmap_2d(&tx.box[0], x, (uint64_t)T, (uint64_t)K, (uint64_t)x_row_stride, (uint32_t)p.xbox, fp16);
   }
   if (rc) return rc;
-  return gemm_launch<GEMM_PLAIN>(tw, tx, p, (long long)p.w_tiles * p.dense_t_tiles * ex.batch, (cudaStream_t)stream);
+  const long long tiles = (long long)p.w_tiles * p.dense_t_tiles * ex.batch;
+  return pair ? gemm_launch<GEMM_PLAIN, true>(tw, tx, p, tiles, (cudaStream_t)stream)
+              : gemm_launch<GEMM_PLAIN>(tw, tx, p, tiles, (cudaStream_t)stream);
 }
 }  // namespace b200
 
@@ -1122,9 +1201,9 @@ inline int gemm_dense_gated(const void* x, const void* w, const void* scale_out,
   p.w_rows_per_group = 2 * n_out;
   p.up_offset = n_out;
   p.t_rows = (int)T;
-  gemm_dense_tiles(p, T, n_out, 1, 64);
+  const bool pair = gemm_dense_tiles(p, T, n_out, 1, 64);
   p.tokens_first = 1;
-  p.xbox = p.rows_per_tile;
+  p.xbox = pair ? p.rows_per_tile / 2 : p.rows_per_tile;
   p.xrows_max = p.rows_per_tile;
   p.out = out;
   p.ldo = out_row_stride;
@@ -1136,7 +1215,9 @@ inline int gemm_dense_gated(const void* x, const void* w, const void* scale_out,
   int rc = make_tmap_2d(&tw, w, 2 * (uint64_t)n_out, (uint64_t)K, (uint64_t)w_row_stride, 64);
   if (!rc) rc = make_tmap_2d(&tx.box[0], x, (uint64_t)T, (uint64_t)K, (uint64_t)x_row_stride, (uint32_t)p.xbox);
   if (rc) return rc;
-  return gemm_launch<GEMM_SWIGLU>(tw, tx, p, (long long)p.w_tiles * p.dense_t_tiles, (cudaStream_t)stream);
+  const long long tiles = (long long)p.w_tiles * p.dense_t_tiles;
+  return pair ? gemm_launch<GEMM_SWIGLU, true>(tw, tx, p, tiles, (cudaStream_t)stream)
+              : gemm_launch<GEMM_SWIGLU>(tw, tx, p, tiles, (cudaStream_t)stream);
 }
 }  // namespace b200
 
@@ -1326,6 +1407,7 @@ inline int moe_grouped_gemm_impl(const void* x, long long x_rows, long long x_ro
   // expert's weight tiles run side by side over one token tile, so that both come from HBM once.
   p.tokens_first = 0;
   p.split_boxes = tile_rows_max > 64 && !gather_index;
+  if (p.split_boxes) p.w_tiles = (p.w_tiles + 1) / 2;   // of a CTA pair
   p.xrows_max = tile_rows_max;
   p.out = out;
   p.ldo = out_row_stride;
@@ -1362,6 +1444,10 @@ inline int moe_grouped_gemm_impl(const void* x, long long x_rows, long long x_ro
   }
   if (rc) return rc;
   const long long tiles = (long long)max_tiles * p.w_tiles;
+  if (p.split_boxes)
+    return mode == 1 ? gemm_launch<GEMM_SWIGLU, true>(tw, tx, p, tiles, (cudaStream_t)stream)
+           : w_mn    ? gemm_launch<GEMM_DGRAD, true>(tw, tx, p, tiles, (cudaStream_t)stream)
+                     : gemm_launch<GEMM_PLAIN, true>(tw, tx, p, tiles, (cudaStream_t)stream);
   if (mode == 1) return gemm_launch<GEMM_SWIGLU>(tw, tx, p, tiles, (cudaStream_t)stream);
   if (w_mn) return gemm_launch<GEMM_DGRAD>(tw, tx, p, tiles, (cudaStream_t)stream);
   return gemm_launch<GEMM_PLAIN>(tw, tx, p, tiles, (cudaStream_t)stream);
