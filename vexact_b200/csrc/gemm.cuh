@@ -79,6 +79,7 @@ struct GemmParams {
   // MN-major through 3-D maps, two boxes of 64 k rows x 64 features per atom.  K steps from k_second on come from a second
   // tensor of the same shape (0: there is none).
   int k_second;
+  int deep_w, deep_x;   // operand maps of whole stages (make_tmap_deep): one copy brings all K atoms of a stage
   int split_boxes;   // activation boxes by the binary digits of a tile's height instead of p.xbox rows each
   int xbox;       // rows per activation TMA box (multiple of 16)
   int xrows_max;  // largest token count of any tile (multiple of xbox, <= 256)
@@ -241,7 +242,8 @@ gemm_ws_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__
   const uint32_t stage_base = (smem_base + 256 + 1023) & ~1023u;
   const int atom_bytes = GEMM_WBYTES + p.xrows_max / (PAIR ? 2 : 1) * (GEMM_BK * 2);
   const int KA = p.katoms;
-  const int stage_bytes = atom_bytes * KA;
+  const int stage_bytes = atom_bytes * KA;   // the K atoms of the weights, then those of the tokens
+  const uint32_t x_atom = (uint32_t)(atom_bytes - GEMM_WBYTES), x_base = (uint32_t)KA * GEMM_WBYTES;
   __nv_bfloat16* exch =
       reinterpret_cast<__nv_bfloat16*>(smem_raw + (stage_base - smem_base) + (size_t)S * stage_bytes);
 
@@ -295,6 +297,33 @@ gemm_ws_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__
   auto arm = [&](int s, uint32_t bytes) {
     if (!PAIR || rank == 0) ptx::mbar_expect_tx(full_bar(s), bytes);
   };
+  // A stage's weights by one copy (p.deep_w): K atoms from index z on.
+  auto weights_deep = [&](uint32_t at, int s, int wrow, int z) {
+    if (!SWIGLU) load_3d(at, &tm_w, s, 0, wrow, z, p.w_policy);
+    else if (PAIR) ptx::tma_load_4d_pair(at, &tm_w, ptx::cluster_addr(full_bar(s), 0), 0, wrow, 0, z, p.w_policy);
+    else ptx::tma_load_4d(at, &tm_w, full_bar(s), 0, wrow, 0, z, p.w_policy);
+  };
+  // The weights of K step kb into the stage at `at` (slot s): by one copy, or atom by atom.
+  auto weights = [&](uint32_t at, int s, int kb, const GemmTile& t, int wrow) {
+    if (!W_MN && p.deep_w) {
+      weights_deep(at, s, wrow, kb * KA);
+      return;
+    }
+    for (int a = 0; a < KA; ++a) {
+      const uint32_t sw = at + (uint32_t)a * GEMM_WBYTES;
+      const int kcol = (kb * KA + a) * GEMM_BK;
+      if (W_MN) {
+        const bool second = p.k_second && kcol >= p.k_second;
+#pragma unroll
+        for (int h = 0; h < 2; ++h)
+          load_3d(sw + h * (GEMM_WBYTES / 2), second ? &tm_xs.w2 : &tm_w, s, t.wt * GEMM_WTILE + h * 64,
+                  second ? kcol - p.k_second : kcol, t.group, p.w_policy);
+      } else {
+        load_2d(sw, &tm_w, s, kcol, wrow, p.w_policy);
+        if (SWIGLU) load_2d(sw + 64 * GEMM_BK * 2, &tm_w, s, kcol, wrow + p.up_offset, p.w_policy);
+      }
+    }
+  };
   // Everything above is set-up.  What the previous kernel wrote (activations, the tile table) is read only
   // after pdl_wait().  The weights are not its output: with a static tiling (no tile table) the producer
   // requests its first ring of weight tiles before it waits, so that under programmatic dependent launch
@@ -309,12 +338,7 @@ gemm_ws_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__
         const int wrow = t.group * p.w_rows_per_group + t.wt * (SWIGLU ? 64 : GEMM_WTILE);
         for (int kb = 0; kb < prefetched; ++kb) {
           arm(kb, tx * KA);
-          for (int a = 0; a < KA; ++a) {
-            const uint32_t sw = stage_base + (uint32_t)kb * stage_bytes + (uint32_t)a * atom_bytes;
-            const int kcol = (kb * KA + a) * GEMM_BK;
-            load_2d(sw, &tm_w, kb, kcol, wrow, p.w_policy);
-            if (SWIGLU) load_2d(sw + 64 * GEMM_BK * 2, &tm_w, kb, kcol, wrow + p.up_offset, p.w_policy);
-          }
+          weights(stage_base + (uint32_t)kb * stage_bytes, kb, kb, t, wrow);
         }
       }
     }
@@ -356,8 +380,8 @@ gemm_ws_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__
         if (lane == 0) ptx::mbar_expect_tx(full_bar(s), tx * KA);
         __syncwarp();   // the barrier is armed before any lane's copy can complete on it
         for (int a = 0; a < KA; ++a) {
-          const uint32_t sw = stage_base + (uint32_t)s * stage_bytes + (uint32_t)a * atom_bytes;
-          const uint32_t sx = sw + GEMM_WBYTES;
+          const uint32_t sw = stage_base + (uint32_t)s * stage_bytes + (uint32_t)a * GEMM_WBYTES;
+          const uint32_t sx = stage_base + (uint32_t)s * stage_bytes + x_base + (uint32_t)a * x_atom;
           const int kcol = (kb * KA + a) * GEMM_BK;
           if (lane == 0) {
             if (SWIGLU) {
@@ -387,6 +411,23 @@ gemm_ws_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__
         const uint32_t tx = (PAIR ? 2 : 1) * GEMM_WBYTES + (uint32_t)cols * (GEMM_BK * 2);
         const int own = PAIR ? cols / 2 : cols, row0 = t.row0 + rank * own;   // token rows of this CTA
         const int wrow = t.group * p.w_rows_per_group + t.wt * (SWIGLU ? 64 : GEMM_WTILE);
+        if (!W_MN && p.deep_w && p.deep_x) {
+          // two copies a stage; with few tokens these few instructions are what a K step costs
+          const uint32_t bytes = tx * KA;
+          for (int kb = 0, z = 0; kb < num_kb; ++kb, ++it, z += KA, s = (s + 1 == S ? 0 : s + 1), ph ^= (s == 0)) {
+            const uint32_t stage = stage_base + (uint32_t)s * stage_bytes;
+            if (it >= (uint32_t)prefetched) {
+              if (!ptx::mbar_wait(empty_bar(s), ph ^ 1, abort_flag, 100 + s)) {
+                ok = false;
+                break;
+              }
+              arm(s, bytes);
+              weights_deep(stage, s, wrow, z);
+            }
+            load_3d(stage + x_base, &tm_x, s, 0, row0, z, ptx::kEvictLast);
+          }
+          continue;
+        }
         for (int kb = 0; kb < num_kb; ++kb, ++it, s = (s + 1 == S ? 0 : s + 1), ph ^= (s == 0)) {
           // the first tile's first `prefetched` stages were armed, and their weights requested, before pdl_wait
           const bool early = it < (uint32_t)prefetched;
@@ -397,23 +438,11 @@ gemm_ws_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__
             }
             arm(s, tx * KA);
           }
+          const uint32_t stage = stage_base + (uint32_t)s * stage_bytes;
+          if (!early) weights(stage, s, kb, t, wrow);
           for (int a = 0; a < KA; ++a) {
-            const uint32_t sw = stage_base + (uint32_t)s * stage_bytes + (uint32_t)a * atom_bytes;
-            const uint32_t sx = sw + GEMM_WBYTES;
+            const uint32_t sx = stage + x_base + (uint32_t)a * x_atom;
             const int kcol = (kb * KA + a) * GEMM_BK;
-            if (early) {
-            } else if (W_MN) {
-              const bool second = p.k_second && kcol >= p.k_second;
-#pragma unroll
-              for (int h = 0; h < 2; ++h)
-                load_3d(sw + h * (GEMM_WBYTES / 2), second ? &tm_xs.w2 : &tm_w, s, t.wt * GEMM_WTILE + h * 64,
-                                 second ? kcol - p.k_second : kcol, t.group, p.w_policy);
-            } else if (SWIGLU) {
-              load_2d(sw, &tm_w, s, kcol, wrow, p.w_policy);
-              load_2d(sw + 64 * GEMM_BK * 2, &tm_w, s, kcol, wrow + p.up_offset, p.w_policy);
-            } else {
-              load_2d(sw, &tm_w, s, kcol, wrow, p.w_policy);
-            }
             if (p.split_boxes) {
               int at = 0;
 #pragma unroll
@@ -469,10 +498,11 @@ gemm_ws_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__
           ptx::tc_fence_after();
           if (it == 0) GEMM_STAMP(2);    // first stage landed
           for (int a = 0; a < KA; ++a) {
-            const uint32_t sw = stage_base + (uint32_t)s * stage_bytes + (uint32_t)a * atom_bytes;
+            const uint32_t sw = stage_base + (uint32_t)s * stage_bytes + (uint32_t)a * GEMM_WBYTES;
+            const uint32_t sx = stage_base + (uint32_t)s * stage_bytes + x_base + (uint32_t)a * x_atom;
             // descriptors differ only in the start-address field: +2 (32 bytes) per 16-element K step of a K-major tile
             const uint64_t da = desc_hi | (uint64_t)(((sw & 0x3FFFFu) >> 4) | (w_lead << 16));
-            const uint64_t db = desc_hi | (uint64_t)((((sw + GEMM_WBYTES) & 0x3FFFFu) >> 4) | (1u << 16));
+            const uint64_t db = desc_hi | (uint64_t)(((sx & 0x3FFFFu) >> 4) | (1u << 16));
             if (PAIR) {
 #pragma unroll
               for (int kk = 0; kk < GEMM_BK / 16; ++kk)
@@ -805,6 +835,43 @@ inline int make_tmap_3d(CUtensorMap* m, const void* base, uint64_t batch, uint64
   return r == CUDA_SUCCESS ? B200_OK : B200_ERR_DRIVER;
 }
 
+// 2-D bf16 tensor [rows, cols] seen as [cols / 64, rows, 64]: box = `atoms` K atoms of 64 columns x box_rows rows, 128-byte
+// swizzle, which lands atom after atom.  One copy per operand and stage instead of one per atom: with few tokens a K step costs
+// what issuing its copies costs (0.15 us per atom of 64, whatever the box's bytes and the number of products), not their bytes.
+// cols a multiple of 64.
+inline int make_tmap_deep(CUtensorMap* m, const void* base, uint64_t rows, uint64_t cols, uint64_t row_stride, uint32_t box_rows,
+                          uint32_t atoms, bool fp16 = false) {
+  EncodeTiledFn enc = tensor_map_encoder();
+  if (!enc) return B200_ERR_DRIVER;
+  if ((reinterpret_cast<uintptr_t>(base) & 15) || (row_stride * 2) % 16 || box_rows == 0 || box_rows > 256 || cols % GEMM_BK)
+    return B200_ERR_ARG;
+  cuuint64_t dims[3] = {(cuuint64_t)GEMM_BK, rows, cols / GEMM_BK};
+  cuuint64_t strides[2] = {row_stride * 2, GEMM_BK * 2};
+  cuuint32_t box[3] = {(cuuint32_t)GEMM_BK, box_rows, atoms};
+  cuuint32_t estr[3] = {1, 1, 1};
+  CUresult r = enc(m, fp16 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(base), dims,
+                   strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+                   CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  return r == CUDA_SUCCESS ? B200_OK : B200_ERR_DRIVER;
+}
+
+// The same for the stacked gate and up rows of the gated form, [rows, cols] with the up half `up` rows below the gate half: box =
+// atoms x {gate, up} x 64 rows x 64 columns.  A tile that reaches past its gate rows reads other rows, whose outputs are not stored.
+inline int make_tmap_deep_gated(CUtensorMap* m, const void* base, uint64_t rows, uint64_t up, uint64_t cols, uint64_t row_stride,
+                                uint32_t atoms) {
+  EncodeTiledFn enc = tensor_map_encoder();
+  if (!enc) return B200_ERR_DRIVER;
+  if ((reinterpret_cast<uintptr_t>(base) & 15) || (row_stride * 2) % 16 || cols % GEMM_BK || rows <= up) return B200_ERR_ARG;
+  cuuint64_t dims[4] = {(cuuint64_t)GEMM_BK, rows - up, 2, cols / GEMM_BK};
+  cuuint64_t strides[3] = {row_stride * 2, up * row_stride * 2, GEMM_BK * 2};
+  cuuint32_t box[4] = {(cuuint32_t)GEMM_BK, 64, 2, atoms};
+  cuuint32_t estr[4] = {1, 1, 1, 1};
+  CUresult r = enc(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<void*>(base), dims, strides, box, estr,
+                   CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                   CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  return r == CUDA_SUCCESS ? B200_OK : B200_ERR_DRIVER;
+}
+
 inline int round_up(int v, int m) { return (v + m - 1) / m * m; }
 
 // Development knobs (unset in normal use): B200_GEMM_XBOX = rows per activation box of the grouped
@@ -812,6 +879,20 @@ inline int round_up(int v, int m) { return (v + m - 1) / m * m; }
 inline int env_int(const char* name, int dflt) {
   const char* v = getenv(name);
   return v ? atoi(v) : dflt;
+}
+
+// Epilogue scratch after the stages: the SwiGLU exchange buffer, the head mode's per-warp partials, or the turning tiles.
+inline int gemm_exch_bytes(int mode, int xrows_max) {
+  return mode == GEMM_SWIGLU ? 64 * (xrows_max + GEMM_EXCH_PAD) * 2 : mode == GEMM_HEAD ? 3 * 4 * xrows_max * 4 : 4 * 16 * 32 * 2;
+}
+// K atoms per stage: fewer, larger stages cut the per-stage barrier round trips; keep >= 3 stages.  (One token, 6144 -> 2048, at
+// 1 / 2 / 4 atoms: 31 / 24 / 20 us with a copy per atom.)
+inline int gemm_katoms(int k, int atom_bytes, int exch_bytes) {
+  static const int ka_env = env_int("B200_GEMM_KATOMS", 4);
+  int ka = (ka_env == 1 || ka_env == 2 || ka_env == 4) ? ka_env : 4;
+  while (ka > 1 && ((GEMM_SMEM_BUDGET - 256 - 1024 - exch_bytes) / (atom_bytes * ka) < 3 || (k + GEMM_BK - 1) / GEMM_BK < ka))
+    ka >>= 1;
+  return ka;
 }
 
 // max_tiles: tiles of one CTA, or of a pair.
@@ -822,16 +903,8 @@ inline int gemm_launch(const CUtensorMap& tw, const GemmXMaps& tx, GemmParams& p
   static PerDeviceFlags attr_set;
   if (int rc = set_max_dyn_smem_once(attr_set, gemm_ws_kernel<MODE, PAIR>, GEMM_SMEM_BUDGET)) return rc;
   const int atom_bytes = GEMM_WBYTES + p.xrows_max / (PAIR ? 2 : 1) * GEMM_BK * 2;
-  // epilogue scratch after the stages: the SwiGLU exchange buffer, or the head mode's per-warp partials
-  const int exch_bytes_pre = SWIGLU ? 64 * (p.xrows_max + GEMM_EXCH_PAD) * 2
-                                    : (MODE == GEMM_HEAD ? 3 * 4 * p.xrows_max * 4 : 4 * 16 * 32 * 2);
-  // K atoms per stage: fewer, larger stages cut the per-stage barrier round trips; keep >= 3 stages.
-  static const int ka_env = env_int("B200_GEMM_KATOMS", 2);
-  int ka = (ka_env == 1 || ka_env == 2 || ka_env == 4) ? ka_env : 2;
-  while (ka > 1 && ((GEMM_SMEM_BUDGET - 256 - 1024 - exch_bytes_pre) / (atom_bytes * ka) < 3 ||
-                    (p.k + GEMM_BK - 1) / GEMM_BK < ka))
-    ka >>= 1;
-  p.katoms = ka;
+  const int exch_bytes_pre = gemm_exch_bytes(MODE, p.xrows_max);
+  const int ka = p.katoms = gemm_katoms(p.k, atom_bytes, exch_bytes_pre);
   static const int epi_scalar = env_int("B200_GEMM_EPI_SCALAR", 0);
   p.scalar_epilogue = epi_scalar;
   const int stage_bytes = atom_bytes * ka;
@@ -1177,9 +1250,15 @@ inline int gemm_dense_16bit(const void* x, const void* w, const void* bias, void
     rc = make_tmap_3d(&tx.box[0], x, (uint64_t)ex.batch, (uint64_t)T, (uint64_t)K, (uint64_t)ex.x_batch_stride,
                       (uint64_t)x_row_stride, (uint32_t)p.xbox);
   } else {
-    rc = make_tmap_2d(&tw, w, (uint64_t)N, (uint64_t)K, (uint64_t)w_row_stride, GEMM_WTILE, fp16);
-    if (rc) return rc;
-    rc = make_tmap_2d(&tx.box[0], x, (uint64_t)T, (uint64_t)K, (uint64_t)x_row_stride, (uint32_t)p.xbox, fp16);
+    if (K % GEMM_BK == 0) {
+      const int ka = gemm_katoms(K, GEMM_WBYTES + p.xbox * GEMM_BK * 2, gemm_exch_bytes(GEMM_PLAIN, p.xrows_max));
+      p.deep_w = p.deep_x = 1;
+      rc = make_tmap_deep(&tw, w, (uint64_t)N, (uint64_t)K, (uint64_t)w_row_stride, GEMM_WTILE, ka, fp16);
+      if (!rc) rc = make_tmap_deep(&tx.box[0], x, (uint64_t)T, (uint64_t)K, (uint64_t)x_row_stride, (uint32_t)p.xbox, ka, fp16);
+    } else {
+      rc = make_tmap_2d(&tw, w, (uint64_t)N, (uint64_t)K, (uint64_t)w_row_stride, GEMM_WTILE, fp16);
+      if (!rc) rc = make_tmap_2d(&tx.box[0], x, (uint64_t)T, (uint64_t)K, (uint64_t)x_row_stride, (uint32_t)p.xbox, fp16);
+    }
   }
   if (rc) return rc;
   const long long tiles = (long long)p.w_tiles * p.dense_t_tiles * ex.batch;
@@ -1212,8 +1291,16 @@ inline int gemm_dense_gated(const void* x, const void* w, const void* scale_out,
   p.w_policy = p.dense_t_tiles == 1 ? ptx::kEvictFirst : ptx::kEvictNormal;
   CUtensorMap tw;
   GemmXMaps tx{};
-  int rc = make_tmap_2d(&tw, w, 2 * (uint64_t)n_out, (uint64_t)K, (uint64_t)w_row_stride, 64);
-  if (!rc) rc = make_tmap_2d(&tx.box[0], x, (uint64_t)T, (uint64_t)K, (uint64_t)x_row_stride, (uint32_t)p.xbox);
+  int rc;
+  if (K % GEMM_BK == 0) {
+    const int ka = gemm_katoms(K, GEMM_WBYTES + p.xbox * GEMM_BK * 2, gemm_exch_bytes(GEMM_SWIGLU, p.xrows_max));
+    p.deep_w = p.deep_x = 1;
+    rc = make_tmap_deep_gated(&tw, w, 2 * (uint64_t)n_out, (uint64_t)n_out, (uint64_t)K, (uint64_t)w_row_stride, ka);
+    if (!rc) rc = make_tmap_deep(&tx.box[0], x, (uint64_t)T, (uint64_t)K, (uint64_t)x_row_stride, (uint32_t)p.xbox, ka);
+  } else {
+    rc = make_tmap_2d(&tw, w, 2 * (uint64_t)n_out, (uint64_t)K, (uint64_t)w_row_stride, 64);
+    if (!rc) rc = make_tmap_2d(&tx.box[0], x, (uint64_t)T, (uint64_t)K, (uint64_t)x_row_stride, (uint32_t)p.xbox);
+  }
   if (rc) return rc;
   const long long tiles = (long long)p.w_tiles * p.dense_t_tiles;
   return pair ? gemm_launch<GEMM_SWIGLU, true>(tw, tx, p, tiles, (cudaStream_t)stream)
@@ -1422,6 +1509,8 @@ inline int moe_grouped_gemm_impl(const void* x, long long x_rows, long long x_ro
   CUtensorMap tw;
   GemmXMaps tx{};
   int rc;
+  const int ka = gemm_katoms(K, GEMM_WBYTES + p.xrows_max / (p.split_boxes ? 2 : 1) * GEMM_BK * 2,
+                             gemm_exch_bytes(mode == 1 ? GEMM_SWIGLU : GEMM_PLAIN, p.xrows_max));
   if (w_mn) {
     // [groups, k, features]: rows past a group's k and columns past its features read as zero
     if (mode != 0 || gather_index || n_out % 8 != 0 || (w2 && K % (2 * GEMM_BK) != 0)) return B200_ERR_SHAPE;
@@ -1430,6 +1519,11 @@ inline int moe_grouped_gemm_impl(const void* x, long long x_rows, long long x_ro
     rc = make_tmap_3d(&tw, w, (uint64_t)num_groups, (uint64_t)k_one, (uint64_t)n_out, (uint64_t)k_one * n_out, (uint64_t)n_out, GEMM_BK);
     if (!rc && w2)
       rc = make_tmap_3d(&tx.w2, w2, (uint64_t)num_groups, (uint64_t)k_one, (uint64_t)n_out, (uint64_t)k_one * n_out, (uint64_t)n_out, GEMM_BK);
+  } else if (K % GEMM_BK == 0 && !gather_index) {
+    p.deep_w = 1;
+    const uint64_t w_rows = (uint64_t)num_groups * p.w_rows_per_group;
+    rc = mode == 1 ? make_tmap_deep_gated(&tw, w, w_rows, (uint64_t)n_out, (uint64_t)K, (uint64_t)K, ka)
+                   : make_tmap_deep(&tw, w, w_rows, (uint64_t)K, (uint64_t)K, GEMM_WTILE, ka);
   } else {
     rc = make_tmap_2d(&tw, w, (uint64_t)num_groups * p.w_rows_per_group, (uint64_t)K, (uint64_t)K, mode == 1 ? 64 : GEMM_WTILE);
   }
@@ -1439,6 +1533,9 @@ inline int moe_grouped_gemm_impl(const void* x, long long x_rows, long long x_ro
   } else if (p.split_boxes) {
     for (int i = 0; i < 5 && !rc; ++i)
       rc = make_tmap_2d(&tx.box[i], x, (uint64_t)x_rows, (uint64_t)K, (uint64_t)K, 256u >> i);
+  } else if (p.deep_w && p.xbox == p.xrows_max) {
+    p.deep_x = 1;
+    rc = make_tmap_deep(&tx.box[0], x, (uint64_t)x_rows, (uint64_t)K, (uint64_t)K, (uint32_t)p.xbox, ka);
   } else {
     rc = make_tmap_2d(&tx.box[0], x, (uint64_t)x_rows, (uint64_t)K, (uint64_t)K, (uint32_t)p.xbox);
   }
