@@ -260,6 +260,16 @@ int b200_paged_attn_fwd_ordered(const void* q, const void* k_cache, const void* 
                                 long long kc_head_stride, long long vc_block_stride, long long vc_page_stride,
                                 long long vc_head_stride, float softmax_scale, const void* seq_order,
                                 long long total_q, void* stream);
+/* The same, and lse_f32 [num_q_heads, total_q] receives log2 of every query's sum of 2^(score * softmax_scale * log2 e). */
+int b200_paged_attn_fwd_lse(const void* q, const void* k_cache, const void* v_cache, void* out,
+                                const void* cu_seqlens_q, const void* seqused_k, const void* page_table,
+                                int num_seqs, int max_seqlen_q, int num_q_heads, int num_kv_heads, int dk, int dv,
+                                int num_blocks, int page_size, int max_pages, long long page_table_stride,
+                                long long q_tok_stride, long long q_head_stride, long long o_tok_stride,
+                                long long o_head_stride, long long kc_block_stride, long long kc_page_stride,
+                                long long kc_head_stride, long long vc_block_stride, long long vc_page_stride,
+                                long long vc_head_stride, float softmax_scale, const void* seq_order,
+                                long long total_q, void* lse_f32, void* stream);
 
 /* ---- vexact/batch_invariant_ops/triton_invariant_attention.py:194-431 (_varlen_attn_bwd_dq_kernel,
  *      _varlen_attn_bwd_dkv_kernel): dq, dk, dv of the packed (non-paged) causal varlen attention.  All tensors
@@ -271,6 +281,12 @@ int b200_paged_attn_fwd_ordered(const void* q, const void* k_cache, const void* 
  *      on mma.sync tensor-core instructions (B200_ATTN_BWD_SIMT=1: the CUDA-core form).  Pass zero-filled dq /
  *      dk / dv: rows of no sequence are not written. */
 int b200_varlen_attn_backward(const void* q, const void* k, const void* v, const void* out, const void* dout,
+                              const void* cu_seqlens_q, const void* cu_seqlens_k, void* dq, void* dk, void* dv,
+                              void* lse_scratch_f32, void* delta_scratch_f32, int num_seqs, int max_seqlen_q,
+                              int max_seqlen_k, long long total_q, long long total_k, int num_q_heads,
+                              int num_kv_heads, int dk_dim, int dv_dim, float softmax_scale, void* stream);
+/* The same with the forward's lse_f32 in place of the scratch; (dk_dim, dv_dim) (128, 128) or (192, 128). */
+int b200_varlen_attn_backward_lse(const void* q, const void* k, const void* v, const void* out, const void* dout,
                               const void* cu_seqlens_q, const void* cu_seqlens_k, void* dq, void* dk, void* dv,
                               void* lse_scratch_f32, void* delta_scratch_f32, int num_seqs, int max_seqlen_q,
                               int max_seqlen_k, long long total_q, long long total_k, int num_q_heads,

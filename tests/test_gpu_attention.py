@@ -602,3 +602,30 @@ def test_sequences_by_descending_context(vb, n):
 
     lens = torch.randint(0, 40, (n,), generator=torch.Generator().manual_seed(n)).int().cuda()     # many ties
     assert torch.equal(descending_contexts(lens).long(), torch.sort(lens, descending=True, stable=True).indices)
+
+
+@pytest.mark.parametrize("hq,hkv,dk", [(8, 2, 128), (16, 1, 128), (6, 2, 128), (4, 4, 192)])
+def test_log_sum_exp_of_the_forward(vb, hq, hkv, dk):
+    """The rows-on-lanes kernel's log-sum-exp (log2 of the sum over unrounded weights) against fp64, over whole and partial tiles,
+    a lone query and several blocks; the outputs keep the plain form's bits and the backward does not depend on who made it."""
+    from vexact_b200.attention import packed_to_paged, paged_attention
+
+    g = torch.Generator().manual_seed(hq + dk)
+    q_lens, kv_lens = [1, 130, 300], [5, 130, 421]
+    q = torch.randn(sum(q_lens), hq, dk, generator=g).to(BF).cuda()
+    k = torch.randn(sum(kv_lens), hkv, dk, generator=g).to(BF).cuda()
+    v = torch.randn(sum(kv_lens), hkv, 128, generator=g).to(BF).cuda()
+    cu_q, cu_k = (torch.tensor([0] + torch.tensor(x).cumsum(0).tolist(), dtype=torch.int32).cuda() for x in (q_lens, kv_lens))
+    scale = dk ** -0.5
+    kc, vc, table, lens = packed_to_paged(k, v, cu_k, max(kv_lens))
+    lse = torch.full((hq, q.shape[0]), float("inf"), device="cuda")
+    out = paged_attention(q, kc, vc, cu_q, lens, table, scale, max(q_lens), lse=lse)
+    assert torch.equal(out, paged_attention(q, kc, vc, cu_q, lens, table, scale, max(q_lens)))
+    a = b = 0
+    for nq, nk in zip(q_lens, kv_lens):
+        s = torch.einsum("qhd,khd->hqk", q[a:a + nq].double(), k[b:b + nk].double().repeat_interleave(hq // hkv, 1)) * scale
+        seen = torch.arange(nk, device="cuda")[None] <= torch.arange(nq, device="cuda")[:, None] + nk - nq
+        ref = torch.logsumexp(s.masked_fill(~seen, float("-inf")), -1) * 1.4426950408889634
+        # fp32 scores of magnitude up to 8 and sums of up to 421 of them, ex2 to 2^-22
+        torch.testing.assert_close(lse[:, a:a + nq].double(), ref, rtol=0, atol=2e-5)
+        a, b = a + nq, b + nk

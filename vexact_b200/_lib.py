@@ -85,6 +85,8 @@ SIGNATURES = {
                             LL, LL, F, P],
     "b200_paged_attn_fwd_ordered": [P, P, P, P, P, P, P, I, I, I, I, I, I, I, I, I, LL, LL, LL, LL, LL, LL, LL, LL, LL,
                             LL, LL, F, P, LL, P],
+    "b200_paged_attn_fwd_lse": [P, P, P, P, P, P, P, I, I, I, I, I, I, I, I, I, LL, LL, LL, LL, LL, LL, LL, LL, LL,
+                            LL, LL, F, P, LL, P, P],
     "b200_moe_route_softmax_topk": [P, I, LL, P, P, P, P, LL, I, I, I, P],
     "b200_moe_route_sigmoid_group_topk": [P, LL, P, P, P, P, LL, I, I, I, I, I, F, P],
     "b200_moe_permute": [P, I, P, P, LL, P, P, P, P, P, P, LL, I, I, I, I, I, P],
@@ -106,6 +108,7 @@ SIGNATURES = {
     "b200_moe_grouped_wgrad_strided": [P, LL, P, LL, P, P, LL, I, I, I, P],
     "b200_transpose_last2": [P, P, I, I, I, P],
     "b200_varlen_attn_backward": [P, P, P, P, P, P, P, P, P, P, P, P, I, I, I, LL, LL, I, I, I, I, F, P],
+    "b200_varlen_attn_backward_lse": [P, P, P, P, P, P, P, P, P, P, P, P, I, I, I, LL, LL, I, I, I, I, F, P],
     "b200_moe_unpermute_add_rmsnorm": [P, P, P, P, P, P, P, LL, I, I, F, I, P],
 }
 

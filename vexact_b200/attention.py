@@ -13,6 +13,7 @@
 """
 from __future__ import annotations
 
+import os
 from typing import Optional
 
 import torch
@@ -36,10 +37,11 @@ def _require_cuda_int32(name: str, t: torch.Tensor) -> None:
 def paged_attention(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor, cu_seqlens_q: torch.Tensor,
                     seqused_k: torch.Tensor, page_table: torch.Tensor, softmax_scale: float,
                     max_seqlen_q: int, seq_order: Optional[torch.Tensor] = None,
-                    out: Optional[torch.Tensor] = None) -> torch.Tensor:
+                    out: Optional[torch.Tensor] = None, lse: Optional[torch.Tensor] = None) -> torch.Tensor:
     """q (total_q, heads, dk) against caches (blocks, page, kv_heads, d); returns (total_q, heads, dv)
     (written into `out` when given; rows of q that belong to no sequence are left as they are).
 
+    lse (fp32 [heads, total_q], optional): receives log2 of every query's sum of 2^(score log2 e).
     seq_order (int32 [num_seqs], optional): a permutation of the sequences, longest context first,
     that balances the persistent kernel's CTAs on ragged batches; it never changes a result."""
     for name, t in (("q", q), ("k", k_cache), ("v", v_cache)):
@@ -76,16 +78,17 @@ def paged_attention(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tenso
         _require_cuda_int32("seq_order", seq_order)
         if seq_order.numel() != num_seqs or not seq_order.is_contiguous():
             raise ValueError("seq_order must be a contiguous permutation of the sequences")
+    lib, tail = _lib.load(), ([] if lse is None else [lse.data_ptr()])
     _lib.check(
-        _lib.load().b200_paged_attn_fwd_ordered(
+        (lib.b200_paged_attn_fwd_ordered if lse is None else lib.b200_paged_attn_fwd_lse)(
             q.data_ptr(), k_cache.data_ptr(), v_cache.data_ptr(), out.data_ptr(), cu_seqlens_q.data_ptr(),
             seqused_k.data_ptr(), page_table.data_ptr(), num_seqs, int(max_seqlen_q), q.shape[1],
             k_cache.shape[2], q.shape[-1], v_cache.shape[-1], k_cache.shape[0], k_cache.shape[1],
             page_table.shape[1], page_table.stride(0), q.stride(0), q.stride(1), out.stride(0), out.stride(1),
             k_cache.stride(0), k_cache.stride(1), k_cache.stride(2), v_cache.stride(0), v_cache.stride(1),
             v_cache.stride(2), float(softmax_scale), seq_order.data_ptr() if seq_order is not None else None,
-            q.shape[0], _lib.current_stream()),
-        "b200_paged_attn_fwd_ordered",
+            q.shape[0], *tail, _lib.current_stream()),
+        "b200_paged_attn_fwd_ordered" if lse is None else "b200_paged_attn_fwd_lse",
     )
     return out
 
@@ -228,27 +231,38 @@ class _PackedVarlenForward(torch.autograd.Function):
         # zero-filled: a sequence the kernel refuses (more queries than keys: reported through the status word)
         # leaves zeros, not whatever the allocator handed out
         out = torch.zeros((qp.shape[0], qp.shape[1], vp.shape[-1]), dtype=qp.dtype, device=qp.device)
-        paged_attention(qp, k_cache, v_cache, cu_q, lens, table, scale, max_seqlen_q, out=out)
-        if any(ctx.needs_input_grad[:3]):
+        needed = any(ctx.needs_input_grad[:3])
+        lse = None
+        # the rows-on-lanes kernel leaves it, where it is the one that runs
+        if needed and (qp.shape[-1], vp.shape[-1]) != (64, 64) and qp.stride(-1) == 1 and qp.shape[0] > 0 \
+                and os.environ.get("B200_ATTN", "")[:1] != "s" \
+                and qp.data_ptr() % 16 == 0 and qp.stride(0) % 8 == 0 and qp.stride(1) % 8 == 0:
+            # (inf: queries of a refused sequence weigh nothing)
+            lse = torch.full((qp.shape[1], qp.shape[0]), float("inf"), dtype=torch.float32, device=qp.device)
+        paged_attention(qp, k_cache, v_cache, cu_q, lens, table, scale, max_seqlen_q, out=out, lse=lse)
+        if needed:
             cu_k = cu_seqlens_k if cu_seqlens_k.dtype == torch.int32 else cu_seqlens_k.to(torch.int32)
             ctx.save_for_backward(qp.contiguous(), kp.contiguous(), vp.contiguous(), out, cu_q.contiguous(),
-                                  cu_k.contiguous())
+                                  cu_k.contiguous(), lse)
             ctx.scale, ctx.max_q, ctx.max_k, ctx.dims = float(scale), int(max_seqlen_q), int(max_seqlen_k), (dk, dv)
         return out if out.shape[-1] == dv else out[..., :dv].contiguous()
 
     @staticmethod
     def backward(ctx, grad_out):
-        q, k, v, out, cu_q, cu_k = ctx.saved_tensors
+        q, k, v, out, cu_q, cu_k, lse = ctx.saved_tensors
         dk_dim, dv_dim = ctx.dims
         dout = grad_out.to(torch.bfloat16)
         if dout.shape[-1] != out.shape[-1]:
             dout = torch.nn.functional.pad(dout, (0, out.shape[-1] - dout.shape[-1]))
         dout = dout.contiguous()
         dq, dkk, dvv = torch.zeros_like(q), torch.zeros_like(k), torch.zeros_like(v)
-        lse = torch.empty(q.shape[:2], dtype=torch.float32, device=q.device)
+        lib = _lib.load()
+        backward = lib.b200_varlen_attn_backward_lse if lse is not None else lib.b200_varlen_attn_backward
+        if lse is None:
+            lse = torch.empty((q.shape[1], q.shape[0]), dtype=torch.float32, device=q.device)
         delta = torch.empty_like(lse)
         _lib.check(
-            _lib.load().b200_varlen_attn_backward(
+            backward(
                 q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(), dout.data_ptr(), cu_q.data_ptr(),
                 cu_k.data_ptr(), dq.data_ptr(), dkk.data_ptr(), dvv.data_ptr(), lse.data_ptr(), delta.data_ptr(),
                 cu_q.numel() - 1, ctx.max_q, ctx.max_k, q.shape[0], k.shape[0], q.shape[1], k.shape[1], q.shape[2],

@@ -71,6 +71,8 @@ struct AttnParams {
   AttnExtras extras;     // the same with extras: capped scores, sink, output gate, sigmoid weights
   int g_tma;             // the same with extras: a warp's gate columns arrive by one TMA box
   int dv;                // rows-on-lanes kernel, exact form: value columns of a head (at most 128)
+  float* lse;            // rows-on-lanes kernel, form ATTN_LSE: [num_q_heads, lse_stride], log2 of the rows' sums of 2^score
+  long long lse_stride;
   int scalar_out;        // development knob B200_ATTN_OUT_SCALAR=1: 2-byte output stores in the keys-on-lanes kernel
 };
 
@@ -402,7 +404,7 @@ inline bool attn_use_tensor_memory() {
 int attn_tc_dispatch(const CUtensorMap& tk, const CUtensorMap& tv, const AttnParams& p, dim3 grid, int dk, int nc,
                      cudaStream_t st);
 int attn_rows_dispatch(const CUtensorMap& tk, const CUtensorMap& tv, const CUtensorMap& tq, const CUtensorMap& to,
-                       const AttnParams& p, int dk, cudaStream_t st);
+                       const AttnParams& p, int dk, cudaStream_t st);   // with p.lse: form ATTN_LSE
 
 // Queries as a 3-D tensor [tokens][heads][dim] with a box of {64 dims, box_heads, box_tokens}: the box's rows
 // land in shared memory in (token, head) order, 128 bytes each, 128-byte swizzle, which is the row order of a
@@ -466,6 +468,16 @@ extern "C" int b200_paged_attn_fwd(const void* q, const void* k_cache, const voi
                                      vc_block_stride, vc_page_stride, vc_head_stride, softmax_scale, nullptr, 0, stream);
 }
 
+namespace b200 {
+int paged_attn_fwd_impl(const void* q, const void* k_cache, const void* v_cache, void* out, const void* cu_seqlens_q,
+                        const void* seqused_k, const void* page_table, int num_seqs, int max_seqlen_q, int num_q_heads,
+                        int num_kv_heads, int dk, int dv, int num_blocks, int page_size, int max_pages, long long page_table_stride,
+                        long long q_tok_stride, long long q_head_stride, long long o_tok_stride, long long o_head_stride,
+                        long long kc_block_stride, long long kc_page_stride, long long kc_head_stride, long long vc_block_stride,
+                        long long vc_page_stride, long long vc_head_stride, float softmax_scale, const void* seq_order,
+                        long long total_q, void* lse, void* stream);
+}  // namespace b200
+
 // Same, with an optional processing order: seq_order[i] (int32, a permutation of 0..num_seqs-1, e.g.
 // sequences by descending context length) is the sequence the i-th group of tiles belongs to.  The
 // order changes which CTA computes a sequence and when, never a result.  The mma.sync kernel ignores it.
@@ -479,6 +491,42 @@ extern "C" int b200_paged_attn_fwd_ordered(const void* q, const void* k_cache, c
                                            long long kc_head_stride, long long vc_block_stride,
                                            long long vc_page_stride, long long vc_head_stride, float softmax_scale,
                                            const void* seq_order, long long total_q, void* stream) {
+  return b200::paged_attn_fwd_impl(
+      q, k_cache, v_cache, out, cu_seqlens_q, seqused_k, page_table, num_seqs, max_seqlen_q, num_q_heads, num_kv_heads, dk, dv,
+      num_blocks, page_size, max_pages, page_table_stride, q_tok_stride, q_head_stride, o_tok_stride, o_head_stride, kc_block_stride,
+      kc_page_stride, kc_head_stride, vc_block_stride, vc_page_stride, vc_head_stride, softmax_scale, seq_order, total_q, nullptr, stream);
+}
+
+// The same, and lse_f32 [num_q_heads, total_q] receives log2 of every query's sum of 2^(score * softmax_scale * log2 e) over the
+// unrounded weights (queries of a refused sequence keep what it held).  Head dims (128, 128) and (192, 128), 16-byte aligned
+// queries.
+extern "C" int b200_paged_attn_fwd_lse(const void* q, const void* k_cache, const void* v_cache, void* out,
+                                           const void* cu_seqlens_q, const void* seqused_k, const void* page_table,
+                                           int num_seqs, int max_seqlen_q, int num_q_heads, int num_kv_heads,
+                                           int dk, int dv, int num_blocks, int page_size, int max_pages,
+                                           long long page_table_stride, long long q_tok_stride,
+                                           long long q_head_stride, long long o_tok_stride, long long o_head_stride,
+                                           long long kc_block_stride, long long kc_page_stride,
+                                           long long kc_head_stride, long long vc_block_stride,
+                                           long long vc_page_stride, long long vc_head_stride, float softmax_scale,
+                                           const void* seq_order, long long total_q, void* lse_f32, void* stream) {
+  if (!lse_f32) return B200_ERR_ARG;
+  return b200::paged_attn_fwd_impl(
+      q, k_cache, v_cache, out, cu_seqlens_q, seqused_k, page_table, num_seqs, max_seqlen_q, num_q_heads, num_kv_heads, dk, dv,
+      num_blocks, page_size, max_pages, page_table_stride, q_tok_stride, q_head_stride, o_tok_stride, o_head_stride, kc_block_stride,
+      kc_page_stride, kc_head_stride, vc_block_stride, vc_page_stride, vc_head_stride, softmax_scale, seq_order, total_q, lse_f32, stream);
+}
+
+int b200::paged_attn_fwd_impl(const void* q, const void* k_cache, const void* v_cache, void* out,
+                                           const void* cu_seqlens_q, const void* seqused_k, const void* page_table,
+                                           int num_seqs, int max_seqlen_q, int num_q_heads, int num_kv_heads,
+                                           int dk, int dv, int num_blocks, int page_size, int max_pages,
+                                           long long page_table_stride, long long q_tok_stride,
+                                           long long q_head_stride, long long o_tok_stride, long long o_head_stride,
+                                           long long kc_block_stride, long long kc_page_stride,
+                                           long long kc_head_stride, long long vc_block_stride,
+                                           long long vc_page_stride, long long vc_head_stride, float softmax_scale,
+                                           const void* seq_order, long long total_q, void* lse, void* stream) {
   using namespace b200;
   if (!q || !k_cache || !v_cache || !out || !cu_seqlens_q || !seqused_k || !page_table || num_seqs < 0 ||
       max_seqlen_q < 0 || num_q_heads <= 0 || num_kv_heads <= 0 || num_blocks <= 0 || page_size <= 0 ||
@@ -533,8 +581,10 @@ extern "C" int b200_paged_attn_fwd_ordered(const void* q, const void* k_cache, c
     // columns); steps with longer query runs use 128-row tiles with two threads per row (attn_rows.cuh): four
     // prompts of together 3001 tokens, 16 heads of 192 / 128, took 225 us on 32-column keys-on-lanes tiles, whose
     // softmax crosses lanes.  B200_ATTN_PREFILL=cols keeps those tiles (the same bits, for cross-checks).
-    const bool rows = max_seqlen_q > 1 && attn_prefill_rows();
-    const int nc = max_seqlen_q == 1 ? 16 : rows ? 128 : dk == 128 ? 64 : 32;
+    const bool rows = lse || (max_seqlen_q > 1 && attn_prefill_rows());
+    p.lse = (float*)lse;
+    p.lse_stride = total_q;
+    const int nc = rows ? 128 : max_seqlen_q == 1 ? 16 : dk == 128 ? 64 : 32;
     p.pos_per_tile = nc / hh;
     dim3 grid((unsigned)((max_seqlen_q + p.pos_per_tile - 1) / p.pos_per_tile),
               (unsigned)(num_kv_heads * p.head_chunks), (unsigned)num_seqs);
@@ -575,6 +625,7 @@ extern "C" int b200_paged_attn_fwd_ordered(const void* q, const void* k_cache, c
     }
     return attn_tc_dispatch(tk, tv, p, grid, dk, nc, st);
   }
+  if (lse) return B200_ERR_SHAPE;
   const int q_tiles = (max_seqlen_q + p.pos_per_tile - 1) / p.pos_per_tile;
   dim3 grid((unsigned)q_tiles, (unsigned)(num_kv_heads * p.head_chunks), (unsigned)num_seqs);
   if (dk == 128 && dv == 128) return attn_launch<128, 128, 3>(tk, tv, p, grid, st);

@@ -25,11 +25,12 @@ constexpr int AB_THREADS = 256;   // thread (ty, tx) = (tid / 16, tid % 16)
 struct AttnBwdParams {
   const __nv_bfloat16 *q, *k, *v, *out, *dout;   // [total_q, hq, DK], [total_k, hkv, DK], [total_k, hkv, DV], [total_q, hq, DV] x 2
   __nv_bfloat16 *dq, *dk, *dv;
-  float *lse, *delta;                            // scratch [total_q, hq]
+  float *lse, *delta;                            // scratch [total_q, hq]; with have_lse, lse comes from the forward
   const int *cu_q, *cu_k;                        // [num_seqs + 1]
   int hq, hkv;
   long long total_q, total_k;
   float scale;
+  int have_lse = 0;                              // tcgen05 kernels
 };
 
 // rows x D bf16 values (row r at src + r * row_stride) -> fp32 tile dst[32][D + 1]; rows past `valid` are zeros.

@@ -3,7 +3,9 @@
 // 64 rows at a time.
 //
 //   dq kernel:  a CTA owns 128 queries of one head (A operands Q and dO) and walks the keys:
-//               S = Q K^T, dP = dO V^T, dQ += bf16(dS) K.  A first walk over the keys (S alone) gives the log-sum-exp.
+//               S = Q K^T, dP = dO V^T, dQ += bf16(dS) K.  A first walk over the keys (S alone) gives the log-sum-exp, where the
+//               forward did not leave it (4 x 2048 tokens, 32 / 4 heads of 128: 534 us
+//               with that walk, 388 without; the forward's second row sum costs it 334 -> 367).
 //   dkv kernel: a CTA owns 128 keys of one KV head (A operands K and V) and walks its query heads and their queries:
 //               S^T = K Q^T, dP^T = V dO^T, dV += bf16(P^T) dO, dK += bf16(dS^T) Q.
 //
@@ -98,7 +100,7 @@ attn_bwd_tc_kernel(const __grid_constant__ AbtMaps tm, const AttnBwdParams p, in
   const int first = DKV ? max(0, m0 - shift) / ABT_N : 0;
   const int end = DKV ? q_len : min(kv_len, m0 + rows + shift);
   const int nt = max(0, (end + ABT_N - 1) / ABT_N - first);
-  const int walk1 = DKV ? 0 : nt;                    // dq: steps of the first walk
+  const int walk1 = DKV || p.have_lse ? 0 : nt;      // dq: steps of the first walk
   const int steps = walk1 + (DKV ? group * nt : nt);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -293,6 +295,7 @@ attn_bwd_tc_kernel(const __grid_constant__ AbtMaps tm, const AttnBwdParams p, in
       s_row[half * ABT_M + row] = acc;
       ptx::named_barrier_sync(1, 256);
       delta = s_row[row] + s_row[ABT_M + row];
+      if (p.have_lse) lse = live ? p.lse[(long long)head * p.total_q + q0 + own] : INFINITY;
       // first walk: running maximum and sum over this thread's half of every key tile, in units of log2
       float m = -INFINITY, l = 0.f;
       const int pos = own + shift;
@@ -332,16 +335,18 @@ attn_bwd_tc_kernel(const __grid_constant__ AbtMaps tm, const AttnBwdParams p, in
       ptx::named_barrier_sync(1, 256);
       if (*abort_flag) alive = false;
       // join the halves: (m, l) of the partner through shared memory, the sums in the order half 0, half 1
-      s_row[half * ABT_M + row] = m;
-      ptx::named_barrier_sync(1, 256);
-      const float mj = fmaxf(s_row[row], s_row[ABT_M + row]);
-      ptx::named_barrier_sync(1, 256);
-      s_row[half * ABT_M + row] = m > -INFINITY ? l * fast_exp2(m - mj) : 0.f;
-      ptx::named_barrier_sync(1, 256);
-      const float sum = s_row[row] + s_row[ABT_M + row];
-      lse = sum > 0.f ? mj + log2f(sum) : INFINITY;                // no key: every weight is zero
+      if (!p.have_lse) {
+        s_row[half * ABT_M + row] = m;
+        ptx::named_barrier_sync(1, 256);
+        const float mj = fmaxf(s_row[row], s_row[ABT_M + row]);
+        ptx::named_barrier_sync(1, 256);
+        s_row[half * ABT_M + row] = m > -INFINITY ? l * fast_exp2(m - mj) : 0.f;
+        ptx::named_barrier_sync(1, 256);
+        const float sum = s_row[row] + s_row[ABT_M + row];
+        lse = sum > 0.f ? mj + log2f(sum) : INFINITY;              // no key: every weight is zero
+      }
       if (live && half == 0 && alive) {
-        p.lse[(long long)head * p.total_q + q0 + own] = lse;
+        if (!p.have_lse) p.lse[(long long)head * p.total_q + q0 + own] = lse;
         p.delta[(long long)head * p.total_q + q0 + own] = delta;
       }
     }
@@ -487,18 +492,13 @@ inline int attn_bwd_tc_launch(const AttnBwdParams& p, int num_seqs, int max_seql
 
 }  // namespace b200
 
-// dq, dk, dv of packed causal varlen attention (triton_invariant_attention.py:194-431).  All tensors bf16 and
-// contiguous: q / dq [total_q, hq, dk_dim], k / dk [total_k, hkv, dk_dim], v / dv [total_k, hkv, dv_dim], out /
-// dout [total_q, hq, dv_dim]; cu_seqlens_q / _k [num_seqs + 1] int32; lse / delta: fp32 scratch of total_q * hq values.
-// (dk_dim, dv_dim) one of (64, 64), (128, 128), (192, 128).  Keys or queries of no sequence keep what dq / dk / dv
-// held (pass zero-filled tensors).  Sequences longer than max_seqlen_q / max_seqlen_k are reported (status code 2).
-extern "C" int b200_varlen_attn_backward(const void* q, const void* k, const void* v, const void* out, const void* dout,
+namespace b200 {
+inline int varlen_attn_backward_impl(const void* q, const void* k, const void* v, const void* out, const void* dout,
                                          const void* cu_seqlens_q, const void* cu_seqlens_k, void* dq, void* dk,
                                          void* dv, void* lse_scratch_f32, void* delta_scratch_f32, int num_seqs,
                                          int max_seqlen_q, int max_seqlen_k, long long total_q, long long total_k,
                                          int num_q_heads, int num_kv_heads, int dk_dim, int dv_dim,
-                                         float softmax_scale, void* stream) {
-  using namespace b200;
+                                         float softmax_scale, int have_lse, void* stream) {
   if (!q || !k || !v || !out || !dout || !cu_seqlens_q || !cu_seqlens_k || !dq || !dk || !dv || !lse_scratch_f32 ||
       !delta_scratch_f32 || num_seqs < 0 || max_seqlen_q < 0 || max_seqlen_k < 0 || total_q < 0 || total_k < 0 ||
       num_q_heads <= 0 || num_kv_heads <= 0)
@@ -512,13 +512,14 @@ extern "C" int b200_varlen_attn_backward(const void* q, const void* k, const voi
                   (const int*)cu_seqlens_k, num_q_heads, num_kv_heads, total_q, total_k, softmax_scale};
   cudaStream_t st = (cudaStream_t)stream;
   static const int simt = env_int("B200_ATTN_BWD_SIMT", 0);     // development knob: the CUDA-core kernels
-  if (simt) {
+  if (simt) {     // (these make their own log-sum-exp, over the forward's)
     if (dk_dim == 64 && dv_dim == 64) return attn_bwd_launch<64, 64>(p, num_seqs, max_seqlen_q, max_seqlen_k, st);
     if (dk_dim == 128 && dv_dim == 128) return attn_bwd_launch<128, 128>(p, num_seqs, max_seqlen_q, max_seqlen_k, st);
     if (dk_dim == 192 && dv_dim == 128) return attn_bwd_launch<192, 128>(p, num_seqs, max_seqlen_q, max_seqlen_k, st);
     return B200_ERR_SHAPE;
   }
-  if (dk_dim == 64 && dv_dim == 64) return attn_bwd_mma_launch<64, 64>(p, num_seqs, max_seqlen_q, max_seqlen_k, st);
+  p.have_lse = have_lse;
+  if (dk_dim == 64 && dv_dim == 64) return have_lse ? B200_ERR_SHAPE : attn_bwd_mma_launch<64, 64>(p, num_seqs, max_seqlen_q, max_seqlen_k, st);
   if ((reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(k) | reinterpret_cast<uintptr_t>(v) |
        reinterpret_cast<uintptr_t>(out) | reinterpret_cast<uintptr_t>(dout) | reinterpret_cast<uintptr_t>(dq) |
        reinterpret_cast<uintptr_t>(dk) | reinterpret_cast<uintptr_t>(dv)) & 15)
@@ -526,4 +527,34 @@ extern "C" int b200_varlen_attn_backward(const void* q, const void* k, const voi
   if (dk_dim == 128 && dv_dim == 128) return attn_bwd_tc_launch<128, 128>(p, num_seqs, max_seqlen_q, max_seqlen_k, st);
   if (dk_dim == 192 && dv_dim == 128) return attn_bwd_tc_launch<192, 128>(p, num_seqs, max_seqlen_q, max_seqlen_k, st);
   return B200_ERR_SHAPE;
+}
+}  // namespace b200
+
+// dq, dk, dv of packed causal varlen attention (triton_invariant_attention.py:194-431).  All tensors bf16 and
+// contiguous: q / dq [total_q, hq, dk_dim], k / dk [total_k, hkv, dk_dim], v / dv [total_k, hkv, dv_dim], out /
+// dout [total_q, hq, dv_dim]; cu_seqlens_q / _k [num_seqs + 1] int32; lse / delta: fp32 scratch of total_q * hq values.
+// (dk_dim, dv_dim) one of (64, 64), (128, 128), (192, 128).  Keys or queries of no sequence keep what dq / dk / dv
+// held (pass zero-filled tensors).  Sequences longer than max_seqlen_q / max_seqlen_k are reported (status code 2).
+extern "C" int b200_varlen_attn_backward(const void* q, const void* k, const void* v, const void* out, const void* dout,
+                                         const void* cu_seqlens_q, const void* cu_seqlens_k, void* dq, void* dk,
+                                         void* dv, void* lse_scratch_f32, void* delta_scratch_f32, int num_seqs,
+                                         int max_seqlen_q, int max_seqlen_k, long long total_q, long long total_k,
+                                         int num_q_heads, int num_kv_heads, int dk_dim, int dv_dim,
+                                         float softmax_scale, void* stream) {
+  return b200::varlen_attn_backward_impl(q, k, v, out, dout, cu_seqlens_q, cu_seqlens_k, dq, dk, dv, lse_scratch_f32, delta_scratch_f32,
+                                         num_seqs, max_seqlen_q, max_seqlen_k, total_q, total_k, num_q_heads, num_kv_heads, dk_dim,
+                                         dv_dim, softmax_scale, 0, stream);
+}
+
+// The same with lse_scratch_f32 as b200_paged_attn_fwd_lse left it ([num_q_heads, total_q]); it is overwritten where the
+// development knob selects the CUDA-core kernels.  Head dims (128, 128) and (192, 128).
+extern "C" int b200_varlen_attn_backward_lse(const void* q, const void* k, const void* v, const void* out, const void* dout,
+                                         const void* cu_seqlens_q, const void* cu_seqlens_k, void* dq, void* dk,
+                                         void* dv, void* lse_scratch_f32, void* delta_scratch_f32, int num_seqs,
+                                         int max_seqlen_q, int max_seqlen_k, long long total_q, long long total_k,
+                                         int num_q_heads, int num_kv_heads, int dk_dim, int dv_dim,
+                                         float softmax_scale, void* stream) {
+  return b200::varlen_attn_backward_impl(q, k, v, out, dout, cu_seqlens_q, cu_seqlens_k, dq, dk, dv, lse_scratch_f32, delta_scratch_f32,
+                                         num_seqs, max_seqlen_q, max_seqlen_k, total_q, total_k, num_q_heads, num_kv_heads, dk_dim,
+                                         dv_dim, softmax_scale, 1, stream);
 }

@@ -18,6 +18,7 @@ namespace b200 {
 constexpr int GATE_NONE = 0, GATE_HEAD = 1, GATE_COLUMN = 2;
 // Forms of an attention kernel: softmax inside a window and nothing else, softmax with all of the above, sigmoid weights.
 constexpr int ATTN_PLAIN = 0, ATTN_EXTRAS = 1, ATTN_SIGMOID = 2;
+constexpr int ATTN_LSE = 3;   // rows-on-lanes kernel: plain, and the rows' log-sum-exp for the backward
 
 // A cap and the coefficients of cap * tanh(s / cap) = s + c3 s^3 + c5 s^5 + c7 s^7 .. in the scores' units.
 struct ScoreCap {

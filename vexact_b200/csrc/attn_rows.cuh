@@ -26,7 +26,8 @@
 // are not walked), and heads may be narrower than 128 columns (the rest arrives as zeros and is not stored).  The second
 // P tile takes the place of the second Q buffer.  FORM ATTN_EXTRAS: kept first tokens, chunks of keys, capped scores, a sink
 // in the row sum and an output gate besides (attn_extras.cuh).  ATTN_SIGMOID: all but the sink with sigmoid weights; no
-// maximum and no sum then, and O stays in TMEM from a tile's first block to its last.
+// maximum and no sum then, and O stays in TMEM from a tile's first block to its last.  ATTN_LSE: a second row sum over the
+// unrounded weights, and its logarithm for the backward, which then needs no walk of its own for it.
 //
 // Warps (12): 0 K producer, 1 UMMA issuer + TMEM owner, 2 V producer, 3 Q loader, 4-11 compute: a row is
 // shared by two threads (warps w and w + 4 of a lane quadrant), each taking 64 of the block's 128 keys for
@@ -92,7 +93,7 @@ paged_attn_rows_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_co
                        const __grid_constant__ CUtensorMap tm_gate, const AttnParams p) {
   // 192-wide keys: their second ring stage takes the place of the second V block and the second Q buffer
   constexpr int DV = 128, NC = ATR_ROWS, KST = 2, VST = DK > 128 ? 1 : 2;
-  constexpr bool EXTRAS = FORM != ATTN_PLAIN, SIGMOID = FORM == ATTN_SIGMOID;
+  constexpr bool SIGMOID = FORM == ATTN_SIGMOID, EXTRAS = FORM == ATTN_EXTRAS || SIGMOID, LSE = FORM == ATTN_LSE;
   constexpr int KH = DK / 64, VH = DV / 64;
   constexpr int K_BYTES = ATC_BN * DK * 2, V_BYTES = ATC_BN * DV * 2;
   constexpr int KV_BYTES = KST * K_BYTES + VST * V_BYTES;
@@ -404,6 +405,7 @@ paged_attn_rows_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_co
       float bias = 0.f;                                // of sigmoid weights, in units of log2
       if constexpr (SIGMOID) bias = p.extras.sigmoid_bias[t.kvh * p.group + t.hchunk * 8 + hd] * kLog2e;
       float m_run = -INFINITY, l_a = 0.f, l_b = 0.f;   // l of my two key groups (2 half, 2 half + 1)
+      Two l_x(0.f, 0.f);                               // LSE: the sum of unrounded weights, in two chains
       float o[64];
 #pragma unroll
       for (int i = 0; i < 64; ++i) o[i] = 0.f;
@@ -539,9 +541,12 @@ paged_attn_rows_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_co
         } else {
           float pf[32];
           uint32_t pk[16];
+          if constexpr (LSE) l_x = l_x * Two(alpha, alpha);
 #pragma unroll
           for (int i = 0; i < 32; i += 2) {
-            const __nv_bfloat162 b2 = __floats2bfloat162_rn(fast_exp2(v[i] - m_run), fast_exp2(v[i + 1] - m_run));
+            const float e0 = fast_exp2(v[i] - m_run), e1 = fast_exp2(v[i + 1] - m_run);
+            if constexpr (LSE) l_x = l_x + Two(e0, e1);
+            const __nv_bfloat162 b2 = __floats2bfloat162_rn(e0, e1);
             pf[i] = __low2float(b2);
             pf[i + 1] = __high2float(b2);
             pk[i >> 1] = *reinterpret_cast<const uint32_t*>(&b2);
@@ -552,8 +557,9 @@ paged_attn_rows_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_co
             *reinterpret_cast<uint4*>(p_half + sw128(row, q)) = make_uint4(pk[q * 4], pk[q * 4 + 1], pk[q * 4 + 2], pk[q * 4 + 3]);
 #pragma unroll
           for (int i = 0; i < 32; i += 2) {
-            const __nv_bfloat162 b2 =
-                __floats2bfloat162_rn(fast_exp2(v[32 + i] - m_run), fast_exp2(v[32 + i + 1] - m_run));
+            const float e0 = fast_exp2(v[32 + i] - m_run), e1 = fast_exp2(v[32 + i + 1] - m_run);
+            if constexpr (LSE) l_x = l_x + Two(e0, e1);
+            const __nv_bfloat162 b2 = __floats2bfloat162_rn(e0, e1);
             pf[i] = __low2float(b2);
             pf[i + 1] = __high2float(b2);
             pk[i >> 1] = *reinterpret_cast<const uint32_t*>(&b2);
@@ -643,6 +649,17 @@ paged_attn_rows_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_co
           float l_row = s_lh[0][row] + s_lh[1][row];
           if constexpr (EXTRAS) l_row += sink_term(p.extras, head, m_run);
           inv = 1.0f / l_row;
+          if constexpr (LSE) {
+            // both threads have read the sums; the unrounded ones meet in the same places
+            if (!pair_sync()) break;
+            float xa, xb;
+            l_x.get(xa, xb);
+            s_lh[half][row] = xa + xb;
+            if (!pair_sync()) break;
+            if (half == 0 && pi < npos)
+              p.lse[(long long)(t.kvh * p.group + t.hchunk * 8 + hd) * p.lse_stride + t.q_start + t.tile_pos0 + pi] =
+                  m_run + log2f(s_lh[0][row] + s_lh[1][row]);
+          }
         }
         if constexpr (EXTRAS) {
           inv *= p.extras.out_scale * head_gate;
@@ -754,6 +771,9 @@ inline int attn_rows_launch(const CUtensorMap& tk, const CUtensorMap& tv, const 
 
 inline int attn_rows_dispatch(const CUtensorMap& tk, const CUtensorMap& tv, const CUtensorMap& tq, const CUtensorMap& to,
                               const AttnParams& p, int dk, cudaStream_t st) {
+  if (p.lse)
+    return dk == 128 ? attn_rows_launch<128, false, ATTN_LSE>(tk, tv, tq, to, tk, p, st)
+                     : attn_rows_launch<192, false, ATTN_LSE>(tk, tv, tq, to, tk, p, st);
   return dk == 128 ? attn_rows_launch<128, false, ATTN_PLAIN>(tk, tv, tq, to, tk, p, st)
                    : attn_rows_launch<192, false, ATTN_PLAIN>(tk, tv, tq, to, tk, p, st);
 }
