@@ -21,7 +21,7 @@
 //
 // Pipeline.  Persistent CTAs (one per SM) walk a static round-robin tile list.
 // Warp 0 issues TMA loads into a ring of shared-memory stages, warp 1 issues
-// tcgen05.mma into one of two tensor-memory accumulators, warps 2-5 drain the
+// tcgen05.mma into one of two tensor-memory accumulators, warps 2-9 drain the
 // other accumulator (tcgen05.ld), apply the epilogue and store.  All waits are
 // bounded (ptx::mbar_wait).
 //
@@ -36,6 +36,7 @@
 // for decode shapes, so the roofline is HBM bandwidth.
 #pragma once
 #include <stdlib.h>
+#include <type_traits>
 #include <cuda.h>  // CUtensorMap and enums only: the encoder is looked up at run time, libcuda is not linked
 
 #include "ptx.cuh"
@@ -46,7 +47,7 @@ namespace b200 {
 constexpr int GEMM_BK = 64;             // K elements per stage = one 128-byte swizzle row
 constexpr int GEMM_WTILE = 128;         // weight rows per tile = UMMA M
 constexpr int GEMM_WBYTES = GEMM_WTILE * GEMM_BK * 2;
-constexpr int GEMM_THREADS = 192;       // producer warp, MMA warp, 4 epilogue warps
+constexpr int GEMM_THREADS = 320;       // producer warp, MMA warp, 8 epilogue warps: two per tensor-memory quadrant
 constexpr int GEMM_MAX_STAGES = 12;
 constexpr int GEMM_SMEM_BUDGET = 227 * 1024;
 // Tokens from which a dense product may run on CTA pairs: their set-up and the meeting of the CTAs cost about a microsecond,
@@ -262,7 +263,8 @@ gemm_ws_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__
     }
     for (int b = 0; b < 2; ++b) {
       ptx::mbar_init(tfull_bar(b), 1);
-      ptx::mbar_init(tempty_bar(b), PAIR ? 8 : 128);   // pairs: the epilogue warps of both CTAs, on rank 0's barrier
+      // pairs: the epilogue warps of both CTAs, on rank 0's barrier
+      ptx::mbar_init(tempty_bar(b), PAIR ? 16 : HEAD ? 128 : 256);
     }
     ptx::fence_barrier_init();
     ptx::prefetch_tensormap(&tm_w);
@@ -520,19 +522,20 @@ gemm_ws_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__
       }
     }
   } else {
-    // ------------------------------------------------------------ epilogue (warps 2..5)
+    // ------------------------------------------------------------ epilogue (warps 2..9; the head mode 2..5)
     const int q = warp & 3;              // tensor-memory lane quadrant this warp may read
+    const int eh = (warp - 2) >> 2;      // first or second half of the token columns
     uint32_t tile_it = 0;
-    for (long long lin = lin0;; lin += lin_step, ++tile_it) {
+    for (long long lin = lin0; !HEAD || eh == 0; lin += lin_step, ++tile_it) {
       GemmTile t;
       if (!tile_at(t_tiles, lin, t)) break;
       const int buf = tile_it & 1;
       const bool ready = ptx::mbar_wait(tfull_bar(buf), (tile_it >> 1) & 1, abort_flag, 400 + buf);
       if (SWIGLU || HEAD) {
-        // The four epilogue warps meet at named barriers below, so they must leave together: a wait
+        // The epilogue warps meet at named barriers below, so they must leave together: a wait
         // that gave up has raised the abort flag before its warp arrives here, and everyone reads
         // the flag after this barrier.
-        ptx::named_barrier_sync(1, 128);
+        ptx::named_barrier_sync(1, HEAD ? 128 : 256);
         if (*abort_flag) break;
       } else if (!__all_sync(0xffffffffu, ready)) {
         break;
@@ -541,6 +544,7 @@ gemm_ws_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__
       if (threadIdx.x == 64) GEMM_STAMP(4);   // accumulator complete
       const uint32_t taddr = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(buf * p.xrows_max);
       const int ncol = ((t.n + 15) / 16) * 16;
+      const int cmid = (ncol / 16 + 1) / 2 * 16, ca = eh ? cmid : 0, cb = eh ? ncol : cmid;   // this warp's columns
       if (HEAD) {
         // Thread = vocabulary row f of the tile; columns = tokens.  Per 16 columns: every logit is rounded
         // to bf16 (the logits tensor the reference materialises is bf16), then per column the warp's
@@ -664,10 +668,10 @@ gemm_ws_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__
         const bool vec_out = !p.scalar_epilogue && !p.out_f32 && (p.ldo & 7) == 0 && (p.n_w & 7) == 0 &&
                              (p.out_batch_stride & 7) == 0 && (reinterpret_cast<uintptr_t>(p.out) & 15) == 0;
         if (vec_out) {
-          __nv_bfloat16* stg = exch + q * (16 * 32);      // [16 tokens][32 features] per warp
+          __nv_bfloat16* stg = exch + (warp - 2) * (16 * 32);      // [16 tokens][32 features] per warp
           const int part = lane & 3, rsub = lane >> 2;
           const int f8 = t.wt * GEMM_WTILE + q * 32 + part * 8;
-          for (int c0 = 0; c0 < ncol; c0 += 16) {
+          for (int c0 = ca; c0 < cb; c0 += 16) {
             uint32_t r[16];
             ptx::tmem_ld16(taddr + c0, r);
             ptx::tmem_ld_wait();
@@ -686,7 +690,7 @@ gemm_ws_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__
             __syncwarp();
           }
         } else
-        for (int c0 = 0; c0 < ncol; c0 += 16) {
+        for (int c0 = ca; c0 < cb; c0 += 16) {
           uint32_t r[16];
           ptx::tmem_ld16(taddr + c0, r);
           ptx::tmem_ld_wait();
@@ -709,15 +713,17 @@ gemm_ws_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__
         }
       } else {
         // Lanes 0..63 hold the gate rows, lanes 64..127 the up rows of the same 64 features.  In the reference form, whose
-        // gate is a bf16 tensor too, both pairs of warps do the activation: the gate warps for the first half of the columns,
-        // the up warps for the rest, each handing the other what it lacks.  (With the exact exponential and the gate warps
-        // alone this bound the kernel at many rows per expert, and prefill took two plain products and an elementwise
-        // kernel: 2 x 49 + 30 us for 2048 tokens, 1536 -> 8960.)
+        // gate is a bf16 tensor too, gate and up warps share the activation: of a warp's columns the gate warps do the first
+        // half and the up warps the rest, each handing the other what it lacks; results leave 16 bytes a lane, turned around
+        // in shared memory as in the plain form.  (With four warps, the gate warps alone and the exact exponential this
+        // bound the kernel, and prefill took two plain products and an elementwise kernel: 2 x 49 + 30 us for 2048 tokens,
+        // 1536 -> 8960; shared among four warps with 2-byte stores 106 us in one.)
         const int fi = (q & 1) * 32 + lane;
         const bool both = p.glu == GLU_REFERENCE;
-        const int mid = both ? (ncol / 16 + 1) / 2 * 16 : ncol;
-        const int give0 = q < 2 ? mid : 0, give1 = q < 2 ? ncol : mid, take0 = q < 2 ? 0 : mid, take1 = q < 2 ? mid : ncol;
+        const int mid = both ? min(cb, ca + ((cb - ca) / 16 + 1) / 2 * 16) : cb;
+        const int give0 = q < 2 ? mid : ca, give1 = q < 2 ? cb : mid, take0 = q < 2 ? ca : mid, take1 = q < 2 ? mid : cb;
         __nv_bfloat16* mine = exch + fi * exch_pitch;
+        __nv_bfloat16* stg = exch + 64 * exch_pitch + (warp - 2) * (16 * 32);
         for (int c0 = give0; c0 < give1; c0 += 16) {
           uint32_t r[16];
           ptx::tmem_ld16(taddr + c0, r);
@@ -726,49 +732,61 @@ gemm_ws_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__
           for (int j = 0; j < 16; j += 2)
             *reinterpret_cast<uint32_t*>(mine + c0 + j) = pack_bf2(__uint_as_float(r[j]), __uint_as_float(r[j + 1]));
         }
-        ptx::named_barrier_sync(1, 128);
+        ptx::named_barrier_sync(1, 256);
         const int f = t.wt * 64 + fi;
         const bool fvalid = f < p.n_w;
+        const bool vec_out = (p.ldo & 7) == 0 && (p.n_w & 7) == 0 && (reinterpret_cast<uintptr_t>(p.out) & 15) == 0;
+        const int part = lane & 3, rsub = lane >> 2, f8 = t.wt * 64 + (q & 1) * 32 + part * 8;
         for (int c0 = take0; c0 < take1; c0 += 16) {
           uint32_t r[16];
           ptx::tmem_ld16(taddr + c0, r);
           ptx::tmem_ld_wait();
-          float other[16];
+          float h[16];
 #pragma unroll
           for (int j = 0; j < 16; j += 2)
-            unpack_bf2(*reinterpret_cast<const uint32_t*>(mine + c0 + j), other[j], other[j + 1]);
-          if (fvalid && !both) {
+            unpack_bf2(*reinterpret_cast<const uint32_t*>(mine + c0 + j), h[j], h[j + 1]);
+          if (!both) {
 #pragma unroll
             for (int j = 0; j < 16; ++j) {
-              const int c = c0 + j;
-              if (c < t.n) {
-                const float si = p.scale_in ? p.scale_in[t.row0 + c] : 1.f;
-                const float so = p.scale_out ? p.scale_out[t.row0 + c] : 1.f;
-                reinterpret_cast<__nv_bfloat16*>(p.out)[(long long)(t.row0 + c) * p.ldo + f] =
-                    f2bf(so * glu_value<__nv_bfloat16>(p.glu, si * __uint_as_float(r[j]), si * other[j]));
-              }
+              const bool in = c0 + j < t.n;
+              const float si = in && p.scale_in ? p.scale_in[t.row0 + c0 + j] : 1.f;
+              const float so = in && p.scale_out ? p.scale_out[t.row0 + c0 + j] : 1.f;
+              h[j] = so * glu_value<__nv_bfloat16>(p.glu, si * __uint_as_float(r[j]), si * h[j]);
             }
-          } else if (fvalid) {
-            float h[16];
+          } else {
 #pragma unroll
             for (int j = 0; j < 16; ++j) {
               // rounding points of fused_moe.py:319-336: each GEMM output, silu(), the gate*up product and (below) the
               // routing-weight product are bf16 tensors
               const float own = round_bf(__uint_as_float(r[j]));
-              h[j] = swiglu_reference(q < 2 ? own : other[j], q < 2 ? other[j] : own);
+              h[j] = swiglu_reference(q < 2 ? own : h[j], q < 2 ? h[j] : own);
             }
             if (p.row_scale) {
 #pragma unroll
               for (int j = 0; j < 16; ++j)
                 if (c0 + j < t.n) h[j] *= bf2f(p.row_scale[t.row0 + c0 + j]);
             }
+          }
+          if (vec_out) {
+#pragma unroll
+            for (int j = 0; j < 16; ++j) stg[j * 32 + lane] = f2bf(h[j]);
+            __syncwarp();
+#pragma unroll
+            for (int k = 0; k < 2; ++k) {
+              const int row = k * 8 + rsub, c = c0 + row;
+              const uint4 v = *reinterpret_cast<const uint4*>(stg + row * 32 + part * 8);
+              if (c < t.n && f8 < p.n_w)
+                *reinterpret_cast<uint4*>(reinterpret_cast<__nv_bfloat16*>(p.out) + (long long)(t.row0 + c) * p.ldo + f8) = v;
+            }
+            __syncwarp();
+          } else if (fvalid) {
 #pragma unroll
             for (int j = 0; j < 16; ++j)
               if (c0 + j < t.n)
                 reinterpret_cast<__nv_bfloat16*>(p.out)[(long long)(t.row0 + c0 + j) * p.ldo + f] = f2bf(h[j]);
           }
         }
-        ptx::named_barrier_sync(1, 128);  // exchange buffer is reused by the next tile
+        ptx::named_barrier_sync(1, 256);  // exchange buffer is reused by the next tile
       }
       ptx::tc_fence_before();
       if (PAIR) {
@@ -883,7 +901,8 @@ inline int env_int(const char* name, int dflt) {
 
 // Epilogue scratch after the stages: the SwiGLU exchange buffer, the head mode's per-warp partials, or the turning tiles.
 inline int gemm_exch_bytes(int mode, int xrows_max) {
-  return mode == GEMM_SWIGLU ? 64 * (xrows_max + GEMM_EXCH_PAD) * 2 : mode == GEMM_HEAD ? 3 * 4 * xrows_max * 4 : 4 * 16 * 32 * 2;
+  const int turn = 8 * 16 * 32 * 2;
+  return mode == GEMM_SWIGLU ? 64 * (xrows_max + GEMM_EXCH_PAD) * 2 + turn : mode == GEMM_HEAD ? 3 * 4 * xrows_max * 4 : turn;
 }
 // K atoms per stage: fewer, larger stages cut the per-stage barrier round trips; keep >= 3 stages.  (One token, 6144 -> 2048, at
 // 1 / 2 / 4 atoms: 31 / 24 / 20 us with a copy per atom.)
@@ -964,16 +983,12 @@ gemm_f32_kernel(const TIn* __restrict__ x, const TIn* __restrict__ w, const floa
 // four each (8- or 16-byte loads), of 4 tokens x 4 features, so eight loads feed 64 FMAs and the FMA pipe is the bound.
 constexpr int GF_TOKENS = 8, GF_FEATURES = 64;     // of a CTA: 2 x 4 warps of 4 tokens x 16 features
 template <typename TIn>
-__device__ __forceinline__ void gf_load(const TIn* p, float (&v)[4]) {
-  if constexpr (sizeof(TIn) == 2) {
-    const uint2 t = *reinterpret_cast<const uint2*>(p);
-    unpack_bf2(t.x, v[0], v[1]);
-    unpack_bf2(t.y, v[2], v[3]);
-  } else {
-    const float4 t = *reinterpret_cast<const float4*>(p);
-    v[0] = t.x, v[1] = t.y, v[2] = t.z, v[3] = t.w;
-  }
+using GfRaw = typename std::conditional<sizeof(TIn) == 2, uint2, float4>::type;
+__device__ __forceinline__ void gf_unpack(const uint2& t, float (&v)[4]) {
+  unpack_bf2(t.x, v[0], v[1]);
+  unpack_bf2(t.y, v[2], v[3]);
 }
+__device__ __forceinline__ void gf_unpack(const float4& t, float (&v)[4]) { v[0] = t.x, v[1] = t.y, v[2] = t.z, v[3] = t.w; }
 template <typename TIn>
 __global__ void __launch_bounds__(256)
 gemm_f32_group_kernel(const TIn* __restrict__ x, const TIn* __restrict__ w, const float* __restrict__ bias,
@@ -991,13 +1006,23 @@ gemm_f32_group_kernel(const TIn* __restrict__ x, const TIn* __restrict__ w, cons
     wr[i] = w + (long long)min(n0 + i, N - 1) * w_stride + 4 * l;
   }
   float acc[4][4][4] = {};
-#pragma unroll 2
+  GfRaw<TIn> xq[4], wq[4];      // requested one step ahead: sixteen warps an SM do not hide the loads by themselves
+  auto request = [&](int k) {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      xq[i] = *reinterpret_cast<const GfRaw<TIn>*>(xr[i] + k);
+      wq[i] = *reinterpret_cast<const GfRaw<TIn>*>(wr[i] + k);
+    }
+  };
+  request(0);
   for (int k = 0; k < K; k += 32) {
     float a[4][4], b[4][4];
 #pragma unroll
-    for (int i = 0; i < 4; ++i) gf_load(xr[i] + k, a[i]);
-#pragma unroll
-    for (int i = 0; i < 4; ++i) gf_load(wr[i] + k, b[i]);
+    for (int i = 0; i < 4; ++i) {
+      gf_unpack(xq[i], a[i]);
+      gf_unpack(wq[i], b[i]);
+    }
+    if (k + 32 < K) request(k + 32);
 #pragma unroll
     for (int i = 0; i < 4; ++i)
 #pragma unroll

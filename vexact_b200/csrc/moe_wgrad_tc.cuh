@@ -15,14 +15,14 @@
 // instruction and issues no instruction beyond.  An empty group gets zeros.  A group whose bounds leave [0, rows] or decrease
 // is clipped and reported through the status word.
 //
-// Warps (8): 0 TMA producer, 1 MMA issuer and TMEM owner, 2 - 3 idle, 4 - 7 epilogue.
+// Warps (12): 0 TMA producer, 1 MMA issuer and TMEM owner, 2 - 3 idle, 4 - 11 epilogue, two per tensor-memory quadrant.
 #pragma once
 #include "attn_tc.cuh"
 #include "gemm.cuh"
 
 namespace b200 {
 
-constexpr int WGT_THREADS = 256, WGT_M = 128, WGT_N = 256, WGT_ROWS = 64, WGT_STAGES = 3;
+constexpr int WGT_THREADS = 384, WGT_M = 128, WGT_N = 256, WGT_ROWS = 64, WGT_STAGES = 3;
 constexpr int WGT_BOX = WGT_ROWS * 128;                              // bytes of a 64 x 64 operand box
 constexpr int WGT_BOXES = (WGT_M + WGT_N) / 64, WGT_STAGE = WGT_BOXES * WGT_BOX;
 constexpr int WGT_OUT = WGT_M * WGT_N * 2;
@@ -43,7 +43,7 @@ __device__ __forceinline__ int wgrad_rows(const int* cu_seqlens, int g, int rows
 
 __global__ void __launch_bounds__(WGT_THREADS, 1)
 moe_wgrad_tc_kernel(const __grid_constant__ WgradMaps tm, const int* __restrict__ cu_seqlens, int rows, int groups, int m_tiles,
-                    int n_tiles, int N) {
+                    int n_tiles, int N, bool deep) {
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw = ptx::smem_u32(smem_raw);
   const uint32_t stage0 = (raw + 1023) & ~1023u, out0 = stage0 + WGT_STAGES * WGT_STAGE;
@@ -65,7 +65,7 @@ moe_wgrad_tc_kernel(const __grid_constant__ WgradMaps tm, const int* __restrict_
     }
     for (int b = 0; b < 2; ++b) {
       ptx::mbar_init(tfull(b), 1);
-      ptx::mbar_init(tempty(b), 128);
+      ptx::mbar_init(tempty(b), 256);
     }
     ptx::fence_barrier_init();
     ptx::prefetch_tensormap(&tm.a);
@@ -103,6 +103,11 @@ moe_wgrad_tc_kernel(const __grid_constant__ WgradMaps tm, const int* __restrict_
           }
           ptx::mbar_expect_tx(full(s), WGT_STAGE);
           const uint32_t at = stage0 + s * WGT_STAGE;
+          if (deep) {      // one copy an operand (make_tmap_deep): six boxes a step took longer to issue than to arrive
+            ptx::tma_load_3d(at, &tm.a, full(s), 0, r0 + r, m0 / 64, ptx::kEvictLast);
+            ptx::tma_load_3d(at + WGT_M / 64 * WGT_BOX, &tm.b, full(s), 0, r0 + r, n0 / 64, ptx::kEvictLast);
+            continue;
+          }
 #pragma unroll
           for (int h = 0; h < WGT_M / 64; ++h)
             ptx::tma_load_2d(at + h * WGT_BOX, &tm.a, full(s), m0 + h * 64, r0 + r, ptx::kEvictLast);
@@ -154,7 +159,7 @@ moe_wgrad_tc_kernel(const __grid_constant__ WgradMaps tm, const int* __restrict_
     }
   } else if (warp >= 4) {
     // ------------------------------------------------------------ epilogue
-    const int q = warp & 3, row = q * 32 + lane;
+    const int q = warp & 3, row = q * 32 + lane, half = (warp - 4) >> 2;
     uint32_t tile_it = 0;
     for (long long lin = blockIdx.x; lin < total; lin += gridDim.x, ++tile_it) {
       const int g = (int)(lin / per_group), t = (int)(lin % per_group), buf = tile_it & 1;
@@ -163,13 +168,14 @@ moe_wgrad_tc_kernel(const __grid_constant__ WgradMaps tm, const int* __restrict_
       const int n = wgrad_rows(cu_seqlens, g, rows, r0, false);
       ptx::mbar_wait(tfull(buf), (tile_it >> 1) & 1, abort_flag, 930 + buf);
       if (threadIdx.x == 128) ptx::bulk_wait_read0();      // the previous tile's copy out has read the staging tile
-      // a wait that gave up raised the flag before this barrier: all four warps leave together
-      ptx::named_barrier_sync(1, 128);
+      // a wait that gave up raised the flag before this barrier: all eight warps leave together
+      ptx::named_barrier_sync(1, 256);
       if (*abort_flag) break;
       ptx::tc_fence_after();
       const uint32_t taddr = tmem + ((uint32_t)(q * 32) << 16) + buf * WGT_N;
 #pragma unroll
-      for (int c = 0; c < WGT_N; c += 16) {
+      for (int i = 0; i < WGT_N / 2; i += 16) {
+        const int c = half * (WGT_N / 2) + i;
         uint32_t r[16];
         ptx::tmem_ld16(taddr + c, r);
         ptx::tmem_ld_wait();
@@ -187,7 +193,7 @@ moe_wgrad_tc_kernel(const __grid_constant__ WgradMaps tm, const int* __restrict_
       ptx::tc_fence_before();
       ptx::mbar_arrive(tempty(buf));
       ptx::fence_proxy_async_smem();
-      ptx::named_barrier_sync(1, 128);
+      ptx::named_barrier_sync(1, 256);
       if (threadIdx.x == 128) {
         for (int h = 0; h < WGT_N / 64; ++h)
           if (n0 + h * 64 < N) ptx::tma_store_3d(&tm.c, out0 + h * (WGT_M * 128), n0 + h * 64, m0, g);
@@ -219,14 +225,18 @@ inline int moe_wgrad_tc_launch(const void* a, long long a_stride, const void* b,
   WgradMaps tm;
   // a map has at least one row; without rows nothing is read
   const uint64_t map_rows = rows > 0 ? (uint64_t)rows : 1;
-  int rc = make_tmap_2d(&tm.a, a, map_rows, (uint64_t)M, (uint64_t)a_stride, WGT_ROWS);
-  if (!rc) rc = make_tmap_2d(&tm.b, b, map_rows, (uint64_t)N, (uint64_t)b_stride, WGT_ROWS);
+  const bool deep = M % 64 == 0 && N % 64 == 0;
+  int rc = deep ? make_tmap_deep(&tm.a, a, map_rows, (uint64_t)M, (uint64_t)a_stride, WGT_ROWS, WGT_M / 64)
+                : make_tmap_2d(&tm.a, a, map_rows, (uint64_t)M, (uint64_t)a_stride, WGT_ROWS);
+  if (!rc)
+    rc = deep ? make_tmap_deep(&tm.b, b, map_rows, (uint64_t)N, (uint64_t)b_stride, WGT_ROWS, WGT_N / 64)
+              : make_tmap_2d(&tm.b, b, map_rows, (uint64_t)N, (uint64_t)b_stride, WGT_ROWS);
   if (!rc) rc = make_tmap_3d(&tm.c, c, (uint64_t)groups, (uint64_t)M, (uint64_t)N, (uint64_t)M * N, (uint64_t)N, WGT_M);
   if (rc) return rc;
   const int m_tiles = (M + WGT_M - 1) / WGT_M, n_tiles = (N + WGT_N - 1) / WGT_N;
   const long long total = (long long)m_tiles * n_tiles * groups;
   launch_k(moe_wgrad_tc_kernel, dim3((unsigned)(total < sm_count() ? total : sm_count())), dim3(WGT_THREADS), WGT_SMEM, st, tm,
-           cu_seqlens, (int)rows, groups, m_tiles, n_tiles, N);
+           cu_seqlens, (int)rows, groups, m_tiles, n_tiles, N, deep);
   return launch_status();
 }
 
