@@ -335,20 +335,17 @@ moe_route_sigmoid_group_topk_kernel(const float* __restrict__ logits, long long 
   }
 }
 
-// Index build: one CTA of 1024 threads.  For flat index f = t * topk + k (the order
-// expert_index.flatten() has) computes its position in the stable sort by expert:
+// Index build.  For flat index f = t * topk + k (the order expert_index.flatten() has) computes its position in the stable
+// sort by expert:
 //   scatter_index[f] = cu_seqlens[e_f] + #{f' < f : e_f' == e_f}
 // plus cu_seqlens[E + 1] and the token-tile table of the grouped GEMM (tiles of at most
 // `tile_rows` consecutive rows of one expert).
 //
-// Warp w owns the contiguous segment [w * seg, (w + 1) * seg) of the flat array and walks it 32
-// entries at a time: __match_any_sync groups equal experts, the lowest lane of a group bumps the
-// warp's private per-expert counter, so every entry learns its rank among the warp's earlier
-// entries of the same expert.  A per-expert scan over the 32 warps and a scan over the experts
-// turn those ranks into global positions.  All of it is integer arithmetic: bit-exact.
-//
-// The walk is bound by the latency of its loads (16384 / 32768 entries took 25 / 47 us one step at a time), so a warp requests
-// eight steps' entries at once.
+// One CTA of 1024 threads per expert; each reads all entries and needs nothing from the others.  Warp w owns the contiguous
+// segment [w * seg, (w + 1) * seg) of the flat array and walks it 32 entries at a time, eight steps' entries requested at once:
+// a histogram of all experts in shared memory gives the rows and tiles before this one, a ballot per step the expert's own
+// entries in order.  All of it is integer arithmetic: bit-exact.  (One CTA for all experts, ranking by __match_any_sync, which
+// takes a turn per distinct value: 25 / 47 us for 16384 / 32768 entries of 128 experts.)
 constexpr int MOE_INDEX_AHEAD = 8;
 template <typename TIdx>
 __global__ void __launch_bounds__(1024)
@@ -358,124 +355,84 @@ moe_index_kernel(const TIdx* __restrict__ experts, long long n, int E, int tile_
                  const __nv_bfloat16* __restrict__ weights, __nv_bfloat16* __restrict__ row_scale) {
   pdl_trigger();
   pdl_wait();
-  __shared__ int cnt[32][MOE_MAX_EXPERTS];  // per-warp counts, then per-warp exclusive offsets
-  __shared__ int base[MOE_MAX_EXPERTS];     // expert totals, then exclusive prefix (cu_seqlens)
-  __shared__ int tbase[MOE_MAX_EXPERTS];    // first tile index of each expert
-  __shared__ int wsum[32];
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  for (int i = tid; i < 32 * MOE_MAX_EXPERTS; i += 1024) (&cnt[0][0])[i] = 0;
+  __shared__ int hist[MOE_MAX_EXPERTS];
+  __shared__ int own[32];                   // entries of this expert in each warp's segment
+  __shared__ int before[2];                 // rows and tiles of the experts before this one
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, mine = blockIdx.x;
+  for (int i = tid; i < MOE_MAX_EXPERTS; i += 1024) hist[i] = 0;
   __syncthreads();
   const long long seg = ((n + 31) / 32 + 31) / 32 * 32;  // entries per warp, a multiple of 32
   const long long w0 = warp * seg;
-  // pass 1: rank of every entry among the warp's earlier entries of the same expert
+  auto request = [&](long long o, int (&ev)[MOE_INDEX_AHEAD]) {     // -1: no entry, -2: not an expert
+#pragma unroll
+    for (int u = 0; u < MOE_INDEX_AHEAD; ++u) {
+      const long long i = w0 + o + 32 * u + lane;
+      ev[u] = -1;
+      if (o + 32 * u < seg && i < n) {
+        const long long v = (long long)experts[i];
+        ev[u] = v >= 0 && v < E ? (int)v : -2;
+      }
+    }
+  };
+  int count = 0;
   for (long long o = 0; o < seg; o += 32 * MOE_INDEX_AHEAD) {
-    long long ev[MOE_INDEX_AHEAD];
+    int ev[MOE_INDEX_AHEAD];
+    request(o, ev);
 #pragma unroll
     for (int u = 0; u < MOE_INDEX_AHEAD; ++u) {
-      const long long i = w0 + o + 32 * u + lane;
-      ev[u] = o + 32 * u < seg && i < n ? (long long)experts[i] : -1;
+      if (ev[u] >= 0) {
+        atomicAdd(&hist[ev[u]], 1);
+      } else if (ev[u] == -2 && mine == 0) {
+        const long long i = w0 + o + 32 * u + lane;
+        scatter_index[i] = -1;
+        report_status(B200_STATUS_BAD_INDEX, (int)experts[i]);
+      }
+      count += __popc(__ballot_sync(0xffffffffu, ev[u] == mine));
     }
-#pragma unroll
-    for (int u = 0; u < MOE_INDEX_AHEAD; ++u) {
-      if (o + 32 * u >= seg) break;
-      const long long i = w0 + o + 32 * u + lane;
-      int e = -1;
-      if (i < n) {
-        if (ev[u] >= 0 && ev[u] < E)
-          e = (int)ev[u];
-        else
-          report_status(B200_STATUS_BAD_INDEX, (int)ev[u]);
-      }
-      const unsigned mask = __match_any_sync(0xffffffffu, e);
-      const int rank = __popc(mask & ((1u << lane) - 1u));
-      const int leader = __ffs(mask) - 1;
-      int old = 0;
-      if (rank == 0 && e >= 0) {
-        old = cnt[warp][e];
-        cnt[warp][e] = old + __popc(mask);
-      }
-      old = __shfl_sync(0xffffffffu, old, leader);
-      if (i < n) scatter_index[i] = e >= 0 ? old + rank : -1;
-      __syncwarp();
+  }
+  if (lane == 0) own[warp] = count;
+  __syncthreads();
+  if (warp == 0) {
+    int rows = 0, tiles = 0;
+    for (int e = lane; e < mine; e += 32) {
+      rows += hist[e];
+      tiles += (hist[e] + tile_rows - 1) / tile_rows;
+    }
+    rows = __reduce_add_sync(0xffffffffu, rows);
+    tiles = __reduce_add_sync(0xffffffffu, tiles);
+    if (lane == 0) {
+      before[0] = rows;
+      before[1] = tiles;
     }
   }
   __syncthreads();
-  // per expert: exclusive scan over the warps, total into base[]
-  if (tid < E) {
-    int run = 0;
-#pragma unroll 8
-    for (int w = 0; w < 32; ++w) {
-      const int c = cnt[w][tid];
-      cnt[w][tid] = run;
-      run += c;
-    }
-    base[tid] = run;
-  }
-  __syncthreads();
-  // exclusive scans over the experts (rows and tiles), 256 threads = 8 warps
-  if (tid < MOE_MAX_EXPERTS) {
-    const int rows = tid < E ? base[tid] : 0;
-    const int tiles = (rows + tile_rows - 1) / tile_rows;
-    int r = rows, t = tiles;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const int r2 = __shfl_up_sync(0xffffffffu, r, o);
-      const int t2 = __shfl_up_sync(0xffffffffu, t, o);
-      if (lane >= o) {
-        r += r2;
-        t += t2;
-      }
-    }
-    if (lane == 31) {
-      wsum[warp] = r;
-      wsum[8 + warp] = t;
-    }
-    // (only warps 0..7 reach here; named barrier over their 256 threads)
-    asm volatile("bar.sync 2, 256;" ::: "memory");
-    int roff = 0, toff = 0;
-    for (int w = 0; w < warp; ++w) {
-      roff += wsum[w];
-      toff += wsum[8 + w];
-    }
-    const int rexcl = roff + r - rows;
-    const int texcl = toff + t - tiles;
-    asm volatile("bar.sync 2, 256;" ::: "memory");
-    if (tid < E) {
-      base[tid] = rexcl;
-      tbase[tid] = texcl;
-      cu_seqlens[tid] = rexcl;
-      for (int j = 0; j < tiles; ++j)
-        if (texcl + j < max_tiles)
-          tile_table[texcl + j] = token_tile(tid, rexcl, rows, tiles, j);
-      if (tid == E - 1) {
-        cu_seqlens[E] = rexcl + rows;
-        *tile_count = min(texcl + tiles, max_tiles);
-      }
+  const int row0 = before[0], rows = hist[mine], tiles = (rows + tile_rows - 1) / tile_rows;
+  if (tid == 0) {
+    cu_seqlens[mine] = row0;
+    if (mine == E - 1) {
+      cu_seqlens[E] = row0 + rows;
+      *tile_count = min(before[1] + tiles, max_tiles);
     }
   }
-  __syncthreads();
-  // pass 2: local rank -> global position
+  for (int j = tid; j < tiles; j += 1024)
+    if (before[1] + j < max_tiles) tile_table[before[1] + j] = token_tile(mine, row0, rows, tiles, j);
+  int at = row0 + __reduce_add_sync(0xffffffffu, lane < warp ? own[lane] : 0);
   for (long long o = 0; o < seg; o += 32 * MOE_INDEX_AHEAD) {
-    long long ev[MOE_INDEX_AHEAD];
-    int rank[MOE_INDEX_AHEAD];
+    int ev[MOE_INDEX_AHEAD];
+    request(o, ev);
 #pragma unroll
     for (int u = 0; u < MOE_INDEX_AHEAD; ++u) {
-      const long long i = w0 + o + 32 * u + lane;
-      const bool in = o + 32 * u < seg && i < n;
-      ev[u] = in ? (long long)experts[i] : -1;
-      rank[u] = in ? scatter_index[i] : 0;
-    }
-#pragma unroll
-    for (int u = 0; u < MOE_INDEX_AHEAD; ++u) {
-      const long long i = w0 + o + 32 * u + lane;
-      if (ev[u] >= 0 && ev[u] < E) {
-        const int pos = rank[u] + base[(int)ev[u]] + cnt[warp][(int)ev[u]];
+      const unsigned mask = __ballot_sync(0xffffffffu, ev[u] == mine);
+      if (ev[u] == mine) {
+        const long long i = w0 + o + 32 * u + lane;
+        const int pos = at + __popc(mask & ((1u << lane) - 1u));
         scatter_index[i] = pos;
         // the inverse map for a GEMM that gathers its rows (sorted row -> token), and the routing weight
         // of each sorted row, so that no permuted copy of the activations has to be made
         if (gather_index) gather_index[pos] = (int)(i / topk);
         if (row_scale) row_scale[pos] = weights[i];
       }
+      at += __popc(mask);
     }
   }
 }
@@ -1221,11 +1178,11 @@ extern "C" int b200_moe_permute(const void* experts, int experts_dtype /*0 = i32
   cudaStream_t st = (cudaStream_t)stream;
   const long long n = T * topk;
   if (experts_dtype == 0)
-    launch_k(moe_index_kernel<int>, dim3(1), dim3(1024), 0, st, (const int*)experts, n, E, tile_rows, (int*)scatter_index,
+    launch_k(moe_index_kernel<int>, dim3((unsigned)E), dim3(1024), 0, st, (const int*)experts, n, E, tile_rows, (int*)scatter_index,
              (int*)cu_seqlens, (int4*)tile_table, (int*)tile_count, max_tiles, 1, (int*)nullptr,
              (const __nv_bfloat16*)nullptr, (__nv_bfloat16*)nullptr);
   else if (experts_dtype == 1)
-    launch_k(moe_index_kernel<long long>, dim3(1), dim3(1024), 0, st, (const long long*)experts, n, E, tile_rows,
+    launch_k(moe_index_kernel<long long>, dim3((unsigned)E), dim3(1024), 0, st, (const long long*)experts, n, E, tile_rows,
              (int*)scatter_index, (int*)cu_seqlens, (int4*)tile_table, (int*)tile_count, max_tiles, 1,
              (int*)nullptr, (const __nv_bfloat16*)nullptr, (__nv_bfloat16*)nullptr);
   else
@@ -1254,11 +1211,11 @@ extern "C" int b200_moe_permute_index(const void* experts, int experts_dtype /*0
   cudaStream_t st = (cudaStream_t)stream;
   const long long n = T * topk;
   if (experts_dtype == 0)
-    launch_k(moe_index_kernel<int>, dim3(1), dim3(1024), 0, st, (const int*)experts, n, E, tile_rows,
+    launch_k(moe_index_kernel<int>, dim3((unsigned)E), dim3(1024), 0, st, (const int*)experts, n, E, tile_rows,
              (int*)scatter_index, (int*)cu_seqlens, (int4*)tile_table, (int*)tile_count, max_tiles, topk,
              (int*)gather_index, (const __nv_bfloat16*)weights_bf16, (__nv_bfloat16*)row_scale);
   else if (experts_dtype == 1)
-    launch_k(moe_index_kernel<long long>, dim3(1), dim3(1024), 0, st, (const long long*)experts, n, E, tile_rows,
+    launch_k(moe_index_kernel<long long>, dim3((unsigned)E), dim3(1024), 0, st, (const long long*)experts, n, E, tile_rows,
              (int*)scatter_index, (int*)cu_seqlens, (int4*)tile_table, (int*)tile_count, max_tiles, topk,
              (int*)gather_index, (const __nv_bfloat16*)weights_bf16, (__nv_bfloat16*)row_scale);
   else
