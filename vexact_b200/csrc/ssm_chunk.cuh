@@ -61,20 +61,21 @@ struct SsmChunkParams {
   int min_len;
 };
 
-template <int NMAX, int PS>
+template <int NMAX, int PS, int ST_N>
 struct SscLayout {
-  static constexpr int STAGES = NMAX <= 128 ? 2 : 1;
+  static constexpr int STAGES = ST_N;
   static constexpr int LDN = NMAX + 8, LDP = PS + 8;          // padded pitches: ldmatrix rows in distinct banks
   static constexpr int BC = SSC_L * LDN * 2;                   // bytes of one B or C tile
   static constexpr int X = SSC_L * LDP * 2;
   static constexpr int ST = NMAX * LDP * 2;
   static constexpr int STAGE = 2 * BC + X + SSC_L * 4;         // B, C, x, dt
   static constexpr int BYTES = STAGES * STAGE + 2 * X + 2 * ST + SSC_L * 4;
+  static constexpr int PER_SM = 227 * 1024 / (BYTES + 1024);   // CTAs that share an SM (1 KB of each is the system's)
 };
 
-template <int NMAX, int PS>
+template <int NMAX, int PS, int ST_N>
 __global__ void __launch_bounds__(SSC_THREADS) ssm_chunk_kernel(const SsmChunkParams p) {
-  using L = SscLayout<NMAX, PS>;
+  using L = SscLayout<NMAX, PS, ST_N>;
   constexpr int NT = NMAX / 64;                      // state row tiles per warp
   constexpr bool KEEP_C = NMAX <= 128;               // the warp's rows of C stay in registers
   constexpr int PT = PS / 8;
@@ -333,15 +334,29 @@ __global__ void __launch_bounds__(SSC_THREADS) ssm_chunk_kernel(const SsmChunkPa
   }
 }
 
-template <int NMAX, int PS>
-inline int ssm_chunk_launch(const SsmChunkParams& p, cudaStream_t st) {
-  constexpr int smem = SscLayout<NMAX, PS>::BYTES;
+template <int NMAX, int PS, int ST_N>
+inline int ssm_chunk_launch_staged(const SsmChunkParams& p, cudaStream_t st) {
+  constexpr int smem = SscLayout<NMAX, PS, ST_N>::BYTES;
   static_assert(smem <= 227 * 1024, "shared memory budget");
   static PerDeviceFlags attr_set;
-  if (int rc = set_max_dyn_smem_once(attr_set, ssm_chunk_kernel<NMAX, PS>, smem)) return rc;
-  launch_k(ssm_chunk_kernel<NMAX, PS>, dim3((unsigned)((p.P + PS - 1) / PS), (unsigned)p.heads, (unsigned)p.seqs.num_seqs),
+  if (int rc = set_max_dyn_smem_once(attr_set, ssm_chunk_kernel<NMAX, PS, ST_N>, smem)) return rc;
+  launch_k(ssm_chunk_kernel<NMAX, PS, ST_N>, dim3((unsigned)((p.P + PS - 1) / PS), (unsigned)p.heads, (unsigned)p.seqs.num_seqs),
            dim3(SSC_THREADS), (size_t)smem, st, p);
   return launch_status();
+}
+
+// Two stages hide a chunk's copies under the one before; one stage lets more CTAs share an SM.  A CTA walks its chunks one after
+// the other, so what counts first is that all of them run at once: one stage where two would leave some for a second round
+// (4096 tokens of three prompts, 64 heads of 64 x 128 state: 384 CTAs, two or three to an SM; the hybrid prefill 3365 -> 3223 us).
+template <int NMAX, int PS>
+inline int ssm_chunk_launch(const SsmChunkParams& p, cudaStream_t st) {
+  if constexpr (NMAX <= 128) {
+    const long long ctas = (long long)((p.P + PS - 1) / PS) * p.heads * p.seqs.num_seqs;
+    constexpr int two = SscLayout<NMAX, PS, 2>::PER_SM, one = SscLayout<NMAX, PS, 1>::PER_SM;
+    auto rounds = [&](int per_sm) { return (ctas + (long long)per_sm * sm_count() - 1) / ((long long)per_sm * sm_count()); };
+    if (rounds(one) >= rounds(two)) return ssm_chunk_launch_staged<NMAX, PS, 2>(p, st);
+  }
+  return ssm_chunk_launch_staged<NMAX, PS, 1>(p, st);
 }
 
 }  // namespace b200
