@@ -202,10 +202,20 @@ def ptr(t) -> int | None:
     return None if t is None else t.data_ptr()
 
 
-def current_stream() -> int:
-    import torch
+_current_stream = None
 
-    return torch.cuda.current_stream().cuda_stream
+
+def current_stream() -> int:
+    """The current stream of the current device, without a Stream object in between: the operator suite at
+    7 rows, four eager calls, takes 59 us so and 78 with one."""
+    global _current_stream
+    if _current_stream is None:
+        import torch
+
+        torch.cuda.current_stream()      # brings CUDA up, or says why not
+        raw, device = torch._C._cuda_getCurrentRawStream, torch._C._cuda_getDevice
+        _current_stream = lambda: raw(device())  # noqa: E731
+    return _current_stream()
 
 
 def read_status() -> tuple[int, int, int, int]:
