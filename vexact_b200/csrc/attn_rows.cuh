@@ -76,14 +76,17 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t* r) {
 
 // Sum of 32 values in the butterfly order of a warp reduction (xor 16, 8, 4, 2, 1), done by one thread.
 __device__ __forceinline__ float butterfly_order_sum32(const float (&p)[32]) {
-  float a[16], b[8], c[4];
+  Two a[8];        // two neighbouring sums an instruction
 #pragma unroll
-  for (int i = 0; i < 16; ++i) a[i] = p[i] + p[i + 16];
+  for (int i = 0; i < 8; ++i) a[i] = Two(p[2 * i], p[2 * i + 1]) + Two(p[2 * i + 16], p[2 * i + 17]);
 #pragma unroll
-  for (int i = 0; i < 8; ++i) b[i] = a[i] + a[i + 8];
+  for (int w = 4; w > 0; w >>= 1)
 #pragma unroll
-  for (int i = 0; i < 4; ++i) c[i] = b[i] + b[i + 4];
-  return (c[0] + c[2]) + (c[1] + c[3]);
+    for (int i = 0; i < 4; ++i)
+      if (i < w) a[i] = a[i] + a[i + w];
+  float u, v;
+  a[0].get(u, v);
+  return u + v;
 }
 
 template <int DK, bool EXACT, int FORM>
@@ -435,9 +438,11 @@ paged_attn_rows_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_co
           ptx::tmem_ld_wait();
           const float shift = SIGMOID && !(p.extras.cap.cap > 0.f) ? bias : 0.f;
 #pragma unroll
-          for (int i = 0; i < 32; ++i) {
-            v[i] = SIGMOID ? fmaf(__uint_as_float(r0[i]), p.qk_scale, shift) : __uint_as_float(r0[i]) * p.qk_scale;
-            v[32 + i] = SIGMOID ? fmaf(__uint_as_float(r1[i]), p.qk_scale, shift) : __uint_as_float(r1[i]) * p.qk_scale;
+          for (int i = 0; i < 32; i += 2) {
+            const Two s0(__uint_as_float(r0[i]), __uint_as_float(r0[i + 1])), s1(__uint_as_float(r1[i]), __uint_as_float(r1[i + 1]));
+            const Two sc(p.qk_scale, p.qk_scale), sh(shift, shift);
+            (SIGMOID ? fma2(s0, sc, sh) : s0 * sc).get(v[i], v[i + 1]);
+            (SIGMOID ? fma2(s1, sc, sh) : s1 * sc).get(v[32 + i], v[32 + i + 1]);
           }
         }
         if constexpr (EXTRAS) {
@@ -505,9 +510,10 @@ paged_attn_rows_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_co
               ptx::tmem_ld16(o_addr + c * 32 + 16, r1);
               ptx::tmem_ld_wait();
 #pragma unroll
-              for (int i = 0; i < 16; ++i) {
-                o[c * 32 + i] = (o[c * 32 + i] + __uint_as_float(r0[i])) * alpha;
-                o[c * 32 + 16 + i] = (o[c * 32 + 16 + i] + __uint_as_float(r1[i])) * alpha;
+              for (int i = 0; i < 16; i += 2) {
+                float *a = o + c * 32 + i, *b = a + 16;
+                ((Two(a[0], a[1]) + Two(__uint_as_float(r0[i]), __uint_as_float(r0[i + 1]))) * Two(alpha, alpha)).get(a[0], a[1]);
+                ((Two(b[0], b[1]) + Two(__uint_as_float(r1[i]), __uint_as_float(r1[i + 1]))) * Two(alpha, alpha)).get(b[0], b[1]);
               }
             }
             ptx::tc_fence_before();
@@ -544,7 +550,9 @@ paged_attn_rows_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_co
           if constexpr (LSE) l_x = l_x * Two(alpha, alpha);
 #pragma unroll
           for (int i = 0; i < 32; i += 2) {
-            const float e0 = fast_exp2(v[i] - m_run), e1 = fast_exp2(v[i + 1] - m_run);
+            float e0, e1;
+            (Two(v[i], v[i + 1]) + Two(-m_run, -m_run)).get(e0, e1);
+            e0 = fast_exp2(e0), e1 = fast_exp2(e1);
             if constexpr (LSE) l_x = l_x + Two(e0, e1);
             const __nv_bfloat162 b2 = __floats2bfloat162_rn(e0, e1);
             pf[i] = __low2float(b2);
@@ -557,7 +565,9 @@ paged_attn_rows_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_co
             *reinterpret_cast<uint4*>(p_half + sw128(row, q)) = make_uint4(pk[q * 4], pk[q * 4 + 1], pk[q * 4 + 2], pk[q * 4 + 3]);
 #pragma unroll
           for (int i = 0; i < 32; i += 2) {
-            const float e0 = fast_exp2(v[32 + i] - m_run), e1 = fast_exp2(v[32 + i + 1] - m_run);
+            float e0, e1;
+            (Two(v[32 + i], v[32 + i + 1]) + Two(-m_run, -m_run)).get(e0, e1);
+            e0 = fast_exp2(e0), e1 = fast_exp2(e1);
             if constexpr (LSE) l_x = l_x + Two(e0, e1);
             const __nv_bfloat162 b2 = __floats2bfloat162_rn(e0, e1);
             pf[i] = __low2float(b2);
