@@ -529,6 +529,23 @@ def test_grouped_gemm_tile_heights_and_unfused_swiglu(vb, E, k, T, H, I):
     assert vb._lib.read_status()[0] == 0
 
 
+@pytest.mark.parametrize("width", [8192, 8191])
+def test_swiglu_rounds_every_bf16_gate_as_the_exact_form(width):
+    """silu(g) of all 65536 bf16 values, in 16-byte and in 2-byte accesses, has torch's bits (NaN stays NaN), down to the
+    values around -88 whose exponential is near the largest float and beyond, where it is infinite."""
+    from vexact_b200 import _lib
+
+    gate = torch.arange(65536, dtype=torch.int32).to(torch.int16).view(BF).cuda()
+    gate = torch.cat([gate, gate.new_zeros(-65536 % width)]).view(-1, width)
+    one, out = torch.ones_like(gate), torch.empty_like(gate)
+    _lib.check(_lib.load().b200_swiglu_scale(gate.data_ptr(), one.data_ptr(), None, out.data_ptr(), gate.shape[0], width,
+                                             _lib.current_stream()), "swiglu")
+    want = torch.nn.functional.silu(gate)
+    assert torch.equal(out.isnan(), want.isnan())
+    assert torch.equal(out.nan_to_num(0.0, float("inf"), -float("inf")).view(torch.int16),
+                       want.nan_to_num(0.0, float("inf"), -float("inf")).view(torch.int16))
+
+
 @pytest.mark.parametrize("M, N", [(8, 8), (128, 256), (136, 264), (200, 520), (768, 64)])
 def test_grouped_weight_gradient_edges(M, N):
     """Groups of every length around the 16 rows of an instruction and the 64 of a step, empty ones between them; a group's

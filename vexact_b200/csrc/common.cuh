@@ -81,18 +81,21 @@ __device__ __forceinline__ Two fma2(const Two& a, const Two& b, const Two& c) {
   return r;
 }
 
-// 1 / (1 + exp(-g)) on the special-function unit: 2^x and 1 / x with relative errors below 2^-22, far inside the bf16 rounding
-// that follows every use (the exact exponential and division took 45 of the 60 instructions per element of the SwiGLU kernels,
-// which they bound).  exp(-g) = inf gives 0.
-__device__ __forceinline__ float sigmoid_sfu(float g) {
+// silu(g) = g / (1 + exp(-g)) on the special-function unit.  The error grows with |g|, the rounding of g log2 e being one of
+// the exponent: a relative |g| 2^-24 and 2^-22 from the unit.  For bf16 gates, which is what every use has, the result rounded to
+// bf16 is that of the exact exponential and division for each of the 65536 values (tests/test_gpu_moe.py); the denominator is
+// scaled by 2^-24 where it may pass 2^126, whose reciprocal the unit flushes to zero.  (The exact forms took 45 of the 60
+// instructions per element of the SwiGLU kernels, which they bound.)
+__device__ __forceinline__ float silu_sfu(float g) {
+  const float s = g < 0.f ? 0x1p-24f : 1.f;
   float e, r;
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e) : "f"(g * -1.4426950408889634f));
-  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(1.f + e));
-  return r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(fmaf(e, s, s)));
+  return g * r * s;
 }
 // One element of the expert and dense SwiGLU with the rounding points of fused_moe.py:319-336: silu(g) and its product with u
-// are bf16 tensors.
-__device__ __forceinline__ float swiglu_reference(float g, float u) { return round_bf(round_bf(g * sigmoid_sfu(g)) * u); }
+// are bf16 tensors.  g holds a bf16 value.
+__device__ __forceinline__ float swiglu_reference(float g, float u) { return round_bf(round_bf(silu_sfu(g)) * u); }
 
 // Fixed butterfly reductions over a full warp.
 __device__ __forceinline__ float warp_sum(float v) {

@@ -850,7 +850,8 @@ swiglu_backward_kernel(const __nv_bfloat16* __restrict__ gate, const __nv_bfloat
       unpack_bf2(d4[j], d[0], d[1]);
 #pragma unroll
       for (int k = 0; k < 2; ++k) {
-        const float sig = sigmoid_sfu(g[k]), sg = round_bf(g[k] * sig), act = round_bf(sg * u[k]);
+        // (the derivative's sigmoid is not rounded before its products, so it is the exact one)
+        const float sig = 1.f / (1.f + expf(-g[k])), sg = round_bf(silu_sfu(g[k])), act = round_bf(sg * u[k]);
         const float da = round_bf(d[k] * s);
         sum += round_bf(act * d[k]);
         oh[k] = act * s;
