@@ -81,7 +81,7 @@ struct GemmParams {
   // tensor of the same shape (0: there is none).
   int k_second;
   int deep_w, deep_x;   // operand maps of whole stages (make_tmap_deep): one copy brings all K atoms of a stage
-  int split_boxes;   // activation boxes by the binary digits of a tile's height instead of p.xbox rows each
+  int split_boxes;   // CTA pairs: activation boxes by the binary digits of a tile's height instead of p.xbox rows each
   int xbox;       // rows per activation TMA box (multiple of 16)
   int xrows_max;  // largest token count of any tile (multiple of xbox, <= 256)
   int stages;
@@ -173,11 +173,11 @@ struct GemmTile {
 };
 
 // Activation maps of one launch.  box[0] serves tiles that are fetched in boxes of p.xbox rows.  Tall grouped tiles
-// (p.split_boxes) are fetched exactly, rounded up to 16 rows, as the binary digits of their height: box[i] is 256 >> i rows
-// high, so a tile of 144 rows is one box of 128 and one of 16.  Fewer copies per stage matter: at 256-row tiles, boxes of
-// 64 / 32 / 16 rows made fc1 of 4096 tokens (128 experts, 2048 -> 1536) 260 / 297 / 393 us.
+// (p.split_boxes, on CTA pairs) are fetched exactly, rounded up to 16 rows for either CTA, as the binary digits of that height:
+// box[i] is 128 >> i rows high, so a CTA's 80 rows are one box of 64 and one of 16.  (Before there were pairs, with 256-row tiles,
+// boxes of 64 / 32 / 16 rows made fc1 of 4096 tokens, 128 experts, 2048 -> 1536, 260 / 297 / 393 us: copies per stage matter.)
 struct GemmXMaps {
-  CUtensorMap box[5];
+  CUtensorMap box[4];
   CUtensorMap w2;      // p.k_second
 };
 
@@ -185,7 +185,7 @@ struct GemmXMaps {
 template <bool PAIR>
 __device__ __forceinline__ int gemm_tile_cols(const GemmParams& p, int n) {
   if (PAIR) return p.split_boxes ? (n + 31) & ~31 : 2 * p.xbox;   // half in either CTA, in whole steps of 16
-  return p.split_boxes ? (n + 15) & ~15 : (n + p.xbox - 1) / p.xbox * p.xbox;
+  return (n + p.xbox - 1) / p.xbox * p.xbox;
 }
 
 __device__ __forceinline__ bool gemm_tile(const GemmParams& p, int t_tiles, long long linear, GemmTile& t) {
@@ -445,14 +445,14 @@ gemm_ws_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__
           for (int a = 0; a < KA; ++a) {
             const uint32_t sx = stage + x_base + (uint32_t)a * x_atom;
             const int kcol = (kb * KA + a) * GEMM_BK;
-            if (p.split_boxes) {
+            if (PAIR && p.split_boxes) {
               int at = 0;
 #pragma unroll
-              for (int i = 0; i < 5; ++i)
-                if (own & (256 >> i)) {
+              for (int i = 0; i < 4; ++i)
+                if (own & (128 >> i)) {
                   load_2d(sx + (uint32_t)at * (GEMM_BK * 2), &tm_xs.box[i], s, kcol, row0 + at,
                                    ptx::kEvictLast);
-                  at += 256 >> i;
+                  at += 128 >> i;
                 }
             } else {
               for (int at = 0; at < own; at += p.xbox) {
@@ -1556,8 +1556,8 @@ inline int moe_grouped_gemm_impl(const void* x, long long x_rows, long long x_ro
   if (gather_index) {
     rc = make_tmap_2d(&tx.box[0], x, (uint64_t)x_rows, (uint64_t)K, (uint64_t)x_row_stride, 1u);
   } else if (p.split_boxes) {
-    for (int i = 0; i < 5 && !rc; ++i)
-      rc = make_tmap_2d(&tx.box[i], x, (uint64_t)x_rows, (uint64_t)K, (uint64_t)K, 256u >> i);
+    for (int i = 0; i < 4 && !rc; ++i)
+      rc = make_tmap_2d(&tx.box[i], x, (uint64_t)x_rows, (uint64_t)K, (uint64_t)K, 128u >> i);
   } else if (p.deep_w && p.xbox == p.xrows_max) {
     p.deep_x = 1;
     rc = make_tmap_deep(&tx.box[0], x, (uint64_t)x_rows, (uint64_t)K, (uint64_t)K, (uint32_t)p.xbox, ka);
