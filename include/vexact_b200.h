@@ -360,6 +360,12 @@ int b200_moe_grouped_gemm_noalloc(const void* x, const void* w, const void* row_
 int b200_moe_grouped_dgrad(const void* x, const void* w, const void* w2, void* out, const void* tile_table,
                            const void* tile_count, long long x_rows, int num_groups, int n_out, int K,
                            long long out_row_stride, int max_tiles, int tile_rows_max, void* stream);
+/* out = bf16(bf16(x . w) + bf16(x2 . w2)): the two products of a gated layer's data gradient with the rounding points of
+ * fused_moe.py:216-236; x and x2 rows x_row_stride apart, groups of w and w2 w_group_stride elements apart. */
+int b200_moe_grouped_dgrad_sum(const void* x, const void* x2, long long x_row_stride, const void* w, const void* w2,
+                               long long w_group_stride, void* out, const void* tile_table, const void* tile_count,
+                               long long x_rows, int num_groups, int n_out, int K, long long out_row_stride, int max_tiles,
+                               int tile_rows_max, void* stream);
 int b200_moe_grouped_dgrad_noalloc(const void* x, const void* w, void* out, const void* cu_seqlens, long long x_rows,
                                    int num_groups, int n_out, int K, long long out_row_stride, void* stream);
 

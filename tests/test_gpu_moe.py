@@ -462,6 +462,48 @@ def test_fused_moe_backward_against_autograd_of_the_fp32_formula(vb, fused_weigh
         assert not ours[n].grad[E - 1].any()
 
 
+@pytest.mark.parametrize("stacked", [False, True])
+@pytest.mark.parametrize("T, E, k, H, I", [(64, 16, 4, 512, 256), (150, 8, 2, 512, 200), (1100, 6, 2, 256, 128)])
+def test_fused_moe_backward_rounds_as_the_chain_of_operators(vb, T, E, k, H, I, stacked):
+    """The backward against the reference's chain (fused_moe.py:113-236) of single operators under its names and torch's
+    silu_backward: the same bits for every gradient, whatever the width (multiples of 64 or not) and the storage of fc1's
+    weights.  The routing weights' gradient is an fp32 sum of I bf16 values in another order, so one bf16 rounding apart."""
+    from vexact_b200 import group_gemm as gg
+
+    hidden, gate_up, down, sel, rw = (t.cuda() for t in _moe_case(T, E, k, H, I, seed=77))
+    gate_up, g_out = gate_up * 4, _seeded(T, H, seed=78).cuda()         # gates spread over the bend of silu
+    x, w3, wr = (t.clone().requires_grad_() for t in (hidden, down, rw))
+    if stacked:
+        leaves = [gate_up.clone().requires_grad_()]
+        out = vb.fused_moe_forward(E, wr, sel, x, fc2_weight=w3, fc1_1_2_weight=leaves[0])
+    else:
+        leaves = [gate_up[:, i * I:(i + 1) * I].clone().requires_grad_() for i in (0, 1)]
+        out = vb.fused_moe_forward(E, wr, sel, x, *leaves, w3)
+    got = torch.autograd.grad(out, [wr, x, w3, *leaves], g_out)
+
+    w1, w2 = gate_up[:, :I].contiguous(), gate_up[:, I:].contiguous()
+    cu, _, index = vb.fused_moe.build_moe_indices(sel, E)
+    ends, rows, at = cu[1:], T * k, index.flatten().long()
+
+    def product(a, w, forward):
+        return gg.group_gemm_same_nk(a, w, ends, rows, transpose_b=forward)
+
+    def weight(a, b, like):
+        return gg.group_gemm_same_mn(a, b, torch.empty_like(like), ends, rows, transpose_a=True, transpose_b=False)
+
+    xs, g_y = gg.moe_scatter(hidden, index), gg.moe_scatter(g_out, index)
+    gate, up = product(xs, w1, True), product(xs, w2, True)
+    act = torch.nn.functional.silu(gate) * up
+    row_w = torch.empty((rows, 1), dtype=BF, device="cuda")
+    row_w[at] = rw.reshape(-1, 1)
+    g_in = product(g_y, down, False)
+    g_act = g_in * row_w
+    g_up, g_gate = torch.nn.functional.silu(gate) * g_act, torch.ops.aten.silu_backward(g_act * up, gate)
+    g_xs = product(g_gate, w1, False) + product(g_up, w2, False)
+    torch.testing.assert_close(got[0], (act * g_in).sum(-1)[at].reshape(rw.shape), rtol=2 ** -7, atol=1e-6 * I)
+    assert torch.equal(got[1], gg.moe_gather(g_xs, index))
+    assert torch.equal(got[2], weight(g_y, act * row_w, down))
+    assert torch.equal(torch.cat(got[3:], 1), torch.cat([weight(g_gate, xs, w1), weight(g_up, xs, w2)], 1))
 
 
 def test_weight_gradient_kernels_tensor_core_and_cuda_core_forms(vb):

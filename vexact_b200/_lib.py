@@ -102,6 +102,7 @@ SIGNATURES = {
     "b200_gemm_swiglu": [P, P, P, LL, I, I, LL, LL, LL, P],
     "b200_seq_order": [P, P, I, P],
     "b200_moe_grouped_dgrad": [P, P, P, P, P, P, LL, I, I, I, LL, I, I, P],
+    "b200_moe_grouped_dgrad_sum": [P, P, LL, P, P, LL, P, P, P, LL, I, I, I, LL, I, I, P],
     "b200_moe_grouped_dgrad_noalloc": [P, P, P, P, LL, I, I, I, LL, P],
     "b200_swiglu_backward": [P, P, LL, P, P, P, P, P, LL, P, LL, I, P],
     "b200_moe_grouped_wgrad": [P, P, P, P, LL, I, I, I, P],

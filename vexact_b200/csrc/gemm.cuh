@@ -80,6 +80,7 @@ struct GemmParams {
   // MN-major through 3-D maps, two boxes of 64 k rows x 64 features per atom.  K steps from k_second on come from a second
   // tensor of the same shape (0: there is none).
   int k_second;
+  int two;           // the same mode: out = bf16(bf16(x . w) + bf16(x2 . w2)), k terms each
   int deep_w, deep_x;   // operand maps of whole stages (make_tmap_deep): one copy brings all K atoms of a stage
   int split_boxes;   // CTA pairs: activation boxes by the binary digits of a tile's height instead of p.xbox rows each
   int xbox;       // rows per activation TMA box (multiple of 16)
@@ -178,7 +179,8 @@ struct GemmTile {
 // boxes of 64 / 32 / 16 rows made fc1 of 4096 tokens, 128 experts, 2048 -> 1536, 260 / 297 / 393 us: copies per stage matter.)
 struct GemmXMaps {
   CUtensorMap box[4];
-  CUtensorMap w2;      // p.k_second
+  CUtensorMap w2;      // p.k_second, p.two
+  CUtensorMap x2[4];   // p.two: as box
 };
 
 // Token columns that a tile of n rows occupies in shared and tensor memory.
@@ -230,6 +232,14 @@ gemm_ws_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__
     if (!gemm_tile(p, t_tiles, lin, t)) return false;
     if (PAIR) t.wt = 2 * t.wt + rank;
     return true;
+  };
+  auto next_product = [&](long long& lin, int& half) {      // p.two: a tile's second product follows its first
+    if (W_MN && p.two && half == 0) {
+      half = 1;
+    } else {
+      half = 0;
+      lin += lin_step;
+    }
   };
   const CUtensorMap& tm_x = tm_xs.box[0];
   extern __shared__ uint8_t smem_raw[];
@@ -306,7 +316,7 @@ gemm_ws_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__
     else ptx::tma_load_4d(at, &tm_w, full_bar(s), 0, wrow, 0, z, p.w_policy);
   };
   // The weights of K step kb into the stage at `at` (slot s): by one copy, or atom by atom.
-  auto weights = [&](uint32_t at, int s, int kb, const GemmTile& t, int wrow) {
+  auto weights = [&](uint32_t at, int s, int kb, const GemmTile& t, int wrow, int half) {
     if (!W_MN && p.deep_w) {
       weights_deep(at, s, wrow, kb * KA);
       return;
@@ -315,11 +325,11 @@ gemm_ws_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__
       const uint32_t sw = at + (uint32_t)a * GEMM_WBYTES;
       const int kcol = (kb * KA + a) * GEMM_BK;
       if (W_MN) {
-        const bool second = p.k_second && kcol >= p.k_second;
+        const bool behind = p.k_second && kcol >= p.k_second, second = behind || half != 0;
 #pragma unroll
         for (int h = 0; h < 2; ++h)
           load_3d(sw + h * (GEMM_WBYTES / 2), second ? &tm_xs.w2 : &tm_w, s, t.wt * GEMM_WTILE + h * 64,
-                  second ? kcol - p.k_second : kcol, t.group, p.w_policy);
+                  behind ? kcol - p.k_second : kcol, t.group, p.w_policy);
       } else {
         load_2d(sw, &tm_w, s, kcol, wrow, p.w_policy);
         if (SWIGLU) load_2d(sw + 64 * GEMM_BK * 2, &tm_w, s, kcol, wrow + p.up_offset, p.w_policy);
@@ -340,7 +350,7 @@ gemm_ws_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__
         const int wrow = t.group * p.w_rows_per_group + t.wt * (SWIGLU ? 64 : GEMM_WTILE);
         for (int kb = 0; kb < prefetched; ++kb) {
           arm(kb, tx * KA);
-          weights(stage_base + (uint32_t)kb * stage_bytes, kb, kb, t, wrow);
+          weights(stage_base + (uint32_t)kb * stage_bytes, kb, kb, t, wrow, 0);
         }
       }
     }
@@ -406,7 +416,8 @@ gemm_ws_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__
       int s = 0;         // ring slot of `it`
       uint32_t ph = 0;   // parity of the slot's current use
       bool ok = true;
-      for (long long lin = lin0; ok; lin += lin_step) {
+      int half = 0;
+      for (long long lin = lin0; ok; next_product(lin, half)) {
         GemmTile t;
         if (!tile_at(t_tiles, lin, t)) break;
         const int cols = gemm_tile_cols<PAIR>(p, t.n);
@@ -441,7 +452,8 @@ gemm_ws_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__
             arm(s, tx * KA);
           }
           const uint32_t stage = stage_base + (uint32_t)s * stage_bytes;
-          if (!early) weights(stage, s, kb, t, wrow);
+          if (!early) weights(stage, s, kb, t, wrow, half);
+          const CUtensorMap* xmaps = W_MN && half ? tm_xs.x2 : tm_xs.box;
           for (int a = 0; a < KA; ++a) {
             const uint32_t sx = stage + x_base + (uint32_t)a * x_atom;
             const int kcol = (kb * KA + a) * GEMM_BK;
@@ -450,7 +462,7 @@ gemm_ws_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__
 #pragma unroll
               for (int i = 0; i < 4; ++i)
                 if (own & (128 >> i)) {
-                  load_2d(sx + (uint32_t)at * (GEMM_BK * 2), &tm_xs.box[i], s, kcol, row0 + at,
+                  load_2d(sx + (uint32_t)at * (GEMM_BK * 2), xmaps + i, s, kcol, row0 + at,
                                    ptx::kEvictLast);
                   at += 128 >> i;
                 }
@@ -460,7 +472,7 @@ gemm_ws_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__
                   load_3d(sx + (uint32_t)at * (GEMM_BK * 2), &tm_x, s, kcol, row0 + at, t.group,
                                    ptx::kEvictLast);
                 else
-                  load_2d(sx + (uint32_t)at * (GEMM_BK * 2), &tm_x, s, kcol, row0 + at,
+                  load_2d(sx + (uint32_t)at * (GEMM_BK * 2), xmaps, s, kcol, row0 + at,
                                    ptx::kEvictLast);
               }
             }
@@ -478,7 +490,8 @@ gemm_ws_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__
       uint32_t it = 0, tile_it = 0, ph = 0;
       int s = 0;
       bool ok = true;
-      for (long long lin = lin0; ok; lin += lin_step, ++tile_it) {
+      int half = 0;
+      for (long long lin = lin0; ok; next_product(lin, half), ++tile_it) {
         GemmTile t;
         if (!tile_at(t_tiles, lin, t)) break;
         const int buf = tile_it & 1;
@@ -526,7 +539,10 @@ gemm_ws_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__
     const int q = warp & 3;              // tensor-memory lane quadrant this warp may read
     const int eh = (warp - 2) >> 2;      // first or second half of the token columns
     uint32_t tile_it = 0;
-    for (long long lin = lin0; !HEAD || eh == 0; lin += lin_step, ++tile_it) {
+    // p.two: the first product of this thread's columns, rounded, until the second is there (gemm_exch_bytes)
+    uint4* held = reinterpret_cast<uint4*>(exch + 8 * 16 * 32) + (threadIdx.x - 64);
+    int half = 0;
+    for (long long lin = lin0; !HEAD || eh == 0; next_product(lin, half), ++tile_it) {
       GemmTile t;
       if (!tile_at(t_tiles, lin, t)) break;
       const int buf = tile_it & 1;
@@ -644,6 +660,18 @@ gemm_ws_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__
         auto finish = [&](const uint32_t (&r)[16], float (&v)[16], int c0) {
 #pragma unroll
           for (int j = 0; j < 16; ++j) v[j] = __uint_as_float(r[j]) + bias;
+          if (W_MN && half) {      // (half is 1 for p.two alone)
+            const uint4* h = held + (c0 - ca) / 8 * 256;
+            const uint4 h0 = h[0], h1 = h[256];
+            const uint32_t hv[8] = {h0.x, h0.y, h0.z, h0.w, h1.x, h1.y, h1.z, h1.w};
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+              float a, b;
+              unpack_bf2(hv[j], a, b);
+              v[2 * j] = a + round_bf(v[2 * j]);
+              v[2 * j + 1] = b + round_bf(v[2 * j + 1]);
+            }
+          }
           if (act == GEMM_ACT_GELU_TANH) {
 #pragma unroll
             for (int j = 0; j < 16; ++j) v[j] = gelu_tanh_fast(v[j]);
@@ -667,7 +695,19 @@ gemm_ws_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__
         // instruction covers eight token rows, instead of one 2-byte store per (feature, token).
         const bool vec_out = !p.scalar_epilogue && !p.out_f32 && (p.ldo & 7) == 0 && (p.n_w & 7) == 0 &&
                              (p.out_batch_stride & 7) == 0 && (reinterpret_cast<uintptr_t>(p.out) & 15) == 0;
-        if (vec_out) {
+        if (W_MN && p.two && half == 0) {
+          for (int c0 = ca; c0 < cb; c0 += 16) {
+            uint32_t r[16];
+            ptx::tmem_ld16(taddr + c0, r);
+            ptx::tmem_ld_wait();
+            uint32_t h[8];
+#pragma unroll
+            for (int j = 0; j < 8; ++j) h[j] = pack_bf2(__uint_as_float(r[2 * j]), __uint_as_float(r[2 * j + 1]));
+            uint4* d = held + (c0 - ca) / 8 * 256;
+            d[0] = make_uint4(h[0], h[1], h[2], h[3]);
+            d[256] = make_uint4(h[4], h[5], h[6], h[7]);
+          }
+        } else if (vec_out) {
           __nv_bfloat16* stg = exch + (warp - 2) * (16 * 32);      // [16 tokens][32 features] per warp
           const int part = lane & 3, rsub = lane >> 2;
           const int f8 = t.wt * GEMM_WTILE + q * 32 + part * 8;
@@ -900,8 +940,8 @@ inline int env_int(const char* name, int dflt) {
 }
 
 // Epilogue scratch after the stages: the SwiGLU exchange buffer, the head mode's per-warp partials, or the turning tiles.
-inline int gemm_exch_bytes(int mode, int xrows_max) {
-  const int turn = 8 * 16 * 32 * 2;
+inline int gemm_exch_bytes(int mode, int xrows_max, bool two = false) {
+  const int turn = 8 * 16 * 32 * 2 + (two ? 256 * 2 * round_up(xrows_max / 2, 16) : 0);   // and the rounded first products
   return mode == GEMM_SWIGLU ? 64 * (xrows_max + GEMM_EXCH_PAD) * 2 + turn : mode == GEMM_HEAD ? 3 * 4 * xrows_max * 4 : turn;
 }
 // K atoms per stage: fewer, larger stages cut the per-stage barrier round trips; keep >= 3 stages.  (One token, 6144 -> 2048, at
@@ -922,7 +962,7 @@ inline int gemm_launch(const CUtensorMap& tw, const GemmXMaps& tx, GemmParams& p
   static PerDeviceFlags attr_set;
   if (int rc = set_max_dyn_smem_once(attr_set, gemm_ws_kernel<MODE, PAIR>, GEMM_SMEM_BUDGET)) return rc;
   const int atom_bytes = GEMM_WBYTES + p.xrows_max / (PAIR ? 2 : 1) * GEMM_BK * 2;
-  const int exch_bytes_pre = gemm_exch_bytes(MODE, p.xrows_max);
+  const int exch_bytes_pre = gemm_exch_bytes(MODE, p.xrows_max, p.two);
   const int ka = p.katoms = gemm_katoms(p.k, atom_bytes, exch_bytes_pre);
   static const int epi_scalar = env_int("B200_GEMM_EPI_SCALAR", 0);
   p.scalar_epilogue = epi_scalar;
@@ -1486,14 +1526,17 @@ extern "C" int b200_lm_head_greedy(const void* x, const void* w, void* partials,
 //   mode 1: out[r, i] = silu(x . w[g, i, :]) * (x . w[g, I + i, :]) * row_scale[r]   (w: [G, 2I, K], n_out = I)
 // tile_table / tile_count come from b200_moe_permute: every tile lies inside one group.
 namespace b200 {
-// gather_index == nullptr: x holds the expert-sorted rows ([x_rows, K], contiguous).  Otherwise x is the
-// unpermuted [x_rows, K] matrix with rows x_row_stride apart and sorted row r is x[gather_index[r]].
+// gather_index == nullptr: x holds the expert-sorted rows, x_row_stride apart.  Otherwise x is the unpermuted
+// [x_rows, K] matrix with rows x_row_stride apart and sorted row r is x[gather_index[r]].
+// w_group_stride and x2: data gradient, elements from a group's weights to the next's, and the rows that w2 multiplies
+// (GemmParams::two; null with a w2: GemmParams::k_second).
 inline int moe_grouped_gemm_impl(const void* x, long long x_rows, long long x_row_stride, const void* gather_index,
                                  const void* w, const void* row_scale, void* out, const void* tile_table,
                                  const void* tile_count, int num_groups, int n_out, int K, long long out_row_stride,
                                  int max_tiles, int tile_rows_max, int mode, void* stream, int glu = GLU_REFERENCE,
                                  const void* scale_in = nullptr, const void* scale_out = nullptr,
-                                 int act = GEMM_ACT_NONE, bool w_mn = false, const void* w2 = nullptr) {
+                                 int act = GEMM_ACT_NONE, bool w_mn = false, const void* w2 = nullptr, long long w_group_stride = 0,
+                                 const void* x2 = nullptr) {
   if (!x || !w || !out || !tile_table || !tile_count || x_rows < 0 || num_groups <= 0 || n_out <= 0 || K <= 0 ||
       max_tiles < 0 || (mode != 0 && mode != 1))
     return B200_ERR_ARG;
@@ -1522,6 +1565,7 @@ inline int moe_grouped_gemm_impl(const void* x, long long x_rows, long long x_ro
   if (p.split_boxes) p.w_tiles = (p.w_tiles + 1) / 2;   // of a CTA pair
   p.xrows_max = tile_rows_max;
   p.out = out;
+  p.two = x2 != nullptr;
   p.ldo = out_row_stride;
   p.out_f32 = 0;
   p.bias = nullptr;
@@ -1538,12 +1582,13 @@ inline int moe_grouped_gemm_impl(const void* x, long long x_rows, long long x_ro
                              gemm_exch_bytes(mode == 1 ? GEMM_SWIGLU : GEMM_PLAIN, p.xrows_max));
   if (w_mn) {
     // [groups, k, features]: rows past a group's k and columns past its features read as zero
-    if (mode != 0 || gather_index || n_out % 8 != 0 || (w2 && K % (2 * GEMM_BK) != 0)) return B200_ERR_SHAPE;
-    const int k_one = w2 ? K / 2 : K;
-    p.k_second = w2 ? k_one : 0;
-    rc = make_tmap_3d(&tw, w, (uint64_t)num_groups, (uint64_t)k_one, (uint64_t)n_out, (uint64_t)k_one * n_out, (uint64_t)n_out, GEMM_BK);
+    if (mode != 0 || gather_index || n_out % 8 != 0 || (w2 && !x2 && K % (2 * GEMM_BK) != 0)) return B200_ERR_SHAPE;
+    const int k_one = w2 && !x2 ? K / 2 : K;
+    const uint64_t w_group = w_group_stride ? (uint64_t)w_group_stride : (uint64_t)k_one * n_out;
+    p.k_second = w2 && !x2 ? k_one : 0;
+    rc = make_tmap_3d(&tw, w, (uint64_t)num_groups, (uint64_t)k_one, (uint64_t)n_out, w_group, (uint64_t)n_out, GEMM_BK);
     if (!rc && w2)
-      rc = make_tmap_3d(&tx.w2, w2, (uint64_t)num_groups, (uint64_t)k_one, (uint64_t)n_out, (uint64_t)k_one * n_out, (uint64_t)n_out, GEMM_BK);
+      rc = make_tmap_3d(&tx.w2, w2, (uint64_t)num_groups, (uint64_t)k_one, (uint64_t)n_out, w_group, (uint64_t)n_out, GEMM_BK);
   } else if (K % GEMM_BK == 0 && !gather_index) {
     p.deep_w = 1;
     const uint64_t w_rows = (uint64_t)num_groups * p.w_rows_per_group;
@@ -1556,13 +1601,16 @@ inline int moe_grouped_gemm_impl(const void* x, long long x_rows, long long x_ro
   if (gather_index) {
     rc = make_tmap_2d(&tx.box[0], x, (uint64_t)x_rows, (uint64_t)K, (uint64_t)x_row_stride, 1u);
   } else if (p.split_boxes) {
-    for (int i = 0; i < 4 && !rc; ++i)
-      rc = make_tmap_2d(&tx.box[i], x, (uint64_t)x_rows, (uint64_t)K, (uint64_t)K, 128u >> i);
+    for (int i = 0; i < 8 && !rc; ++i)
+      if (i < 4 || x2)
+        rc = make_tmap_2d(i < 4 ? &tx.box[i] : &tx.x2[i - 4], i < 4 ? x : x2, (uint64_t)x_rows, (uint64_t)K, (uint64_t)x_row_stride,
+                          128u >> (i & 3));
   } else if (p.deep_w && p.xbox == p.xrows_max) {
     p.deep_x = 1;
-    rc = make_tmap_deep(&tx.box[0], x, (uint64_t)x_rows, (uint64_t)K, (uint64_t)K, (uint32_t)p.xbox, ka);
+    rc = make_tmap_deep(&tx.box[0], x, (uint64_t)x_rows, (uint64_t)K, (uint64_t)x_row_stride, (uint32_t)p.xbox, ka);
   } else {
-    rc = make_tmap_2d(&tx.box[0], x, (uint64_t)x_rows, (uint64_t)K, (uint64_t)K, (uint32_t)p.xbox);
+    rc = make_tmap_2d(&tx.box[0], x, (uint64_t)x_rows, (uint64_t)K, (uint64_t)x_row_stride, (uint32_t)p.xbox);
+    if (!rc && x2) rc = make_tmap_2d(&tx.x2[0], x2, (uint64_t)x_rows, (uint64_t)K, (uint64_t)x_row_stride, (uint32_t)p.xbox);
   }
   if (rc) return rc;
   const long long tiles = (long long)max_tiles * p.w_tiles;
@@ -1594,6 +1642,21 @@ extern "C" int b200_moe_grouped_dgrad(const void* x, const void* w, const void* 
   return b200::moe_grouped_gemm_impl(x, x_rows, K, nullptr, w, nullptr, out, tile_table, tile_count, num_groups, n_out, K,
                                      out_row_stride, max_tiles, tile_rows_max, 0, stream, b200::GLU_REFERENCE, nullptr, nullptr,
                                      b200::GEMM_ACT_NONE, true, w2);
+}
+
+// The data gradient through two weights, as a chain of two calls and an addition rounds it: out = bf16(bf16(x . w) +
+// bf16(x2 . w2)), x and x2 with rows x_row_stride apart, w and w2 [num_groups, K, n_out] with groups w_group_stride apart (the
+// halves of stacked weights lie so).  One launch: a tile's first product waits, rounded, in shared memory (64 KB of the ring at 256
+// columns) for the second.  32768 rows of 2 x 768 to 2048 in 128 groups: 268 us; two launches, the second adding to what the first
+// left, 380; one accumulation of 1536 terms, which rounds otherwise, 235.
+extern "C" int b200_moe_grouped_dgrad_sum(const void* x, const void* x2, long long x_row_stride, const void* w, const void* w2,
+                                          long long w_group_stride, void* out, const void* tile_table, const void* tile_count,
+                                          long long x_rows, int num_groups, int n_out, int K, long long out_row_stride,
+                                          int max_tiles, int tile_rows_max, void* stream) {
+  if (!x2 || !w2 || w_group_stride < (long long)K * n_out || x_row_stride < K) return B200_ERR_ARG;
+  return b200::moe_grouped_gemm_impl(x, x_rows, x_row_stride, nullptr, w, nullptr, out, tile_table, tile_count, num_groups, n_out, K,
+                                     out_row_stride, max_tiles, tile_rows_max, 0, stream, b200::GLU_REFERENCE, nullptr, nullptr,
+                                     b200::GEMM_ACT_NONE, true, w2, w_group_stride, x2);
 }
 
 // The same GEMM reading its activation rows where they lie: x is the unpermuted [T, K] matrix and sorted row r
