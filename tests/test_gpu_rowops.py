@@ -286,6 +286,19 @@ def test_gather_logprob_backward_matches_autograd(vb, dtype):
 
 
 @pytest.mark.parametrize("dtype", [torch.float32, BF])
+def test_gather_logprob_backward_keeps_probabilities_below_the_normal_range(vb, dtype):
+    """Probabilities from 1 down to 2^-149, the smallest fp32 number, against fp64: none is cut off at 2^-126."""
+    x = torch.linspace(0.0, -103.0, 4099).to(dtype)[None].cuda()
+    leaf = x.clone().requires_grad_(True)
+    vb.logprobs_from_logits_flash_attn(leaf, torch.zeros(1, dtype=torch.int64, device="cuda")).sum().backward()
+    got, p = leaf.grad[0, 1:].double(), torch.softmax(x.double(), -1)[0, 1:]
+    # the fp32 difference x - lse (below 128: 2^-18 and lse's own 2^-21 as a relative error of the exponential), the exponential,
+    # the output's rounding, and two subnormal steps (of 2^-149, or 2^-133 in bf16)
+    rel, step = (2 ** -17, 2.0 ** -149) if dtype == torch.float32 else (2 ** -8, 2.0 ** -133)
+    assert ((got + p).abs() <= rel * p + 2 * step).all()
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, BF])
 @pytest.mark.parametrize("vocab", [5, 1000, 8192, 8195, 40008])
 def test_row_softmax_in_a_cluster_and_in_one_cta(vb, dtype, vocab):
     """Up to 64 rows are spread over eight CTAs each, more rows take one CTA each: the same bits either way, against fp64;

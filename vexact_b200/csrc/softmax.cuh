@@ -36,8 +36,10 @@ __device__ __forceinline__ MaxSum ms_merge(MaxSum a, MaxSum b) {
 
 // exp of two values that are at most 0 (-inf gives 0, NaN stays): 2^h (1 + l ln 2) with h + l = t log2(e), the product
 // carried in two floats (the exact remainder of h by fma, and log2(e) itself in two parts), 2^h on the special-function
-// unit.  Results below the normal range are 0.  The walk over 2000 x 151936 bf16 logits is bound by issue slots, not by HBM,
+// unit.  TINY: results below the normal range are subnormal, as the exact exponential's, and not 0; a term of a sum whose largest
+// is 1 does not need that.  The walk over 2000 x 151936 bf16 logits is bound by issue slots, not by HBM,
 // and the exact exponential took most of them: 214 us with it, 164 so.
+template <bool TINY = false>
 __device__ __forceinline__ Two exp_nonpos(const Two& t_in) {
   float a, b;
   t_in.get(a, b);
@@ -47,8 +49,13 @@ __device__ __forceinline__ Two exp_nonpos(const Two& t_in) {
   const Two t(a, b), h = t * Two(L, L);
   const Two neg_l = fma2(t, Two(-L_LO, -L_LO), fma2(t, Two(-L, -L), h));
   h.get(a, b);
-  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(a) : "f"(a));
-  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(b) : "f"(b));
+  if constexpr (TINY) {
+    asm("ex2.approx.f32 %0, %1;" : "=f"(a) : "f"(a));
+    asm("ex2.approx.f32 %0, %1;" : "=f"(b) : "f"(b));
+  } else {
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(a) : "f"(a));
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(b) : "f"(b));
+  }
   const Two e(a, b);
   return fma2(e, neg_l * Two(-LN2, -LN2), e);
 }
@@ -327,7 +334,7 @@ gather_logprob_backward_kernel(const T* x, const long long* __restrict__ labels,
   const Two neg_lse(-lse, -lse);
   auto grad = [&](float& u, float& v, int i) {   // elements i and i + 1
     float a, b;
-    exp_nonpos(Two(u, v) + neg_lse).get(a, b);
+    exp_nonpos<true>(Two(u, v) + neg_lse).get(a, b);
     u = live ? g * ((i == lab ? 1.f : 0.f) - a) : 0.f;
     v = live ? g * ((i + 1 == lab ? 1.f : 0.f) - b) : 0.f;
   };
