@@ -571,6 +571,52 @@ def test_grouped_gemm_tile_heights_and_unfused_swiglu(vb, E, k, T, H, I):
     assert vb._lib.read_status()[0] == 0
 
 
+@pytest.mark.parametrize("K", [192, 200])
+@pytest.mark.parametrize("height", [16, 48, 80, 96, 112, 144, 176, 208, 240, 256])
+def test_grouped_products_at_every_tile_height(vb, height, K):
+    """Every multiple of 16 up to 256 is a tile height, also those above 64 that are no multiple of the 32 columns in which CTA
+    pairs take tiles: the bits of 64-row tiles, for the plain, gated, squared and data-gradient products, with full tiles
+    and more of them than the pairs of the chip.  The sum of two data gradients is that of the rounded two."""
+    from vexact_b200 import _lib, fused_moe as fm
+
+    E, N, cu = 3, 2048, [0, 700, 1411, 2111]
+    gen = torch.Generator(device="cuda").manual_seed(height + K)
+    R = cu[-1]
+    x = torch.randn(R, K, device="cuda", generator=gen).to(BF)
+    w = (torch.randn(E, N, K, device="cuda", generator=gen) * 0.1).to(BF)
+    wt, x2 = w.transpose(1, 2).contiguous(), torch.randn(R, K, device="cuda", generator=gen).to(BF)
+    wt2 = (torch.randn(E, K, N, device="cuda", generator=gen) * 0.1).to(BF)
+    scale = torch.rand(R, device="cuda", generator=gen).to(BF)
+
+    def products(plan):
+        common = plan["tile_table"].data_ptr(), plan["tile_count"].data_ptr()
+        act, back, other, both = (torch.empty(R, N, dtype=BF, device="cuda") for _ in range(4))
+        _lib.check(_lib.load().b200_moe_grouped_gemm_act(
+            x.data_ptr(), w.data_ptr(), None, act.data_ptr(), *common, R, E, N, K, N, plan["max_tiles"], plan["tile_rows"], 3,
+            _lib.current_stream()), "act")
+        for rows, weights, out in ((x, wt, back), (x2, wt2, other)):
+            _lib.check(_lib.load().b200_moe_grouped_dgrad(
+                rows.data_ptr(), weights.data_ptr(), None, out.data_ptr(), *common, R, E, N, K, N, plan["max_tiles"],
+                plan["tile_rows"], _lib.current_stream()), "dgrad")
+        pair, stacked = torch.cat([x, x2], 1), torch.cat([wt, wt2], 1)      # both halves as they lie in one tensor
+        _lib.check(_lib.load().b200_moe_grouped_dgrad_sum(
+            pair.data_ptr(), pair[:, K:].data_ptr(), 2 * K, stacked.data_ptr(), stacked[:, K:].data_ptr(), 2 * K * N, both.data_ptr(),
+            *common, R, E, N, K, N, plan["max_tiles"], plan["tile_rows"], _lib.current_stream()), "dgrad_sum")
+        assert torch.equal(both, back + other)
+        return (fm._grouped_gemm(x, w, None, plan, N, mode=0), fm._grouped_gemm(x, w, scale, plan, N // 2, mode=1), act, back)
+
+    for got, want in zip(products(_tile_table(cu, height)), products(_tile_table(cu, 64))):
+        assert torch.equal(got, want)
+    torch.cuda.synchronize()
+    assert vb._lib.read_status()[0] == 0
+
+
+def _tile_table(cu, height):
+    rows = [(e, r, min(height, cu[e + 1] - r), 0) for e in range(len(cu) - 1) for r in range(cu[e], cu[e + 1], height)]
+    return dict(tile_table=torch.tensor(rows, dtype=torch.int32, device="cuda"), max_tiles=len(rows), tile_rows=height,
+                tile_count=torch.tensor([len(rows)], dtype=torch.int32, device="cuda"))
+
+
 @pytest.mark.parametrize("width", [8192, 8191])
 def test_swiglu_rounds_every_bf16_gate_as_the_exact_form(width):
     """silu(g) of all 65536 bf16 values, in 16-byte and in 2-byte accesses, has torch's bits (NaN stays NaN), down to the

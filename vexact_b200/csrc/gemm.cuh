@@ -1563,7 +1563,8 @@ inline int moe_grouped_gemm_impl(const void* x, long long x_rows, long long x_ro
   p.tokens_first = 0;
   p.split_boxes = tile_rows_max > 64 && !gather_index;
   if (p.split_boxes) p.w_tiles = (p.w_tiles + 1) / 2;   // of a CTA pair
-  p.xrows_max = tile_rows_max;
+  // a pair's tile takes whole steps of 32 token columns (gemm_tile_cols), so its slots are that wide
+  p.xrows_max = p.split_boxes ? round_up(tile_rows_max, 32) : tile_rows_max;
   p.out = out;
   p.two = x2 != nullptr;
   p.ldo = out_row_stride;
