@@ -611,10 +611,78 @@ def test_grouped_products_at_every_tile_height(vb, height, K):
     assert vb._lib.read_status()[0] == 0
 
 
-def _tile_table(cu, height):
-    rows = [(e, r, min(height, cu[e + 1] - r), 0) for e in range(len(cu) - 1) for r in range(cu[e], cu[e + 1], height)]
-    return dict(tile_table=torch.tensor(rows, dtype=torch.int32, device="cuda"), max_tiles=len(rows), tile_rows=height,
-                tile_count=torch.tensor([len(rows)], dtype=torch.int32, device="cuda"))
+@pytest.mark.parametrize("tile_rows", [1, 7, 16, 24, 40, 64, 100, 200, 256])
+def test_tile_tables_cover_the_rows_at_any_height(vb, tile_rows):
+    """A token tile has at least one row and at most tile_rows, whatever tile_rows is, and an expert's tiles cover its rows in
+    order, as few as they can be."""
+    from vexact_b200 import _lib
+
+    counts = [0, 1, 15, 16, 17, 201, 40, 333, 0, 64, 640]
+    E, n = len(counts), sum(counts)
+    sel = torch.repeat_interleave(torch.arange(E), torch.tensor(counts))
+    sel = sel[torch.randperm(n, generator=torch.Generator().manual_seed(tile_rows))].cuda()
+    max_tiles = sum(-(-c // tile_rows) for c in counts)
+    index, cu, table, count, gather = (torch.zeros(s, dtype=torch.int32, device="cuda") for s in (n, E + 1, (max_tiles, 4), 1, n))
+    _lib.check(_lib.load().b200_moe_permute_index(
+        sel.data_ptr(), 1, None, index.data_ptr(), cu.data_ptr(), gather.data_ptr(), None, table.data_ptr(), count.data_ptr(), n, 1,
+        E, tile_rows, max_tiles, _lib.current_stream()), "permute")
+    _check_tiles(table[:int(count)].tolist(), counts, tile_rows)
+    T = 150
+    logits = torch.randn(T, E, generator=torch.Generator().manual_seed(5)).cuda()
+    logits[:, 3] += 3.0
+    weights, rank = torch.empty(T, 2, dtype=BF, device="cuda"), torch.empty(2 * T, dtype=torch.int32, device="cuda")
+    chosen = torch.empty(T, 2, dtype=torch.int64, device="cuda")
+    counters = torch.zeros(1024, dtype=torch.int32, device="cuda")
+    table = torch.zeros(2 * T + E, 4, dtype=torch.int32, device="cuda")
+    _lib.check(_lib.load().b200_moe_route_plan_softmax_topk(
+        logits.data_ptr(), 0, E, weights.data_ptr(), chosen.data_ptr(), rank.data_ptr(), counters.data_ptr(), cu.data_ptr(),
+        table.data_ptr(), count.data_ptr(), T, E, 2, 1, tile_rows, len(table), _lib.current_stream()), "plan")
+    _check_tiles(table[:int(count)].tolist(), torch.bincount(chosen.flatten(), minlength=E).tolist(), tile_rows)
+
+
+def _check_tiles(table, counts, tile_rows):
+    at, start = 0, 0
+    for e, c in enumerate(counts):
+        mine, end = table[at:at - (-c // tile_rows)], start + c
+        at += len(mine)
+        for group, first, rows, _ in mine:
+            assert (group, first) == (e, start) and 0 < rows <= tile_rows
+            start += rows
+        assert start == end
+    assert at == len(table)
+
+
+@pytest.mark.parametrize("M, N", [(8, 8), (136, 264), (200, 520)])
+def test_weight_gradient_has_the_same_bits_wherever_it_is_written(vb, M, N):
+    """c on 16, 8 and 4 bytes: the tensor-core kernel serves all three."""
+    from vexact_b200 import _lib
+
+    lens = [5, 0, 64, 100]
+    cu = torch.tensor([0, *torch.tensor(lens).cumsum(0)], dtype=torch.int32, device="cuda")
+    gen = torch.Generator(device="cuda").manual_seed(M)
+    a, b = (torch.randn(sum(lens), n, device="cuda", generator=gen).to(BF) for n in (M, N))
+    size, got = len(lens) * M * N, []
+    for at in (8, 12, 10):
+        store = torch.full((size + 24,), 7.0, dtype=BF, device="cuda")
+        _lib.check(_lib.load().b200_moe_grouped_wgrad(a.data_ptr(), b.data_ptr(), store.data_ptr() + 2 * at, cu.data_ptr(),
+                                                      sum(lens), len(lens), M, N, _lib.current_stream()), "wgrad")
+        assert (store[:at] == 7).all() and (store[at + size:] == 7).all()
+        got.append(store[at:at + size])
+    assert torch.equal(got[0], got[1]) and torch.equal(got[0], got[2])
+    refused = torch.empty(size + 8, dtype=BF, device="cuda")      # 2 bytes: neither kernel's accesses fit
+    assert _lib.load().b200_moe_grouped_wgrad(a.data_ptr(), b.data_ptr(), refused.data_ptr() + 2, cu.data_ptr(), sum(lens),
+                                              len(lens), M, N, _lib.current_stream()) == -2
+
+
+@pytest.mark.parametrize("G, R, C", [(1, 8, 8), (3, 64, 72), (2, 200, 136)])
+def test_transpose_of_the_last_two_dimensions(vb, G, R, C):
+    """`b200_transpose_last2`, whole and partial 64 x 64 tiles."""
+    from vexact_b200 import _lib
+
+    x = torch.randint(-32768, 32767, (G, R, C), dtype=torch.int16, device="cuda")
+    out = torch.empty(G, C, R, dtype=torch.int16, device="cuda")
+    _lib.check(_lib.load().b200_transpose_last2(x.data_ptr(), out.data_ptr(), G, R, C, _lib.current_stream()), "transpose")
+    assert torch.equal(out, x.transpose(1, 2))
 
 
 @pytest.mark.parametrize("width", [8192, 8191])

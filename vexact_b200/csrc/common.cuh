@@ -251,10 +251,11 @@ inline int sm_count() {
 inline int grouped_tile_rows(long long rows, long long groups) {
   return rows <= 64 * groups ? 64 : rows <= 112 * groups ? 128 : 256;
 }
-// Tile j of a group's `tiles`: {group, first row, rows, 0}.  The tiles of a group are equally high, in steps of 16, so that
-// none is a remainder that pays for a whole weight tile.
-__device__ __forceinline__ int4 token_tile(int group, int row0, int rows, int tiles, int j) {
-  const int h = ((rows + tiles - 1) / tiles + 15) & ~15;
+// Tile j of a group's `tiles`, which is rows / tile_rows rounded up: {group, first row, rows, 0}.  The tiles of a group are equally
+// high, in steps of 16, so that none is a remainder that pays for a whole weight tile, and at most tile_rows, which need not be
+// such a step.  With h <= tile_rows the first tiles - 1 cover less than the rows, so that the last has some.
+__device__ __forceinline__ int4 token_tile(int group, int row0, int rows, int tiles, int j, int tile_rows) {
+  const int h = min(((rows + tiles - 1) / tiles + 15) & ~15, tile_rows);
   return make_int4(group, row0 + j * h, min(h, rows - j * h), 0);
 }
 

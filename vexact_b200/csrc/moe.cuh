@@ -415,7 +415,7 @@ moe_index_kernel(const TIdx* __restrict__ experts, long long n, int E, int tile_
     }
   }
   for (int j = tid; j < tiles; j += 1024)
-    if (before[1] + j < max_tiles) tile_table[before[1] + j] = token_tile(mine, row0, rows, tiles, j);
+    if (before[1] + j < max_tiles) tile_table[before[1] + j] = token_tile(mine, row0, rows, tiles, j, tile_rows);
   int at = row0 + __reduce_add_sync(0xffffffffu, lane < warp ? own[lane] : 0);
   for (long long o = 0; o < seg; o += 32 * MOE_INDEX_AHEAD) {
     int ev[MOE_INDEX_AHEAD];
@@ -980,7 +980,7 @@ moe_route_plan_kernel(const TIn* __restrict__ logits, long long row_stride, __nv
     cu_seqlens[e] = rexcl;
     for (int j = 0; j < tiles; ++j)
       if (texcl + j < max_tiles)
-        tile_table[texcl + j] = token_tile(e, rexcl, rows, tiles, j);
+        tile_table[texcl + j] = token_tile(e, rexcl, rows, tiles, j, tile_rows);
     if (e == E - 1) {
       cu_seqlens[E] = rexcl + rows;
       *tile_count = min(texcl + tiles, max_tiles);

@@ -88,7 +88,7 @@ tiles_from_cu_seqlens_kernel(const int* __restrict__ cu_seqlens, int num_groups,
     const int t0 = first_tile[g];
     for (int j = 0; j < tiles; ++j)
       if (t0 + j < max_tiles)
-        table[1 + t0 + j] = token_tile(g, r0, rows, tiles, j);
+        table[1 + t0 + j] = token_tile(g, r0, rows, tiles, j, tile_rows);
   }
 }
 
