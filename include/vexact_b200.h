@@ -379,6 +379,12 @@ int b200_swiglu_backward(const void* gate, const void* up, long long in_row_stri
                          void* h_scaled, void* d_gate, void* d_up, long long d_row_stride, void* d_scale, long long rows,
                          int I, void* stream);
 
+/* No counterpart in the reference.  By default nothing is read before the launch before is over, the second operand w of a product
+ * included.  Between b200_settled_weights(1) and b200_settled_weights(0) the calling thread states that no work it launches
+ * writes the w of its dense products (b200_gemm_bf16, _f16, _bf16_ex, b200_gemm_glu, b200_gemm_swiglu), which may then be
+ * requested early.  Work launched before may have written it: the first launch in between waits for all of that. */
+int b200_settled_weights(int on);
+
 /* ---- vexact/batch_invariant_ops/fused_moe.py:319-336 for one dense MLP: out[t, i] = silu(x[t] . w[i]) *
  *      (x[t] . w[n_out + i]), w [2 * n_out, K] with the gate rows first; each product, silu and the result bf16. */
 int b200_gemm_swiglu(const void* x, const void* w, void* out, long long T, int n_out, int K, long long x_row_stride,

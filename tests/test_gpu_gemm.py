@@ -237,3 +237,42 @@ def test_products_on_cta_pairs_have_the_single_ctas_bits(vb, T, N, K):
     g, u = (x.double() @ w.double().t()).to(torch.bfloat16).double().chunk(2, 1)
     # three bf16 roundings after the products
     torch.testing.assert_close(gated(x).double(), torch.nn.functional.silu(g) * u, rtol=2 ** -6, atol=2 ** -6 * K ** 0.5)
+
+
+@pytest.mark.parametrize("T, N, K", [(64, 128, 512), (16, 256, 2048), (1500, 512, 256)])
+def test_second_operand_may_be_the_output_of_the_launch_before(vb, T, N, K):
+    """`k = x @ w^T; s = q @ k^T`, and a norm's output as the second operand: nothing is read from k before the launch that
+    makes it is over, however early the next launch starts.  k's storage holds the result for other inputs before each call."""
+    gen = torch.Generator(device="cuda").manual_seed(T + N)
+    w, gamma = torch.randn(K, K, device="cuda", generator=gen).to(BF), torch.ones(K, device="cuda", dtype=BF)
+    q = torch.randn(T, K, device="cuda", generator=gen).to(BF)
+    xs = [torch.randn(N, K, device="cuda", generator=gen).to(BF) for _ in range(8)]
+
+    def chain(x):
+        k = vb.linear(x, w)
+        s = vb.linear(q, k)
+        n = vb.batch_invariant_rms_norm(k, gamma, 1e-6)
+        return s, vb.linear(q, n)
+
+    def apart(x):
+        out = []
+        k = vb.linear(x, w)
+        torch.cuda.synchronize()
+        out.append(vb.linear(q, k))
+        n = vb.batch_invariant_rms_norm(k, gamma, 1e-6)
+        torch.cuda.synchronize()
+        return out + [vb.linear(q, n)]
+
+    want = [apart(x) for x in xs]
+    torch.cuda.synchronize()
+    got = [chain(x) for x in xs]
+    for a, b in zip(got, want):
+        assert torch.equal(a[0], b[0]) and torch.equal(a[1], b[1])
+    static = xs[0].clone()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        out = chain(static)
+    for x, b in zip(xs, want):
+        static.copy_(x)
+        graph.replay()
+        assert torch.equal(out[0], b[0]) and torch.equal(out[1], b[1])

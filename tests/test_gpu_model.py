@@ -218,3 +218,40 @@ def test_dense_mlp_routes_agree_bitwise():
     small = r._dense_mlp(x[:64], lw.gate_up, lw.down, shape.ffn)         # 64 tokens: fused route
     one = r._dense_mlp(x[17:18], lw.gate_up, lw.down, shape.ffn)
     assert torch.equal(big[:64], small) and torch.equal(big[17:18], one)
+
+
+@pytest.mark.parametrize("moe", [False, "dsv3"])
+def test_weights_written_right_before_a_step_are_the_ones_it_uses(moe):
+    """A forward pass may request weights before the launch before a product is over, but never before the work that was
+    launched ahead of the pass: weights copied in on the same stream, by a copy or by a kernel of this library, without a
+    synchronisation."""
+    import vexact_b200 as vb
+    from vexact_b200.inferencer import StageRunner, StageWeights, allocate_kv_cache
+
+    dev = torch.device("cuda")
+    shape = _tiny(moe)
+    sets = [StageWeights.random_init(shape, device=dev, seed=s, std=0.05) for s in (1, 2, 3)]
+    host, inp, nblocks = _inputs(shape, [5, 1, 20, 1], [5, 1, 20, 1], 16, dev)
+
+    def tensors(w):
+        return [t for lw in w.layers for _, t in sorted(vars(lw).items()) if isinstance(t, torch.Tensor)]
+
+    def logits(w):
+        kc, vc = allocate_kv_cache(shape, 0, shape.num_layers, nblocks, 16, device=dev)
+        torch.cuda.synchronize()
+        return StageRunner(w, kc, vc), kc
+
+    want = []
+    for w in sets[1:]:
+        w.embed, w.final_norm, w.lm_head = sets[0].embed, sets[0].final_norm, sets[0].lm_head
+        want.append(logits(w)[0].step(inp)[2].clone())
+    runner, _ = logits(sets[0])
+    eye = torch.eye(shape.hidden, device=dev, dtype=BF)
+    for turn in range(6):
+        new = sets[1 + turn % 2]
+        for dst, src in zip(tensors(sets[0]), tensors(new)):
+            if turn >= 3 and dst.dim() == 2 and dst.shape[1] == shape.hidden and dst.dtype == BF:
+                dst.copy_(vb.linear(src, eye))       # (the product with the identity: the same values)
+            else:
+                dst.copy_(src)
+        assert torch.equal(runner.step(inp)[2], want[turn % 2])

@@ -99,6 +99,7 @@ SIGNATURES = {
     "b200_moe_unpermute_reduce": [P, P, P, P, LL, I, I, P],
     "b200_moe_scatter": [P, LL, P, LL, LL, P, LL, LL, I, I, P],
     "b200_moe_gather": [P, LL, P, LL, LL, P, LL, I, I, P],
+    "b200_settled_weights": [I],
     "b200_gemm_swiglu": [P, P, P, LL, I, I, LL, LL, LL, P],
     "b200_seq_order": [P, P, I, P],
     "b200_moe_grouped_dgrad": [P, P, P, P, P, P, LL, I, I, I, LL, I, I, P],
@@ -217,6 +218,17 @@ def current_stream() -> int:
         raw, device = torch._C._cuda_getCurrentRawStream, torch._C._cuda_getDevice
         _current_stream = lambda: raw(device())  # noqa: E731
     return _current_stream()
+
+
+class settled_weights:
+    """`with settled_weights():` around the launches of a forward pass, none of which writes a weight: its dense products may
+    request their weights before the launch before them is over.  Weights written before it are waited for."""
+
+    def __enter__(self):
+        load().b200_settled_weights(1)
+
+    def __exit__(self, *exc):
+        load().b200_settled_weights(0)
 
 
 def read_status() -> tuple[int, int, int, int]:

@@ -164,6 +164,22 @@ inline int pdl_mode() {
   return mode;
 }
 
+// What the calling thread has said about its launches (b200_settled_weights): `ordered`, that its next one waits for all work
+// before it in full, and `settled`, that the weights of its dense products are written by nothing launched since.
+struct LaunchScope {
+  bool settled = false, ordered = false;
+};
+inline LaunchScope& launch_scope() {
+  static thread_local LaunchScope scope;
+  return scope;
+}
+inline bool launch_programmatic(bool pdl) {
+  LaunchScope& scope = launch_scope();
+  pdl = pdl && !scope.ordered;
+  scope.ordered = false;
+  return pdl;
+}
+
 // cluster: CTAs of a cluster along x (1: no cluster launch).
 template <typename... KArgs, typename... Args>
 inline void launch_k_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, bool pdl, int cluster,
@@ -174,7 +190,7 @@ inline void launch_k_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t
   cfg.dynamicSmemBytes = smem;
   cfg.stream = st;
   cudaLaunchAttribute attr[2];
-  if (pdl) {
+  if (launch_programmatic(pdl)) {
     attr[cfg.numAttrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[cfg.numAttrs++].val.programmaticStreamSerializationAllowed = 1;
   }
@@ -200,7 +216,7 @@ inline void launch_k(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t sme
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   const int mode = pdl_mode();
-  cfg.numAttrs = (mode == 1 || (mode >= 2 && smem == 0)) ? 1 : 0;
+  cfg.numAttrs = launch_programmatic(mode == 1 || (mode >= 2 && smem == 0)) ? 1 : 0;
   cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
 }
 

@@ -13,6 +13,7 @@ from typing import Optional
 
 import torch
 
+from ._lib import settled_weights
 from .batch_invariant_ops import gemm
 from .delta import DeltaWeights, delta_mixer
 from .fused_moe import MixtureWeights, mixture_forward
@@ -87,8 +88,11 @@ class HybridRunner:
     def forward(self, step: HybridStep, rows: torch.Tensor, after_layer=None) -> torch.Tensor:
         """Final-normed hidden states [R, width] of the packed token `rows` (int32).  `after_layer(run, streams)`: called
         with the residual streams [T, streams, width] a layer leaves (development and tests)."""
-        one_residual = self.shape.sandwich or self.shape.pre_norm
-        return (self._forward_residual if one_residual else self._forward_hyper)(step, rows, after_layer)
+        run = self._forward_residual if self.shape.sandwich or self.shape.pre_norm else self._forward_hyper
+        if after_layer is not None:      # (what the callback launches is not known here)
+            return run(step, rows, after_layer)
+        with settled_weights():
+            return run(step, rows, None)
 
     def _forward_hyper(self, step, rows, after_layer):
         s, w = self.shape, self.w

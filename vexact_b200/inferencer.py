@@ -388,8 +388,13 @@ class StageRunner:
 
     def forward(self, inp: StepInputs) -> torch.Tensor:
         """Hidden states after the local layers ([T, H]); the residual stream is complete."""
-        if inp.seq_order is None and ORDER_MIN_TILES < inp.context_lens.numel() * self.shape.num_kv_heads \
-                and inp.context_lens.numel() <= SEQ_ORDER_MAX:
+        with _lib.settled_weights():
+            return self._forward(inp)
+
+    def _forward(self, inp: StepInputs) -> torch.Tensor:
+        seqs, s = inp.context_lens.numel(), self.shape
+        if inp.seq_order is None and seqs <= SEQ_ORDER_MAX and order_pays(seqs, s.num_q_heads, s.num_kv_heads,
+                                                                         _lib.sm_count(inp.context_lens.device)):
             inp = replace(inp, seq_order=descending_contexts(inp.context_lens))
         if self.is_first:
             h = _gather_rows(self.w.embed, ids=inp.input_ids)
