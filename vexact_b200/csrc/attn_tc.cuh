@@ -494,8 +494,7 @@ paged_attn_tc_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_cons
         const int pi = c / t.heads_here;
         s_cpos[c] = t.q_abs0 + t.tile_pos0 + (pi < npos ? pi : 0);
       }
-      ptx::named_barrier_sync(3, NCT);
-      if (*abort_flag) break;
+      if (ptx::named_barrier_any(3, NCT, *abort_flag != 0)) break;
 
       float o_acc[NCL];
       float l_w = 0.f;   // running row sum of my warp's 32 keys for local column `mycol`
@@ -561,8 +560,7 @@ paged_attn_tc_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_cons
               for (int h = 0; h < VH; ++h) reinterpret_cast<uint32_t*>(vt + h * (ATC_BN * 128) + r * 128)[lane] = 0u;
           }
         }
-        ptx::named_barrier_sync(3, NCT);
-        if (*abort_flag) break;
+        if (ptx::named_barrier_any(3, NCT, *abort_flag != 0)) break;
         // (B) running maximum and rescale factor, one thread per column
         if constexpr (!LOCAL_M) {
           for (int c = ct; c < NC; c += NCT) {
@@ -573,7 +571,6 @@ paged_attn_tc_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_cons
             s_alpha[b][c] = fast_exp2(m_old - m_new);
           }
           ptx::named_barrier_sync(3, NCT);
-          if (*abort_flag) break;
         }
         // (C) the previous block's PV product has been running meanwhile; once it is over its O^T can be
         //     folded in and the P^T tile it read can be rewritten
@@ -696,8 +693,7 @@ paged_attn_tc_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_cons
         // are added as (l_0 + l_1) + (l_2 + l_3) below
         s_lred[gcol(mycol >> 2) + (mycol & 3)][q4] = l_w;
       }
-      ptx::named_barrier_sync(3, NCT);
-      if (*abort_flag) break;  // uniform over the compute threads: read after a common barrier
+      if (ptx::named_barrier_any(3, NCT, *abort_flag != 0)) break;
       // Output.  A thread holds one value-dim element of NC / 2 columns; stored as they are that is one 2-byte
       // store per column.  Each warp turns 8 columns x its 32 dims around in shared memory instead (its 512-byte
       // slice of the P^T tile, which nothing reads between the tile's last PV product and the barrier that

@@ -550,11 +550,8 @@ gemm_ws_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__
       const int buf = tile_it & 1;
       const bool ready = ptx::mbar_wait(tfull_bar(buf), (tile_it >> 1) & 1, abort_flag, 400 + buf);
       if (SWIGLU || HEAD) {
-        // The epilogue warps meet at named barriers below, so they must leave together: a wait
-        // that gave up has raised the abort flag before its warp arrives here, and everyone reads
-        // the flag after this barrier.
-        ptx::named_barrier_sync(1, HEAD ? 128 : 256);
-        if (*abort_flag) break;
+        // the epilogue warps meet at named barriers below, so they must leave together
+        if (ptx::named_barrier_any(1, HEAD ? 128 : 256, !ready)) break;
       } else if (!__all_sync(0xffffffffu, ready)) {
         break;
       }

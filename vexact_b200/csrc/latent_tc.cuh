@@ -193,22 +193,6 @@ __device__ __forceinline__ LtcItem ltc_item(const LatentTcParams& p, const LtcRa
   return t;
 }
 
-// Named barrier 3 of the compute warps with a vote: true when any of the n threads brings true.
-__device__ __forceinline__ bool barrier_any(bool mine, int n) {
-  uint32_t any;
-  asm volatile(
-      "{\n"
-      ".reg .pred p, q;\n"
-      "setp.ne.u32 q, %1, 0;\n"
-      "barrier.cta.red.or.pred p, 3, %2, q;\n"
-      "selp.u32 %0, 1, 0, p;\n"
-      "}\n"
-      : "=r"(any)
-      : "r"((uint32_t)mine), "r"(n)
-      : "memory");
-  return any != 0;
-}
-
 __device__ __forceinline__ void tmem_ld8(uint32_t taddr, uint32_t* r) {
   asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
                : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
@@ -503,8 +487,7 @@ latent_tc_kernel(const __grid_constant__ CUtensorMap tm, const LatentTcParams p)
             }
           }
         }
-        const bool rescale = barrier_any(over, NCT);
-        if (*abort_flag) break;
+        const bool rescale = ptx::named_barrier_any(3, NCT, over || *abort_flag != 0);
         float alpha[NH];
 #pragma unroll
         for (int i = 0; i < NH; ++i) alpha[i] = 1.f;
@@ -517,8 +500,7 @@ latent_tc_kernel(const __grid_constant__ CUtensorMap tm, const LatentTcParams p)
             if ((lane & 7) == i) mine = w;
           }
           if (lane < 8) s_wmax[b][c0 + lane][q4] = mine;
-          ptx::named_barrier_sync(3, NCT);
-          if (*abort_flag) break;
+          if (ptx::named_barrier_any(3, NCT, *abort_flag != 0)) break;
 #pragma unroll
           for (int i = 0; i < NH; ++i) {
             const float4 w = *reinterpret_cast<const float4*>(s_wmax[b][c0 + i]);
@@ -575,8 +557,7 @@ latent_tc_kernel(const __grid_constant__ CUtensorMap tm, const LatentTcParams p)
         ptx::tc_fence_before();
         s_lred[c0 + mycol][q4] = l_w;
       }
-      ptx::named_barrier_sync(3, NCT);
-      if (*abort_flag) break;
+      if (ptx::named_barrier_any(3, NCT, *abort_flag != 0)) break;
 #pragma unroll
       for (int i = 0; i < NH; ++i) {
         const int c = c0 + i;

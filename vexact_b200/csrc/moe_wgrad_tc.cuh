@@ -168,9 +168,7 @@ moe_wgrad_tc_kernel(const __grid_constant__ WgradMaps tm, const int* __restrict_
       const int n = wgrad_rows(cu_seqlens, g, rows, r0, false);
       ptx::mbar_wait(tfull(buf), (tile_it >> 1) & 1, abort_flag, 930 + buf);
       if (threadIdx.x == 128) ptx::bulk_wait_read0();      // the previous tile's copy out has read the staging tile
-      // a wait that gave up raised the flag before this barrier: all eight warps leave together
-      ptx::named_barrier_sync(1, 256);
-      if (*abort_flag) break;
+      if (ptx::named_barrier_any(1, 256, !ready)) break;   // all eight warps leave together
       ptx::tc_fence_after();
       const uint32_t taddr = tmem + ((uint32_t)(q * 32) << 16) + buf * WGT_N;
 #pragma unroll

@@ -339,6 +339,23 @@ __device__ __forceinline__ uint32_t umma_idesc_f16_m128(uint32_t n) {
 __device__ __forceinline__ void named_barrier_sync(int id, int nthreads) {
   asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(nthreads) : "memory");
 }
+// The same with a vote: true for every thread when any of them brings true.  Warps that meet at named barriers decide by it
+// whether to leave: the abort flag can go up at any time, so a warp that reads it after a barrier may see what another has
+// not, leave alone, and strand the others at their next barrier.
+__device__ __forceinline__ bool named_barrier_any(int id, int nthreads, bool mine) {
+  uint32_t any;
+  asm volatile(
+      "{\n"
+      ".reg .pred p, q;\n"
+      "setp.ne.u32 q, %1, 0;\n"
+      "barrier.cta.red.or.pred p, %2, %3, q;\n"
+      "selp.u32 %0, 1, 0, p;\n"
+      "}\n"
+      : "=r"(any)
+      : "r"((uint32_t)mine), "r"(id), "r"(nthreads)
+      : "memory");
+  return any != 0;
+}
 
 }  // namespace ptx
 }  // namespace b200
