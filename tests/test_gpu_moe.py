@@ -571,6 +571,12 @@ def test_grouped_gemm_tile_heights_and_unfused_swiglu(vb, E, k, T, H, I):
     assert vb._lib.read_status()[0] == 0
 
 
+def _tile_table(cu, height):
+    rows = [(e, r, min(height, cu[e + 1] - r), 0) for e in range(len(cu) - 1) for r in range(cu[e], cu[e + 1], height)]
+    return dict(tile_table=torch.tensor(rows, dtype=torch.int32, device="cuda"), max_tiles=len(rows), tile_rows=height,
+                tile_count=torch.tensor([len(rows)], dtype=torch.int32, device="cuda"))
+
+
 @pytest.mark.parametrize("K", [192, 200])
 @pytest.mark.parametrize("height", [16, 48, 80, 96, 112, 144, 176, 208, 240, 256])
 def test_grouped_products_at_every_tile_height(vb, height, K):

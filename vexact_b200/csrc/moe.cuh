@@ -1280,8 +1280,8 @@ extern "C" int b200_transpose_last2(const void* x, void* out, int G, int R, int 
 }
 
 // c[g] = a[rows of g]^T @ b[rows of g]: a [rows, M], b [rows, N] with rows a_row_stride and b_row_stride apart, c [G, M, N]
-// bf16 contiguous, cu_seqlens [G + 1] i32 (rows of group g are [cu[g], cu[g + 1])).  M, N and the strides multiples of 8
-// and 16-byte aligned pointers; contiguous a and b also with multiples of 4 and 8-byte aligned pointers.
+// bf16 contiguous, cu_seqlens [G + 1] i32 (rows of group g are [cu[g], cu[g + 1])).  M, N and the strides multiples of 8,
+// a and b 16-byte, c 4-byte aligned; contiguous a and b also with multiples of 4 and 8-byte aligned pointers.
 extern "C" int b200_moe_grouped_wgrad_strided(const void* a, long long a_row_stride, const void* b, long long b_row_stride,
                                               void* c, const void* cu_seqlens, long long rows, int num_groups, int M, int N,
                                               void* stream) {
@@ -1295,6 +1295,7 @@ extern "C" int b200_moe_grouped_wgrad_strided(const void* a, long long a_row_str
     return moe_wgrad_tc_launch(a, a_row_stride, b, b_row_stride, c, (const int*)cu_seqlens, rows, num_groups, M, N,
                                (cudaStream_t)stream);
   if (a_row_stride != M || b_row_stride != N) return B200_ERR_SHAPE;
+  if ((reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(b) | reinterpret_cast<uintptr_t>(c)) & 7) return B200_ERR_SHAPE;
   launch_k(moe_wgrad_kernel, dim3((unsigned)((N + WG_TILE - 1) / WG_TILE), (unsigned)((M + WG_TILE - 1) / WG_TILE),
                                   (unsigned)num_groups),
            dim3(256), 0, (cudaStream_t)stream, (const __nv_bfloat16*)a, (const __nv_bfloat16*)b, (__nv_bfloat16*)c,

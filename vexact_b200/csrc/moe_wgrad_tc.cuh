@@ -43,7 +43,7 @@ __device__ __forceinline__ int wgrad_rows(const int* cu_seqlens, int g, int rows
 
 __global__ void __launch_bounds__(WGT_THREADS, 1)
 moe_wgrad_tc_kernel(const __grid_constant__ WgradMaps tm, const int* __restrict__ cu_seqlens, int rows, int groups, int m_tiles,
-                    int n_tiles, int N, bool deep) {
+                    int n_tiles, int N, bool deep, int M, __nv_bfloat16* c_words) {
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw = ptx::smem_u32(smem_raw);
   const uint32_t stage0 = (raw + 1023) & ~1023u, out0 = stage0 + WGT_STAGES * WGT_STAGE;
@@ -192,7 +192,15 @@ moe_wgrad_tc_kernel(const __grid_constant__ WgradMaps tm, const int* __restrict_
       ptx::mbar_arrive(tempty(buf));
       ptx::fence_proxy_async_smem();
       ptx::named_barrier_sync(1, 256);
-      if (threadIdx.x == 128) {
+      if (c_words) {
+        // c on a 4-byte boundary: the staged tile leaves as words, a warp's 128 bytes of a row together
+        for (int i = warp - 4; i < WGT_M * (WGT_N / 64); i += 8) {
+          const int h = i / WGT_M, r = i % WGT_M, col = n0 + h * 64 + lane * 2;
+          if (m0 + r < M && col < N)
+            *reinterpret_cast<uint32_t*>(c_words + ((long long)g * M + m0 + r) * N + col) =
+                *reinterpret_cast<const uint32_t*>(out_ptr + h * (WGT_M * 128) + r * 128 + (((lane >> 2) ^ (r & 7)) << 4) + (lane & 3) * 4);
+        }
+      } else if (threadIdx.x == 128) {
         for (int h = 0; h < WGT_N / 64; ++h)
           if (n0 + h * 64 < N) ptx::tma_store_3d(&tm.c, out0 + h * (WGT_M * 128), n0 + h * 64, m0, g);
         ptx::bulk_commit();
@@ -229,12 +237,14 @@ inline int moe_wgrad_tc_launch(const void* a, long long a_stride, const void* b,
   if (!rc)
     rc = deep ? make_tmap_deep(&tm.b, b, map_rows, (uint64_t)N, (uint64_t)b_stride, WGT_ROWS, WGT_N / 64)
               : make_tmap_2d(&tm.b, b, map_rows, (uint64_t)N, (uint64_t)b_stride, WGT_ROWS);
-  if (!rc) rc = make_tmap_3d(&tm.c, c, (uint64_t)groups, (uint64_t)M, (uint64_t)N, (uint64_t)M * N, (uint64_t)N, WGT_M);
+  const bool words = (reinterpret_cast<uintptr_t>(c) & 15) != 0;
+  if (words) tm.c = tm.a;
+  else if (!rc) rc = make_tmap_3d(&tm.c, c, (uint64_t)groups, (uint64_t)M, (uint64_t)N, (uint64_t)M * N, (uint64_t)N, WGT_M);
   if (rc) return rc;
   const int m_tiles = (M + WGT_M - 1) / WGT_M, n_tiles = (N + WGT_N - 1) / WGT_N;
   const long long total = (long long)m_tiles * n_tiles * groups;
   launch_k(moe_wgrad_tc_kernel, dim3((unsigned)(total < sm_count() ? total : sm_count())), dim3(WGT_THREADS), WGT_SMEM, st, tm,
-           cu_seqlens, (int)rows, groups, m_tiles, n_tiles, N, deep);
+           cu_seqlens, (int)rows, groups, m_tiles, n_tiles, N, deep, M, words ? (__nv_bfloat16*)c : nullptr);
   return launch_status();
 }
 
