@@ -260,7 +260,9 @@ int b200_paged_attn_fwd_ordered(const void* q, const void* k_cache, const void* 
                                 long long kc_head_stride, long long vc_block_stride, long long vc_page_stride,
                                 long long vc_head_stride, float softmax_scale, const void* seq_order,
                                 long long total_q, void* stream);
-/* The same, and lse_f32 [num_q_heads, total_q] receives log2 of every query's sum of 2^(score * softmax_scale * log2 e). */
+/* The same, and lse_f32 [num_q_heads, total_q] receives log2 of every query's sum of 2^(score * softmax_scale * log2 e).  It serves
+ * queries for which b200_paged_attn_has_lse returns 1 (not a status: 0 otherwise). */
+int b200_paged_attn_has_lse(const void* q, int dk, int dv, long long q_tok_stride, long long q_head_stride);
 int b200_paged_attn_fwd_lse(const void* q, const void* k_cache, const void* v_cache, void* out,
                                 const void* cu_seqlens_q, const void* seqused_k, const void* page_table,
                                 int num_seqs, int max_seqlen_q, int num_q_heads, int num_kv_heads, int dk, int dv,

@@ -629,3 +629,37 @@ def test_log_sum_exp_of_the_forward(vb, hq, hkv, dk):
         # fp32 scores of magnitude up to 8 and sums of up to 421 of them, ex2 to 2^-22
         torch.testing.assert_close(lse[:, a:a + nq].double(), ref, rtol=0, atol=2e-5)
         a, b = a + nq, b + nk
+def test_training_forward_asks_the_library_whether_there_is_a_log_sum_exp(tmp_path):
+    """The library reads B200_ATTN once; what the variable holds later changes nothing, and a library without the tensor-memory
+    kernels trains on the backward that makes its own log-sum-exp."""
+    import subprocess
+    import sys
+
+    script = """
+import os, sys, torch
+os.environ["B200_ATTN"] = sys.argv[2]
+import vexact_b200 as vb
+g = torch.Generator().manual_seed(5)
+lens = [70, 33]
+q, k, v = (torch.randn(103, h, 128, generator=g).bfloat16().cuda().requires_grad_() for h in (4, 2, 2))
+cu = torch.tensor([0, 70, 103], dtype=torch.int32).cuda()
+call = lambda: vb.flash_attn_varlen_func(q, k, v, cu, cu, max_seqlen_q=70, max_seqlen_k=70, causal=True)[0]
+with torch.no_grad():
+    call()
+os.environ["B200_ATTN"] = sys.argv[3]
+grads = torch.autograd.grad(call(), (q, k, v), torch.randn(103, 4, 128, generator=g).bfloat16().cuda())
+torch.cuda.synchronize()
+assert vb._lib.read_status()[0] == 0
+torch.save([t.cpu().float() for t in grads], sys.argv[1])
+"""
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    grads = []
+    for first, later in (("", ""), ("sync", ""), ("", "sync")):
+        path = str(tmp_path / f"{first}-{later}.pt")
+        subprocess.run([sys.executable, "-c", script, path, first, later], check=True, env=dict(os.environ, PYTHONPATH=root),
+                       cwd=root, timeout=180)
+        grads.append(torch.load(path))
+    for a, b, c in zip(*grads):
+        # log-sum-exps of two kernels, then bf16 roundings of the same products: one bf16 ulp of the largest gradient
+        torch.testing.assert_close(a, b, rtol=0, atol=2 ** -7 * a.abs().max().item())
+        assert torch.equal(a, c)

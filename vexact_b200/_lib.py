@@ -85,6 +85,7 @@ SIGNATURES = {
                             LL, LL, F, P],
     "b200_paged_attn_fwd_ordered": [P, P, P, P, P, P, P, I, I, I, I, I, I, I, I, I, LL, LL, LL, LL, LL, LL, LL, LL, LL,
                             LL, LL, F, P, LL, P],
+    "b200_paged_attn_has_lse": [P, I, I, LL, LL],
     "b200_paged_attn_fwd_lse": [P, P, P, P, P, P, P, I, I, I, I, I, I, I, I, I, LL, LL, LL, LL, LL, LL, LL, LL, LL,
                             LL, LL, F, P, LL, P, P],
     "b200_moe_route_softmax_topk": [P, I, LL, P, P, P, P, LL, I, I, I, P],

@@ -13,7 +13,6 @@
 """
 from __future__ import annotations
 
-import os
 from typing import Optional
 
 import torch
@@ -233,10 +232,9 @@ class _PackedVarlenForward(torch.autograd.Function):
         out = torch.zeros((qp.shape[0], qp.shape[1], vp.shape[-1]), dtype=qp.dtype, device=qp.device)
         needed = any(ctx.needs_input_grad[:3])
         lse = None
-        # the rows-on-lanes kernel leaves it, where it is the one that runs
-        if needed and (qp.shape[-1], vp.shape[-1]) != (64, 64) and qp.stride(-1) == 1 and qp.shape[0] > 0 \
-                and os.environ.get("B200_ATTN", "")[:1] != "s" \
-                and qp.data_ptr() % 16 == 0 and qp.stride(0) % 8 == 0 and qp.stride(1) % 8 == 0:
+        # the rows-on-lanes kernel leaves it, where it serves these queries
+        if needed and qp.stride(-1) == 1 and qp.shape[0] > 0 and _lib.load().b200_paged_attn_has_lse(
+                qp.data_ptr(), qp.shape[-1], vp.shape[-1], qp.stride(0), qp.stride(1)):
             # (inf: queries of a refused sequence weigh nothing)
             lse = torch.full((qp.shape[1], qp.shape[0]), float("inf"), dtype=torch.float32, device=qp.device)
         paged_attention(qp, k_cache, v_cache, cu_q, lens, table, scale, max_seqlen_q, out=out, lse=lse)

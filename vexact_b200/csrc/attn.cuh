@@ -469,6 +469,11 @@ extern "C" int b200_paged_attn_fwd(const void* q, const void* k_cache, const voi
 }
 
 namespace b200 {
+// The tcgen05 kernels' head dims and queries; they alone can leave the rows' log-sum-exp.
+inline bool attn_on_tensor_memory(const void* q, int dk, int dv, long long q_tok_stride, long long q_head_stride) {
+  return attn_use_tensor_memory() && dv == 128 && (dk == 128 || dk == 192) && q_tok_stride % 8 == 0 && q_head_stride % 8 == 0 &&
+         (reinterpret_cast<uintptr_t>(q) & 15) == 0;
+}
 int paged_attn_fwd_impl(const void* q, const void* k_cache, const void* v_cache, void* out, const void* cu_seqlens_q,
                         const void* seqused_k, const void* page_table, int num_seqs, int max_seqlen_q, int num_q_heads,
                         int num_kv_heads, int dk, int dv, int num_blocks, int page_size, int max_pages, long long page_table_stride,
@@ -477,6 +482,11 @@ int paged_attn_fwd_impl(const void* q, const void* k_cache, const void* v_cache,
                         long long vc_page_stride, long long vc_head_stride, float softmax_scale, const void* seq_order,
                         long long total_q, void* lse, void* stream);
 }  // namespace b200
+
+// 1 where b200_paged_attn_fwd_lse serves these queries, 0 where it refuses them.
+extern "C" int b200_paged_attn_has_lse(const void* q, int dk, int dv, long long q_tok_stride, long long q_head_stride) {
+  return b200::attn_on_tensor_memory(q, dk, dv, q_tok_stride, q_head_stride);
+}
 
 // Same, with an optional processing order: seq_order[i] (int32, a permutation of 0..num_seqs-1, e.g.
 // sequences by descending context length) is the sequence the i-th group of tiles belongs to.  The
@@ -498,8 +508,8 @@ extern "C" int b200_paged_attn_fwd_ordered(const void* q, const void* k_cache, c
 }
 
 // The same, and lse_f32 [num_q_heads, total_q] receives log2 of every query's sum of 2^(score * softmax_scale * log2 e) over the
-// unrounded weights (queries of a refused sequence keep what it held).  Head dims (128, 128) and (192, 128), 16-byte aligned
-// queries.
+// unrounded weights (queries of a refused sequence keep what it held).  For queries that b200_paged_attn_has_lse accepts: head
+// dims (128, 128) and (192, 128), 16-byte aligned.
 extern "C" int b200_paged_attn_fwd_lse(const void* q, const void* k_cache, const void* v_cache, void* out,
                                            const void* cu_seqlens_q, const void* seqused_k, const void* page_table,
                                            int num_seqs, int max_seqlen_q, int num_q_heads, int num_kv_heads,
@@ -575,8 +585,7 @@ int b200::paged_attn_fwd_impl(const void* q, const void* k_cache, const void* v_
   }
   if (num_seqs > 65535 || num_kv_heads * p.head_chunks > 65535) return B200_ERR_SHAPE;
   const int hh = group < 8 ? group : 8;
-  if (attn_use_tensor_memory() && dv == 128 && (dk == 128 || dk == 192) && q_tok_stride % 8 == 0 &&
-      q_head_stride % 8 == 0 && (reinterpret_cast<uintptr_t>(q) & 15) == 0) {
+  if (attn_on_tensor_memory(q, dk, dv, q_tok_stride, q_head_stride)) {
     // tcgen05 kernels.  A decode step (one query per sequence) uses the narrow keys-on-lanes tile (16
     // columns); steps with longer query runs use 128-row tiles with two threads per row (attn_rows.cuh): four
     // prompts of together 3001 tokens, 16 heads of 192 / 128, took 225 us on 32-column keys-on-lanes tiles, whose
