@@ -629,6 +629,33 @@ def test_log_sum_exp_of_the_forward(vb, hq, hkv, dk):
         # fp32 scores of magnitude up to 8 and sums of up to 421 of them, ex2 to 2^-22
         torch.testing.assert_close(lse[:, a:a + nq].double(), ref, rtol=0, atol=2e-5)
         a, b = a + nq, b + nk
+
+
+@pytest.mark.parametrize("hq,hkv", [(4, 4), (8, 2)])
+@pytest.mark.parametrize("q_lens", [[8] * 4, [32] * 3, [33] * 3, [1] * 40 + [32], [1] * 40 + [33], [1] * 40 + [128], [1] * 40 + [129]])
+def test_192_wide_keys_on_either_side_of_the_tile_rule(vb, hq, hkv, q_lens):
+    """Steps that do and do not fill 128-row tiles: the kernel that the rule takes, the keys-on-lanes kernel and the
+    rows-on-lanes kernel (which a log-sum-exp asks for) give the same bits."""
+    from vexact_b200.attention import paged_attention
+
+    S, page = len(q_lens), 16
+    ctx = [n + (37 * i) % 300 for i, n in enumerate(q_lens)]
+    pages = max((c + page - 1) // page for c in ctx)
+    gen = torch.Generator(device="cuda").manual_seed(S + hq)
+    kc, vc = (torch.randn(S * pages, page, hkv, d, device="cuda", generator=gen).to(BF) for d in (192, 128))
+    table = torch.randperm(S * pages, device="cuda", generator=gen).view(S, pages).to(torch.int32)
+    q = torch.randn(sum(q_lens), hq, 192, device="cuda", generator=gen).to(BF)
+    cu = torch.tensor([0] + torch.tensor(q_lens).cumsum(0).tolist(), dtype=torch.int32, device="cuda")
+    args = q, kc, vc, cu, torch.tensor(ctx, dtype=torch.int32, device="cuda"), table, 192 ** -0.5, max(q_lens)
+    out = paged_attention(*args)
+    assert torch.equal(out, paged_attention(*args, lse=torch.empty(hq, q.shape[0], device="cuda")))
+    os.environ["B200_ATTN_PREFILL"] = "cols"
+    try:
+        assert torch.equal(out, paged_attention(*args))
+    finally:
+        del os.environ["B200_ATTN_PREFILL"]
+
+
 def test_training_forward_asks_the_library_whether_there_is_a_log_sum_exp(tmp_path):
     """The library reads B200_ATTN once; what the variable holds later changes nothing, and a library without the tensor-memory
     kernels trains on the backward that makes its own log-sum-exp."""

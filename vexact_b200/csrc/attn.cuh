@@ -590,7 +590,14 @@ int b200::paged_attn_fwd_impl(const void* q, const void* k_cache, const void* v_
     // columns); steps with longer query runs use 128-row tiles with two threads per row (attn_rows.cuh): four
     // prompts of together 3001 tokens, 16 heads of 192 / 128, took 225 us on 32-column keys-on-lanes tiles, whose
     // softmax crosses lanes.  B200_ATTN_PREFILL=cols keeps those tiles (the same bits, for cross-checks).
-    const bool rows = lse || (max_seqlen_q > 1 && attn_prefill_rows());
+    // A tile of 128 rows with 192-wide keys takes 1.2 times as long as one of 32 columns, however few of them are used, so
+    // it is for steps that fill it: a mean of more than 32 queries a sequence, or a sequence of more than 128 (16 heads, us,
+    // rows / columns: 32 sequences of 16 / 33 / 64 queries after 2048 tokens 165 / 141, 165 / 238, 165 / 244; 64 decoding
+    // sequences at 4096 with a prompt of 64 / 192 / 512 tokens 521 / 430, 530 / 532, 538 / 605; 200 at 1024 with one of 64 / 200
+    // 444 / 401, 456 / 569).
+    const long long run = (long long)max_seqlen_q * hh;
+    const bool fills = dk == 128 || run > 128 || total_q * hh > 32LL * num_seqs;
+    const bool rows = lse || (max_seqlen_q > 1 && fills && attn_prefill_rows());
     p.lse = (float*)lse;
     p.lse_stride = total_q;
     const int nc = rows ? 128 : max_seqlen_q == 1 ? 16 : dk == 128 ? 64 : 32;
