@@ -57,7 +57,8 @@ def test_route_sigmoid_group_topk(vb):
         assert torch.equal(torch.sort(idx.cpu(), 1).values, torch.sort(c["experts"], 1).values)
 
 
-@pytest.mark.parametrize("T,k,E", [(12, 4, 8), (512, 8, 128), (2048, 8, 128), (256, 6, 64), (1, 8, 128), (3000, 2, 5)])
+@pytest.mark.parametrize("T,k,E", [(12, 4, 8), (512, 8, 128), (2048, 8, 128), (256, 6, 64), (1, 8, 128), (3000, 2, 5),
+                                   (2048, 1, 7), (2049, 1, 7), (64, 32, 200), (65, 32, 200)])
 def test_moe_indices_bit_exact(vb, T, k, E):
     from vexact_b200.fused_moe import build_moe_indices
 

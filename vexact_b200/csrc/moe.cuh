@@ -341,12 +341,132 @@ moe_route_sigmoid_group_topk_kernel(const float* __restrict__ logits, long long 
 // plus cu_seqlens[E + 1] and the token-tile table of the grouped GEMM (tiles of at most
 // `tile_rows` consecutive rows of one expert).
 //
-// One CTA of 1024 threads per expert; each reads all entries and needs nothing from the others.  Warp w owns the contiguous
-// segment [w * seg, (w + 1) * seg) of the flat array and walks it 32 entries at a time, eight steps' entries requested at once:
-// a histogram of all experts in shared memory gives the rows and tiles before this one, a ballot per step the expert's own
-// entries in order.  All of it is integer arithmetic: bit-exact.  (One CTA for all experts, ranking by __match_any_sync, which
-// takes a turn per distinct value: 25 / 47 us for 16384 / 32768 entries of 128 experts.)
+// Two forms, both integer arithmetic: bit-exact.  In both, warp w owns the contiguous segment [w * seg, (w + 1) * seg) of the flat
+// array and walks it 32 entries at a time.
+//
+// Up to MOE_INDEX_ONE entries: one CTA for all experts.  __match_any_sync groups equal experts of a step, the lowest lane of a group
+// bumps the warp's private per-expert counter, so every entry learns its rank among the warp's earlier entries of the same expert;
+// a per-expert scan over the 32 warps and a scan over the experts turn those ranks into global positions.
+// More: one CTA of 1024 threads per expert; each reads all entries, eight steps' at once, and needs nothing from the others: a
+// histogram of all experts in shared memory gives the rows and tiles before this one, a ballot per step the expert's own entries
+// in order.
+// One CTA / a CTA per expert, 128 experts, us: 8 entries 3.3 / 5.3, 512 3.7 / 5.3, 2048 5.4 / 5.5, 4096 7.9 / 5.5, 32768 45.5 / 13.8 (the
+// first takes a turn per distinct value of a step); with the kernel that moves the rows behind it, which starts the sooner the
+// fewer CTAs are before it: 512 5.4 / 8.3, 2048 8.6 / 9.2, 4096 12.5 / 10.6.
 constexpr int MOE_INDEX_AHEAD = 8;
+constexpr long long MOE_INDEX_ONE = 2048;
+template <typename TIdx>
+__global__ void __launch_bounds__(1024)
+moe_index_one_kernel(const TIdx* __restrict__ experts, long long n, int E, int tile_rows,
+                 int* __restrict__ scatter_index, int* __restrict__ cu_seqlens, int4* __restrict__ tile_table,
+                 int* __restrict__ tile_count, int max_tiles, int topk, int* __restrict__ gather_index,
+                 const __nv_bfloat16* __restrict__ weights, __nv_bfloat16* __restrict__ row_scale) {
+  pdl_trigger();
+  pdl_wait();
+  __shared__ int cnt[32][MOE_MAX_EXPERTS];  // per-warp counts, then per-warp exclusive offsets
+  __shared__ int base[MOE_MAX_EXPERTS];     // expert totals, then exclusive prefix (cu_seqlens)
+  __shared__ int tbase[MOE_MAX_EXPERTS];    // first tile index of each expert
+  __shared__ int wsum[32];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  for (int i = tid; i < 32 * MOE_MAX_EXPERTS; i += 1024) (&cnt[0][0])[i] = 0;
+  __syncthreads();
+  const long long seg = ((n + 31) / 32 + 31) / 32 * 32;  // entries per warp, a multiple of 32
+  const long long w0 = warp * seg;
+  // pass 1: rank of every entry among the warp's earlier entries of the same expert
+  for (long long o = 0; o < seg; o += 32) {
+    const long long i = w0 + o + lane;
+    int e = -1;
+    if (i < n) {
+      const long long ev = (long long)experts[i];
+      if (ev >= 0 && ev < E)
+        e = (int)ev;
+      else
+        report_status(B200_STATUS_BAD_INDEX, (int)ev);
+    }
+    const unsigned mask = __match_any_sync(0xffffffffu, e);
+    const int rank = __popc(mask & ((1u << lane) - 1u));
+    const int leader = __ffs(mask) - 1;
+    int old = 0;
+    if (rank == 0 && e >= 0) {
+      old = cnt[warp][e];
+      cnt[warp][e] = old + __popc(mask);
+    }
+    old = __shfl_sync(0xffffffffu, old, leader);
+    if (i < n) scatter_index[i] = e >= 0 ? old + rank : -1;
+    __syncwarp();
+  }
+  __syncthreads();
+  // per expert: exclusive scan over the warps, total into base[]
+  if (tid < E) {
+    int run = 0;
+#pragma unroll 8
+    for (int w = 0; w < 32; ++w) {
+      const int c = cnt[w][tid];
+      cnt[w][tid] = run;
+      run += c;
+    }
+    base[tid] = run;
+  }
+  __syncthreads();
+  // exclusive scans over the experts (rows and tiles), 256 threads = 8 warps
+  if (tid < MOE_MAX_EXPERTS) {
+    const int rows = tid < E ? base[tid] : 0;
+    const int tiles = (rows + tile_rows - 1) / tile_rows;
+    int r = rows, t = tiles;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int r2 = __shfl_up_sync(0xffffffffu, r, o);
+      const int t2 = __shfl_up_sync(0xffffffffu, t, o);
+      if (lane >= o) {
+        r += r2;
+        t += t2;
+      }
+    }
+    if (lane == 31) {
+      wsum[warp] = r;
+      wsum[8 + warp] = t;
+    }
+    // (only warps 0..7 reach here; named barrier over their 256 threads)
+    asm volatile("bar.sync 2, 256;" ::: "memory");
+    int roff = 0, toff = 0;
+    for (int w = 0; w < warp; ++w) {
+      roff += wsum[w];
+      toff += wsum[8 + w];
+    }
+    const int rexcl = roff + r - rows;
+    const int texcl = toff + t - tiles;
+    asm volatile("bar.sync 2, 256;" ::: "memory");
+    if (tid < E) {
+      base[tid] = rexcl;
+      tbase[tid] = texcl;
+      cu_seqlens[tid] = rexcl;
+      for (int j = 0; j < tiles; ++j)
+        if (texcl + j < max_tiles)
+          tile_table[texcl + j] = token_tile(tid, rexcl, rows, tiles, j, tile_rows);
+      if (tid == E - 1) {
+        cu_seqlens[E] = rexcl + rows;
+        *tile_count = min(texcl + tiles, max_tiles);
+      }
+    }
+  }
+  __syncthreads();
+  // pass 2: local rank -> global position
+  for (long long o = 0; o < seg; o += 32) {
+    const long long i = w0 + o + lane;
+    if (i < n) {
+      const long long ev = (long long)experts[i];
+      if (ev >= 0 && ev < E) {
+        const int pos = scatter_index[i] + base[(int)ev] + cnt[warp][(int)ev];
+        scatter_index[i] = pos;
+        // the inverse map for a GEMM that gathers its rows (sorted row -> token), and the routing weight
+        // of each sorted row, so that no permuted copy of the activations has to be made
+        if (gather_index) gather_index[pos] = (int)(i / topk);
+        if (row_scale) row_scale[pos] = weights[i];
+      }
+    }
+  }
+}
+
 template <typename TIdx>
 __global__ void __launch_bounds__(1024)
 moe_index_kernel(const TIdx* __restrict__ experts, long long n, int E, int tile_rows,
@@ -1179,11 +1299,13 @@ extern "C" int b200_moe_permute(const void* experts, int experts_dtype /*0 = i32
   cudaStream_t st = (cudaStream_t)stream;
   const long long n = T * topk;
   if (experts_dtype == 0)
-    launch_k(moe_index_kernel<int>, dim3((unsigned)E), dim3(1024), 0, st, (const int*)experts, n, E, tile_rows, (int*)scatter_index,
+    launch_k(n <= MOE_INDEX_ONE ? moe_index_one_kernel<int> : moe_index_kernel<int>, dim3(n <= MOE_INDEX_ONE ? 1u : (unsigned)E),
+             dim3(1024), 0, st, (const int*)experts, n, E, tile_rows, (int*)scatter_index,
              (int*)cu_seqlens, (int4*)tile_table, (int*)tile_count, max_tiles, 1, (int*)nullptr,
              (const __nv_bfloat16*)nullptr, (__nv_bfloat16*)nullptr);
   else if (experts_dtype == 1)
-    launch_k(moe_index_kernel<long long>, dim3((unsigned)E), dim3(1024), 0, st, (const long long*)experts, n, E, tile_rows,
+    launch_k(n <= MOE_INDEX_ONE ? moe_index_one_kernel<long long> : moe_index_kernel<long long>, dim3(n <= MOE_INDEX_ONE ? 1u : (unsigned)E),
+             dim3(1024), 0, st, (const long long*)experts, n, E, tile_rows,
              (int*)scatter_index, (int*)cu_seqlens, (int4*)tile_table, (int*)tile_count, max_tiles, 1,
              (int*)nullptr, (const __nv_bfloat16*)nullptr, (__nv_bfloat16*)nullptr);
   else
@@ -1212,11 +1334,13 @@ extern "C" int b200_moe_permute_index(const void* experts, int experts_dtype /*0
   cudaStream_t st = (cudaStream_t)stream;
   const long long n = T * topk;
   if (experts_dtype == 0)
-    launch_k(moe_index_kernel<int>, dim3((unsigned)E), dim3(1024), 0, st, (const int*)experts, n, E, tile_rows,
+    launch_k(n <= MOE_INDEX_ONE ? moe_index_one_kernel<int> : moe_index_kernel<int>, dim3(n <= MOE_INDEX_ONE ? 1u : (unsigned)E),
+             dim3(1024), 0, st, (const int*)experts, n, E, tile_rows,
              (int*)scatter_index, (int*)cu_seqlens, (int4*)tile_table, (int*)tile_count, max_tiles, topk,
              (int*)gather_index, (const __nv_bfloat16*)weights_bf16, (__nv_bfloat16*)row_scale);
   else if (experts_dtype == 1)
-    launch_k(moe_index_kernel<long long>, dim3((unsigned)E), dim3(1024), 0, st, (const long long*)experts, n, E, tile_rows,
+    launch_k(n <= MOE_INDEX_ONE ? moe_index_one_kernel<long long> : moe_index_kernel<long long>, dim3(n <= MOE_INDEX_ONE ? 1u : (unsigned)E),
+             dim3(1024), 0, st, (const long long*)experts, n, E, tile_rows,
              (int*)scatter_index, (int*)cu_seqlens, (int4*)tile_table, (int*)tile_count, max_tiles, topk,
              (int*)gather_index, (const __nv_bfloat16*)weights_bf16, (__nv_bfloat16*)row_scale);
   else
