@@ -400,8 +400,11 @@ greedy_logprob_kernel(const T* __restrict__ x, long long* __restrict__ tokens, f
 }
 
 // CTAs per row.  A cluster spreads few rows over idle SMs; from about a row per two SMs on, whole
-// CTAs do better (log-probabilities of 64 / 148 rows of 151936 bf16: 15 / 14 us in one CTA each, 10 / 24 in eight).
-inline int row_ctas(long long rows) { return rows <= 64 ? 8 : 1; }
+// CTAs do better (log-probabilities of 64 / 148 rows of 151936 bf16: 15 / 14 us in one CTA each, 10 / 24 in eight), and from a
+// row per four SMs on where rows are short (64 fp32 rows of 1000 / 4096 / 16384, log-softmax: 5.2 / 5.8 / 7.7 us in one CTA, 5.7 /
+// 6.8 / 7.8 in eight; 64 bf16 rows of 1000 / 4096, greedy: 5.1 / 5.5 and 6.3 / 5.2; 33 rows gain or stay at every length, 48 of bf16 too).
+template <typename T>
+inline int row_ctas(long long rows, int n) { return rows <= 40 || (rows <= 64 && n >= (sizeof(T) == 2 ? 4096 : 16384)) ? 8 : 1; }
 
 // The row kernels' launch: programmatic like launch_k's, `cl` CTAs to a row and to a cluster.
 template <typename... KArgs, typename... Args>
@@ -418,7 +421,7 @@ extern "C" int b200_log_softmax_f32(const void* x, void* out, long long rows, in
   if (rows == 0) return B200_OK;
   const bool vec = ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(out)) & 15) == 0 &&
                    x_row_stride % 4 == 0 && out_row_stride % 4 == 0;
-  const int cl = row_ctas(rows);
+  const int cl = row_ctas<float>(rows, n);
   launch_rows(cl == 1 ? log_softmax_f32_kernel<1> : log_softmax_f32_kernel<8>, rows, cl, (cudaStream_t)stream,
               (const float*)x, (float*)out, n, x_row_stride, out_row_stride, vec);
   return launch_status();
@@ -429,7 +432,7 @@ template <typename T>
 inline int gather_logprob_launch(const void* logits, const void* labels, void* out, void* lse, long long rows, int n,
                                  long long row_stride, long long ignore_index, void* stream) {
   const bool vec = (reinterpret_cast<uintptr_t>(logits) & 15) == 0 && row_stride % RowLoader<T>::VEC == 0;
-  const int cl = row_ctas(rows);
+  const int cl = row_ctas<T>(rows, n);
   launch_rows(cl == 1 ? gather_logprob_kernel<T, 1> : gather_logprob_kernel<T, 8>, rows, cl, (cudaStream_t)stream,
               (const T*)logits, (const long long*)labels, (float*)out, (float*)lse, n, row_stride, ignore_index, vec);
   return launch_status();
@@ -498,7 +501,7 @@ template <typename T>
 inline int greedy_logprob_launch(const void* logits, void* tokens, void* logprobs, long long rows, int n, long long row_stride,
                                  void* stream) {
   const bool vec = (reinterpret_cast<uintptr_t>(logits) & 15) == 0 && row_stride % RowLoader<T>::VEC == 0;
-  const int cl = row_ctas(rows);
+  const int cl = row_ctas<T>(rows, n);
   launch_rows(cl == 1 ? greedy_logprob_kernel<T, 1> : greedy_logprob_kernel<T, 8>, rows, cl, (cudaStream_t)stream,
               (const T*)logits, (long long*)tokens, (float*)logprobs, n, row_stride, vec);
   return launch_status();
