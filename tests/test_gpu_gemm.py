@@ -211,10 +211,12 @@ def test_conv3d_under_the_mode_is_deterministic_and_batch_invariant(vb):
         torch.use_deterministic_algorithms(False)
 
 
-@pytest.mark.parametrize("T, N, K", [(1000, 128, 64), (1001, 200, 64), (1023, 384, 320), (1300, 1000, 72), (2048, 2056, 128),
+@pytest.mark.parametrize("T, N, K", [(3001, 2056, 2048), (2049, 4104, 1096), (1250, 6152, 1536), (1033, 136, 20000),
+                                     (1000, 128, 64), (1001, 200, 64), (1023, 384, 320), (1300, 1000, 72), (2048, 2056, 128),
                                      (4097, 136, 2048), (1000, 2048, 200)])
 def test_products_on_cta_pairs_have_the_single_ctas_bits(vb, T, N, K):
-    """From 1000 tokens on a product may run on CTA pairs (odd and partial weight tiles, partial token tiles, K with and
+    """From 1000 tokens on a product may run on CTA pairs, where that saves enough, as in the first four sizes (the fourth
+    gated alone) (odd and partial weight tiles, partial token tiles, K with and
     without whole 64-wide atoms): every token's bits are those of the same token in a narrow batch, plain, with bias and gated."""
     from vexact_b200 import _lib
 

@@ -50,10 +50,13 @@ constexpr int GEMM_WBYTES = GEMM_WTILE * GEMM_BK * 2;
 constexpr int GEMM_THREADS = 320;       // producer warp, MMA warp, 8 epilogue warps: two per tensor-memory quadrant
 constexpr int GEMM_MAX_STAGES = 12;
 constexpr int GEMM_SMEM_BUDGET = 227 * 1024;
-// Tokens from which a dense product may run on CTA pairs: their set-up and the meeting of the CTAs cost about a microsecond,
-// which narrow products do not gain back (2048 -> 4096 for 512 / 1000 / 2048 tokens: 13.4 / 18.3 / 29.1 us alone,
-// 14.4 / 17.8 / 26.9 in pairs).
-constexpr int GEMM_PAIR_TOKENS = 1000;
+// A dense product may run on CTA pairs from this many tokens on, and where its shared-memory fill shrinks by this many rows of 128
+// bytes (gemm_dense_tiles: rows a K step x 64-wide K steps; 4096 rows are 8192 cycles): the pairs' set-up and the meeting of
+// their CTAs cost one to two microseconds.  Alone / in pairs, us, with the rows saved: 2048 tokens 1000 -> 200 9.6 / 10.8 (256),
+// 1024 -> 1024 8.4 / 9.1 (1024), 2048 -> 2048 16.1 / 17.6 (3584), 2048 -> 4096 26.8 / 27.0 (7168), 2048 -> 6144 39.1 / 37.1 (10752),
+// 1536 -> 17920 88 / 79 (24576); 1000 tokens 6144 -> 2048 28.2 / 23.6 (4608).  400 and 700 tokens 2048 -> 6144: 16.6 / 18.8,
+// 22.4 / 25.0.
+constexpr int GEMM_PAIR_TOKENS = 1000, GEMM_PAIR_GAIN = 4096;
 constexpr int GEMM_EXCH_PAD = 2;  // the SwiGLU exchange buffer holds xrows_max + 2 bf16 per feature row: an odd pitch in words
 
 struct GemmParams {
@@ -1237,7 +1240,7 @@ struct GemmExtra {
 // more SMs, gain nothing: 6144 -> 2048 took 24 us with 128 rows a tile and 23 with 32.)
 // Pairs, where the caller may use them: the same with two CTAs to a tile, each with half of its token rows.
 inline bool gemm_dense_tiles(GemmParams& p, long long T, int N, int batch, int features = GEMM_WTILE) {
-  const int sms = sm_count();
+  const int sms = sm_count(), k_steps = (p.k + GEMM_BK - 1) / GEMM_BK;
   const int min_tiles = (int)((T + 255) / 256), max_tiles = (int)((T + 15) / 16);
   long long best_cost = -1;
   const int w_tiles = (N + features - 1) / features;
@@ -1254,6 +1257,7 @@ inline bool gemm_dense_tiles(GemmParams& p, long long T, int N, int batch, int f
     }
   }
   bool pair = false;
+  best_cost -= GEMM_PAIR_GAIN / k_steps;
   for (int tt = min_tiles; T >= GEMM_PAIR_TOKENS && tt <= max_tiles; ++tt) {
     const int rows = round_up((int)((T + tt - 1) / tt), 32);
     const int tiles_t = (int)((T + rows - 1) / rows), w2 = (w_tiles + 1) / 2;
