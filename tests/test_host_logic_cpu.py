@@ -89,3 +89,12 @@ def test_attention_keys_and_attn_impl_validation():
     for name in ("fa-invariant", "fa-invariant-cute", "triton-invariant"):
         assert ALL_ATTENTION_FUNCTIONS[name] is attention.flash_attention_forward
     assert ALL_ATTENTION_FUNCTIONS["flex"] is attention.flex_attention_forward
+def test_token_tile_height_of_the_expert_products():
+    """Tall tiles for many rows per expert, unless they would leave more than a third of the chip's CTA pairs without one."""
+    from vexact_b200.fused_moe import grouped_tile_rows
+
+    assert [grouped_tile_rows(n * 128, 128) for n in (1, 64, 65, 112, 113, 1000)] == [64, 64, 128, 128, 256, 256]
+    assert [grouped_tile_rows(n * 128, 128, 1536) for n in (64, 65, 113)] == [64, 128, 256]
+    assert [grouped_tile_rows(n * 8, 8, 1024) for n in (64, 128, 160, 256, 384, 512)] == [64, 64, 128, 128, 256, 256]
+    assert grouped_tile_rows(8 * 256, 8, 512) == 64 and grouped_tile_rows(8 * 2048, 8, 512) == 256
+    assert grouped_tile_rows(8 * 128, 8, 1024, sms=72) == 256

@@ -7,6 +7,7 @@ return code.
 from __future__ import annotations
 
 import ctypes as C
+import functools
 import threading
 from pathlib import Path
 
@@ -203,6 +204,13 @@ def launch_count() -> int:
 def ptr(t) -> int | None:
     """Device pointer of a torch tensor (None passes NULL)."""
     return None if t is None else t.data_ptr()
+
+
+@functools.lru_cache(maxsize=None)
+def sm_count(device) -> int:
+    import torch
+
+    return torch.cuda.get_device_properties(device).multi_processor_count
 
 
 _current_stream = None

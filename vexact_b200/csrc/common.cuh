@@ -260,12 +260,19 @@ inline int sm_count() {
   return n;
 }
 
-// Token tiles of the grouped GEMMs.  Height for `rows` rows over `groups` groups: few rows per group want one low tile each
-// (its pipeline stages are smaller and deeper); many want tall ones, which read a weight tile less often.  fc1 of 128 experts,
-// 2048 -> 1536, at 64 / 128 / 256 rows per tile: 184 / 154 / 170 us for 94 rows per expert, 221 / 180 / 178 us for 128,
-// 383 / 281 / 260 us for 256.
-inline int grouped_tile_rows(long long rows, long long groups) {
-  return rows <= 64 * groups ? 64 : rows <= 112 * groups ? 128 : 256;
+// Token tiles of the grouped GEMMs.  Height for `rows` rows over `groups` groups of products with at least `features` outputs:
+// few rows per group want one low tile each (its pipeline stages are smaller and deeper); many want tall ones, on CTA pairs,
+// which read a weight tile less often.  128 experts, 2048 -> 1536, the same rows for each, at 64 / 128 / 256 rows per tile: 163 /
+// 133 / 142 us for 65 rows per expert, 172 / 146 / 151 for 112, 234 / 206 / 161 for 160, 298 / 223 / 185 for 256.  (Rows are not
+// evenly spread: from a mean of 112 on, some experts pass 128.)
+// A tall tile must not leave the chip idle: there are to be two thirds as many as there are pairs, if they are spread evenly.
+// 8 experts, 1024 -> 1024: 8.7 / 10.6 / 10.7 us for 128 rows per expert (128 tiles, 32 pairs, 32 pairs), 11.8 / 10.7 / 11.2 for 160
+// (192, 64, 32), 15.3 / 14.8 / 12.4 for 384 (384, 96, 64).
+inline int grouped_tile_rows(long long rows, long long groups, int features, int sms) {
+  const long long per = (rows + groups - 1) / groups;
+  for (int h = rows <= 64 * groups ? 64 : rows <= 112 * groups ? 128 : 256; h > 64; h >>= 1)
+    if (3 * groups * ((per + h - 1) / h) * ((features + 255) / 256) >= sms) return h;
+  return 64;
 }
 // Tile j of a group's `tiles`, which is rows / tile_rows rounded up: {group, first row, rows, 0}.  The tiles of a group are equally
 // high, in steps of 16, so that none is a remainder that pays for a whole weight tile, and at most tile_rows, which need not be

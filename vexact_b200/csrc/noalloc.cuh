@@ -102,7 +102,7 @@ inline int grouped_gemm_noalloc(const void* x, const void* w, const void* row_sc
       (mode != 0 && mode != 1))
     return B200_ERR_ARG;
   if (num_groups > NOALLOC_MAX_GROUPS) return B200_ERR_SHAPE;
-  const int tile_rows = mode == 0 ? grouped_tile_rows(x_rows, num_groups) : 64;
+  const int tile_rows = mode == 0 ? grouped_tile_rows(x_rows, num_groups, n_out, sm_count()) : 64;
   const long long bound = (long long)num_groups + x_rows / 64;
   if (bound > NOALLOC_MAX_TILES) return B200_ERR_SHAPE;
   if (x_rows == 0) return B200_OK;
