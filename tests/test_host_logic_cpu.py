@@ -89,6 +89,18 @@ def test_attention_keys_and_attn_impl_validation():
     for name in ("fa-invariant", "fa-invariant-cute", "triton-invariant"):
         assert ALL_ATTENTION_FUNCTIONS[name] is attention.flash_attention_forward
     assert ALL_ATTENTION_FUNCTIONS["flex"] is attention.flex_attention_forward
+
+
+def test_attention_tiles_from_which_a_step_orders_its_sequences():
+    """One tile for a sequence, a KV head and up to eight of its query heads; more of them than SMs."""
+    from vexact_b200.inferencer import order_pays
+
+    assert not order_pays(74, 16, 2, 148) and order_pays(75, 16, 2, 148)
+    assert not order_pays(18, 32, 4, 72) and order_pays(19, 32, 4, 72)
+    assert order_pays(38, 32, 2, 148) and not order_pays(37, 32, 2, 148)       # 16 query heads to a KV head: two tiles
+    assert not order_pays(74, 2, 2, 148) and order_pays(75, 2, 2, 148)
+
+
 def test_token_tile_height_of_the_expert_products():
     """Tall tiles for many rows per expert, unless they would leave more than a third of the chip's CTA pairs without one."""
     from vexact_b200.fused_moe import grouped_tile_rows

@@ -36,9 +36,13 @@ BF = torch.bfloat16
 # default: inside the captured decode step it measured 0.0-0.5 % (32.04 -> 31.87-32.04 ms), within run-to-run
 # noise, and the stable order is the simpler thing to reason about.
 _ROUTE_PLAN = os.environ.get("B200_MOE_ROUTE_PLAN", "0") == "1"
-# (sequence, KV head) pairs from which a step without an order ranks its sequences by context: about one per SM, below which
-# no persistent attention CTA has a second tile
-ORDER_MIN_TILES = 148
+
+
+def order_pays(num_seqs: int, q_heads: int, kv_heads: int, sms: int) -> bool:
+    """Whether a step without an order ranks its sequences by context: one token each already makes more attention tiles (a
+    sequence, a KV head, up to eight of its query heads) than there are SMs, so that some persistent CTA has a second one.
+    (Steps with longer query runs have more tiles than this counts; what ordering gives them was not measured.)"""
+    return num_seqs * kv_heads * -(-(q_heads // kv_heads) // 8) > sms
 
 
 @dataclass(frozen=True)
