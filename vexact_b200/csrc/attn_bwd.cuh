@@ -25,7 +25,7 @@ constexpr int AB_THREADS = 256;   // thread (ty, tx) = (tid / 16, tid % 16)
 struct AttnBwdParams {
   const __nv_bfloat16 *q, *k, *v, *out, *dout;   // [total_q, hq, DK], [total_k, hkv, DK], [total_k, hkv, DV], [total_q, hq, DV] x 2
   __nv_bfloat16 *dq, *dk, *dv;
-  float *lse, *delta;                            // scratch [total_q, hq]; with have_lse, lse comes from the forward
+  float *lse, *delta;                            // scratch of total_q * hq: [total_q, hq], tcgen05 kernels [hq, total_q]; with have_lse, lse comes from the forward
   const int *cu_q, *cu_k;                        // [num_seqs + 1]
   int hq, hkv;
   long long total_q, total_k;

@@ -1414,7 +1414,8 @@ extern "C" int b200_moe_grouped_wgrad_strided(const void* a, long long a_row_str
   if (M % 4 != 0 || N % 4 != 0 || num_groups > 65535 || (M + WG_TILE - 1) / WG_TILE > 65535 || rows > 0x7fffffffLL)
     return B200_ERR_SHAPE;
   const bool vec16 = M % 8 == 0 && N % 8 == 0 && a_row_stride % 8 == 0 && b_row_stride % 8 == 0 &&
-                     ((reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(b) | reinterpret_cast<uintptr_t>(c)) & 15) == 0;
+                     ((reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(b)) & 15) == 0 &&
+                     (reinterpret_cast<uintptr_t>(c) & 3) == 0;
   if (vec16)
     return moe_wgrad_tc_launch(a, a_row_stride, b, b_row_stride, c, (const int*)cu_seqlens, rows, num_groups, M, N,
                                (cudaStream_t)stream);
