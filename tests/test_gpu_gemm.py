@@ -278,3 +278,37 @@ def test_second_operand_may_be_the_output_of_the_launch_before(vb, T, N, K):
         static.copy_(x)
         graph.replay()
         assert torch.equal(out[0], b[0]) and torch.equal(out[1], b[1])
+
+
+def test_copies_of_weights_are_not_read_early(vb, monkeypatch):
+    """Inside a pass with settled weights, a weight that `linear` has to copy (rows or a base that 16-byte accesses do not fit, columns
+    first) is the output of the launch before its product, which therefore runs as outside the pass."""
+    from vexact_b200 import _lib
+
+    lib, calls = _lib.load(), []
+
+    class Recorder:
+        def __getattr__(self, name):
+            f = getattr(lib, name)
+            if not name.startswith("b200_"):
+                return f
+            return lambda *a: (calls.append((name, a[0]) if name == "b200_settled_weights" else name), f(*a))[1]
+
+    monkeypatch.setattr(_lib, "load", lambda recorder=Recorder(): recorder)
+    x = torch.randn(3, 72, device="cuda").to(BF)
+    w = torch.randn(40, 80, device="cuda").to(BF)
+    on, off = (("b200_settled_weights", v) for v in (1, 0))
+    for weight in (w[:, 4:76], w.view(-1)[1:1 + 40 * 72].view(40, 72), w[:, :72].t().contiguous().t()):
+        a = x[:, :weight.shape[1]]
+        calls.clear()
+        with _lib.settled_weights():
+            out = vb.linear(a, weight)
+        assert calls == [on, off, "b200_gemm_bf16", on, off], calls
+        torch.testing.assert_close(out.float(), a.float() @ weight.float().t(), rtol=2 ** -7, atol=2e-2)
+        calls.clear()
+        vb.linear(a, weight)
+        assert calls == ["b200_gemm_bf16"]
+    calls.clear()
+    with _lib.settled_weights():
+        vb.linear(x, w[:, :72])
+    assert calls == [on, "b200_gemm_bf16", off]

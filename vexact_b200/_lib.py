@@ -6,6 +6,7 @@ return code.
 """
 from __future__ import annotations
 
+import contextlib
 import ctypes as C
 import functools
 import threading
@@ -233,11 +234,29 @@ class settled_weights:
     """`with settled_weights():` around the launches of a forward pass, none of which writes a weight: its dense products may
     request their weights before the launch before them is over.  Weights written before it are waited for."""
 
+    _here = threading.local()
+
     def __enter__(self):
+        self._here.on = True
         load().b200_settled_weights(1)
 
     def __exit__(self, *exc):
+        self._here.on = False
         load().b200_settled_weights(0)
+
+
+@contextlib.contextmanager
+def operand_just_made():
+    """Around a product whose second operand is a copy made by the launch before it: no weight is requested early, inside
+    `settled_weights` or not."""
+    inside = getattr(settled_weights._here, "on", False)
+    if inside:
+        load().b200_settled_weights(0)
+    try:
+        yield
+    finally:
+        if inside:
+            load().b200_settled_weights(1)
 
 
 def read_status() -> tuple[int, int, int, int]:

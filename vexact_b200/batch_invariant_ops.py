@@ -54,6 +54,7 @@ def linear(x: torch.Tensor, weight: torch.Tensor, bias: torch.Tensor | None = No
     x2 = x.reshape(-1, K)
     if x2.stride(-1) != 1:
         x2 = x2.contiguous()
+    given = weight
     if weight.stride(-1) != 1:
         weight = weight.contiguous()
     T = x2.shape[0]
@@ -76,11 +77,13 @@ def linear(x: torch.Tensor, weight: torch.Tensor, bias: torch.Tensor | None = No
         out = torch.empty((T, N), device=x.device, dtype=out_dtype)
         fn, name = (lib.b200_gemm_bf16, "b200_gemm_bf16") if x.dtype == torch.bfloat16 else \
             (lib.b200_gemm_f16, "b200_gemm_f16")
-        _lib.check(
-            fn(x2.data_ptr(), weight.data_ptr(), _lib.ptr(bias), out.data_ptr(), T, N, K, x2.stride(0),
-               weight.stride(0), out.stride(0), 0 if out_dtype == x.dtype else 1, _lib.current_stream()),
-            name,
-        )
+        args = (x2.data_ptr(), weight.data_ptr(), _lib.ptr(bias), out.data_ptr(), T, N, K, x2.stride(0), weight.stride(0),
+                out.stride(0), 0 if out_dtype == x.dtype else 1, _lib.current_stream())
+        if weight is given:
+            _lib.check(fn(*args), name)
+        else:
+            with _lib.operand_just_made():
+                _lib.check(fn(*args), name)
     elif x.dtype == torch.float32:
         if bias is not None:
             bias = bias.float().contiguous()
